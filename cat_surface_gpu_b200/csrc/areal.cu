@@ -57,7 +57,8 @@ struct ArealParams {
     int nloc_max;  // vertices owned by one CTA (set at launch)
     int iterations;
     int project_every;
-    int allow_dataflow;  // float32 modes: published (value, version) words instead of per-step barriers
+    int allow_dataflow;  // float32 modes: published (position, version) words instead of per-step barriers
+    unsigned int epoch_magic;  // ceil(2^32 / project_every), 0: divide (see epoch_rest)
     double radius;
     unsigned long long timeout_ns;
 };
@@ -452,10 +453,12 @@ __global__ void __launch_bounds__(512) areal_sweeps_kernel(ArealParams p) {
 // Dataflow form of the sweeps (float32 storage modes).
 //
 // The grid barrier between wavefront steps is replaced by per-vertex versions.
-// Each coordinate of each vertex is published as one 8-byte word
-// (float32 bits | version << 32), version = the number of sweeps the vertex
-// has completed; 8-byte aligned accesses are single-copy atomic, so a word
-// read with a relaxed load carries a value and the version it belongs to.
+// Each vertex is published as one 16-byte word (x, y, z, version), version = the
+// number of sweeps the vertex has completed; a relaxed 16-byte load returns a
+// position and the version it belongs to.  The words sit kWordPitch quads (64
+// bytes) apart, so no two vertices' words share a 32-byte sector or its pair:
+// polls of one vertex do not queue behind the publication of another (61,442
+// vertices, 4,999 sweeps: 61.4 ms at 16 bytes, 53.9 at 32, 50.0 at 64 and at 128).
 // Sweep s of vertex v needs lower-index neighbours at version s and
 // higher-index neighbours and v itself at version s - 1, and neither can be
 // further ahead: a lower neighbour u cannot finish sweep s + 1 before v
@@ -472,123 +475,168 @@ __global__ void __launch_bounds__(512) areal_sweeps_kernel(ArealParams p) {
 // Every wait is bounded: on timeout (or another CTA's failure) the kernel
 // records the status and leaves.
 
-using csg::ld_word;
-using csg::make_word;
-using csg::st_word;
-using csg::word_value;
-using csg::word_version;
-
-// words of vertex v: pub[4 v + k], k = 0, 1, 2 (coordinate k), 3 unused
-template <typename P3>
-__device__ __forceinline__ bool load_versioned(const unsigned long long* pub, int u, unsigned int need, P3& q) {
-    const unsigned long long* w = pub + 4LL * u;
-    const unsigned long long a = ld_word(w), b = ld_word(w + 1), c = ld_word(w + 2);
-    q = {word_value(a), word_value(b), word_value(c)};
-    return word_version(a) == need && word_version(b) == need && word_version(c) == need;
-}
-
-__device__ __forceinline__ bool wait_expired(const ArealParams& p, unsigned int& polls, unsigned long long& start) {
-    return csg::warp_wait_expired(p.ctl, p.timeout_ns, polls, start);
-}
+using csg::ld_quad;
+using csg::make_quad;
+using csg::Quad;
+using csg::quad_point;
+using csg::quad_version;
+using csg::st_quad;
 
 // Ring of a vertex: itself, then the other vertices of its faces (at most
-// kRingMax); each face slot is coded as three ring indices (8 bits each).
+// 2 max_degree + 1 of them, the rows' capacity; the form is taken up to kRingMax);
+// each face slot is coded as three ring indices (8 bits each).
 constexpr int kRingMax = 20;
 
-// One vertex update of sweep s by a group of G lanes (all 32 lanes call it;
-// inactive groups pass v < 0).  The group first polls the words of the ring --
-// lane j loads members j, j + G, ... all at once, one round trip per poll --
-// and stages the positions in shared memory (`pos`, kRingMax entries per
-// group), then computes the faces exactly as update_vertex does (same
-// arithmetic, slot order).  Lanes 0, 1, 2 publish coordinates 0, 1, 2.
-// Returns false to abort.
-template <int MODE, int G>
-__device__ __forceinline__ bool update_vertex_df(const ArealParams& p, unsigned long long* pub,
-                                                 const unsigned long long* prev, unsigned long long* proj_out, int v,
-                                                 const int* ring, int nring, const int* code, int deg, unsigned int s,
-                                                 double (*stage)[32], float3* pos) {
-    using T = Traits<MODE>;
-    using Acc = typename T::Acc;
-    using P3 = typename T::P3;
-    constexpr int kQ = (kRingMax + G - 1) / G;
-    const int lane = threadIdx.x & 31;
-    const int glane = lane & (G - 1);
-    const int gbase = lane & ~(G - 1);
-    if (v < 0) {
-        deg = 0;
-        nring = 0;
+// Vertex v's published word is words[kWordPitch v], its projected word the quad
+// kProjected further on (written once per projection epoch, so it may share the 64 bytes).
+constexpr int kWordPitch = 4, kProjected = 2;
+
+// Entries of a ring row and of a group's staged positions: one for every lane of the group at least.
+__host__ __device__ inline int dataflow_ring_capacity(int max_degree, int lanes) {
+    return 2 * max_degree + 1 > lanes ? 2 * max_degree + 1 : lanes;
+}
+
+// sweep mod project_every (> 0): a high multiply with the host's rounded-up reciprocal,
+// exact while sweep * project_every < 2^32 (the host passes 0 when it may not be).
+__device__ __forceinline__ unsigned int epoch_rest(const ArealParams& p, unsigned int sweep) {
+    const unsigned int pe = static_cast<unsigned int>(p.project_every);
+    if (p.epoch_magic == 0) return sweep % pe;
+    return sweep - __umulhi(sweep, p.epoch_magic) * pe;
+}
+
+// Poll the words of ring members glane, glane + G, ... (`first` is this lane's member 0,
+// -1 for none) until each shows the version this update needs (lower members sweep s, the
+// others and the vertex itself s - 1), then stage their positions.  MEMBERS = 1 serves
+// rings of at most G members (one word per lane).  `late` is kProjected in the sweep after
+// a projection, whose previous-sweep members are the projected points.  A lane that has
+// its version stops loading: the word cannot change before this update publishes, and each
+// word a poll re-reads costs the SM's L1 data path a pass (with the shared-memory staging
+// the kernel's busiest unit), which holds up the updates that could proceed.  For the same
+// reason one poll is in flight per lane: two or three made the sweeps slower (77 and
+// 99 ms against 62).  Returns false to abort.
+template <int MEMBERS, int G>
+__device__ __forceinline__ bool poll_ring(const ArealParams& p, const Quad* words, int late, int v, int first,
+                                          const int* ring, int nring, unsigned int s, float4* pos) {
+    const int glane = threadIdx.x & (G - 1);
+    const Quad* from[MEMBERS];
+    unsigned int need[MEMBERS];
+    Quad w[MEMBERS];
+#pragma unroll
+    for (int q = 0; q < MEMBERS; ++q) {
+        const int u = q == 0 ? first : (glane + q * G < nring ? ring[glane + q * G] : -1);
+        need[q] = u < v ? s : s - 1;
+        w[q] = Quad{0, static_cast<unsigned long long>(need[q]) << 32};  // no member: nothing to wait for
+        from[q] = words + (static_cast<long long>(kWordPitch) * u + (u < v ? 0 : late));
+        if (u >= 0) w[q] = ld_quad(from[q]);
     }
     unsigned int polls = 0;
     unsigned long long start = 0;
-    int who[kQ];
-#pragma unroll
-    for (int q = 0; q < kQ; ++q) {
-        const int k = glane + q * G;
-        who[q] = k < nring ? ring[k] : -1;
-    }
     while (true) {
-        unsigned long long w[kQ][3];
+        bool want = false;
 #pragma unroll
-        for (int q = 0; q < kQ; ++q)
-            if (who[q] >= 0)
+        for (int q = 0; q < MEMBERS; ++q) want = want || quad_version(w[q]) != need[q];
+        if (!__any_sync(kFull, want)) break;
+        if (csg::warp_wait_expired(p.ctl, p.timeout_ns, polls, start)) return false;
 #pragma unroll
-                for (int k = 0; k < 3; ++k) w[q][k] = ld_word((who[q] < v ? pub : prev) + 4LL * who[q] + k);
-        bool ok = true;
+        for (int q = 0; q < MEMBERS; ++q)
+            if (quad_version(w[q]) != need[q]) w[q] = ld_quad(from[q]);
+    }
 #pragma unroll
-        for (int q = 0; q < kQ; ++q)
-            if (who[q] >= 0) {
-                const unsigned int need = who[q] < v ? s : s - 1;  // the vertex itself: s - 1
-                ok = ok && word_version(w[q][0]) == need && word_version(w[q][1]) == need &&
-                     word_version(w[q][2]) == need;
-                pos[glane + q * G] = make_float3(word_value(w[q][0]), word_value(w[q][1]), word_value(w[q][2]));
-            }
-        if (__all_sync(kFull, ok)) break;
-        if (wait_expired(p, polls, start)) return false;
+    for (int q = 0; q < MEMBERS; ++q)
+        if (q == 0 || glane + q * G < nring) pos[glane + q * G] = quad_point(w[q]);
+    return true;
+}
+
+constexpr int kStagePitch = 34;  // doubles per staged row: the four rows of a warp start on different banks
+
+// The area total (lanes 0..2) and one coordinate's weighted sum (lane k: coordinate k) of up
+// to G staged faces, added in slot order.  Slots past the last face hold +0, which leaves a
+// sum that started from +0 unchanged, so the G additions need no test.
+template <int G>
+__device__ __forceinline__ void add_faces(const double (*stage)[kStagePitch], int glane, int gbase, double& total,
+                                          double& wsum) {
+    const double2* ta = reinterpret_cast<const double2*>(&stage[0][gbase]);
+    const double2* tm = reinterpret_cast<const double2*>(&stage[1 + glane][gbase]);
+#pragma unroll
+    for (int q = 0; q < G / 2; ++q) {
+        const double2 x = ta[q], y = tm[q];
+        total = __dadd_rn(__dadd_rn(total, x.x), x.y);
+        wsum = __dadd_rn(__dadd_rn(wsum, y.x), y.y);
+    }
+}
+
+// One vertex update of sweep s by a group of G lanes (all 32 lanes call it;
+// groups without an item pass v < 0 and nring = deg = 0).  The group polls the
+// ring and stages the positions in shared memory (`pos`), then computes the
+// faces exactly as update_vertex does (same arithmetic, slot order).  Lane 0
+// publishes the point.  Returns false to abort.
+template <int MODE, int G>
+__device__ __forceinline__ bool update_vertex_df(const ArealParams& p, Quad* words, int v, const int* ring, int nring,
+                                                 const int* code, int deg, unsigned int s,
+                                                 double (*stage)[kStagePitch], float4* pos) {
+    using T = Traits<MODE>;
+    using Acc = typename T::Acc;
+    using P3 = typename T::P3;
+    const int lane = threadIdx.x & 31;
+    const int glane = lane & (G - 1);
+    const int gbase = lane & ~(G - 1);
+    const int first = glane < nring ? ring[glane] : -1;
+    // sweep s ends a projection epoch (publish the projected point too), or follows one
+    bool at_end = false;
+    int late = 0;
+    if (p.project_every > 0) {
+        const unsigned int rest = epoch_rest(p, s);
+        at_end = rest == 0;
+        if (s > 1 && (p.project_every == 1 || rest == 1)) late = kProjected;
+    }
+    const bool wide = __any_sync(kFull, max(nring, deg) > G);  // more ring members or faces than lanes in the warp
+    if (!wide) {
+        if (!poll_ring<1, G>(p, words, late, v, first, ring, nring, s, pos)) return false;
+    } else {
+        if (!poll_ring<(kRingMax + G - 1) / G, G>(p, words, late, v, first, ring, nring, s, pos)) return false;
     }
     __syncwarp();
-    const int wdeg = __reduce_max_sync(kFull, deg);
     Acc total = 0, wx = 0, wy = 0, wz = 0;  // float path: every lane sums its group's faces
     double wsum = 0;                        // float64 path: lanes 0..2 sum one coordinate each
-    for (int c0 = 0; c0 < wdeg; c0 += G) {
-        const int j = c0 + glane;
-        const bool face = j < deg;
-        P3 a{}, b{}, c{};
-        if (face) {
+    auto corner = [&](int index) {
+        const float4 q = pos[index & 255];
+        return P3{q.x, q.y, q.z};
+    };
+    auto stage_face = [&](int j) {  // float64 path: face slot j's area and weighted centre
+        double fa = 0, fx = 0, fy = 0, fz = 0;
+        if (j < deg) {
             const int cd = code[j];
-            const float3 pa = pos[cd & 255], pb = pos[(cd >> 8) & 255], pc = pos[(cd >> 16) & 255];
-            a = {pa.x, pa.y, pa.z};
-            b = {pb.x, pb.y, pb.z};
-            c = {pc.x, pc.y, pc.z};
+            Acc area, mx, my, mz;
+            T::face(corner(cd), corner(cd >> 8), corner(cd >> 16), area, mx, my, mz);
+            fa = area;
+            fx = __dmul_rn(fa, mx);
+            fy = __dmul_rn(fa, my);
+            fz = __dmul_rn(fa, mz);
         }
-        if constexpr (sizeof(Acc) == 8) {
-            double fa = 0, fx = 0, fy = 0, fz = 0;
-            if (face) {
-                double mx, my, mz;
-                T::face(a, b, c, fa, mx, my, mz);
-                fx = __dmul_rn(fa, mx);
-                fy = __dmul_rn(fa, my);
-                fz = __dmul_rn(fa, mz);
-            }
-            stage[0][lane] = fa;
-            stage[1][lane] = fx;
-            stage[2][lane] = fy;
-            stage[3][lane] = fz;
-            __syncwarp();
-            if (glane < 3) {
-                const double* mine = stage[1 + glane];
-                const int n = min(G, deg - c0);
-#pragma unroll
-                for (int q = 0; q < G; ++q) {
-                    if (q < n) {  // slot order == ascending face id
-                        total = __dadd_rn(total, stage[0][gbase + q]);
-                        wsum = __dadd_rn(wsum, mine[gbase + q]);
-                    }
-                }
-            }
-            __syncwarp();
+        stage[0][lane] = fa;
+        stage[1][lane] = fx;
+        stage[2][lane] = fy;
+        stage[3][lane] = fz;
+        __syncwarp();
+    };
+    if constexpr (sizeof(Acc) == 8) {
+        if (!wide) {
+            stage_face(glane);
+            if (glane < 3) add_faces<G>(stage, glane, gbase, total, wsum);
         } else {
+            for (int c0 = 0; __any_sync(kFull, c0 < deg); c0 += G) {
+                stage_face(c0 + glane);
+                if (glane < 3) add_faces<G>(stage, glane, gbase, total, wsum);
+                __syncwarp();
+            }
+        }
+    } else {
+        for (int c0 = 0; __any_sync(kFull, c0 < deg); c0 += G) {
             Acc fa = 0, fx = 0, fy = 0, fz = 0;
-            if (face) T::face(a, b, c, fa, fx, fy, fz);
+            if (c0 + glane < deg) {
+                const int cd = code[c0 + glane];
+                T::face(corner(cd), corner(cd >> 8), corner(cd >> 16), fa, fx, fy, fz);
+            }
 #pragma unroll
             for (int q = 0; q < G; ++q) {
                 const Acc aa = __shfl_sync(kFull, fa, gbase + q);
@@ -605,51 +653,47 @@ __device__ __forceinline__ bool update_vertex_df(const ArealParams& p, unsigned 
         }
     }
     // a vertex that does not move republishes its own position (ring member 0)
-    float value = 0.0f;
-    if (v >= 0 && glane < 3) value = glane == 0 ? pos[0].x : (glane == 1 ? pos[0].y : pos[0].z);
+    float nx = 0.0f, ny = 0.0f, nz = 0.0f;
     if constexpr (sizeof(Acc) == 8) {
-        // total is summed by each of lanes 0..2 (same order, same value)
-        if (v >= 0 && glane < 3 && total > 0.0) {
-            const double safe = total > 1.0e-20 ? total : 1.0e-20;
-            value = __double2float_rn(__ddiv_rn(wsum, safe));
+        float value = 0.0f;
+        if (v >= 0 && glane < 3) {
+            value = glane == 0 ? pos[0].x : (glane == 1 ? pos[0].y : pos[0].z);
+            if (total > 0.0) {  // summed by each of lanes 0..2 (same order, same value)
+                const double safe = total > 1.0e-20 ? total : 1.0e-20;
+                value = __double2float_rn(__ddiv_rn(wsum, safe));
+            }
         }
-    } else {
-        float nx = 0.0f, ny = 0.0f, nz = 0.0f;
-        const bool moved = v >= 0 && glane == 0 && total > Acc(0);
-        if (moved) {
+        nx = value;
+        ny = __shfl_sync(kFull, value, gbase + 1);
+        nz = __shfl_sync(kFull, value, gbase + 2);
+    } else if (v >= 0 && glane == 0) {
+        nx = pos[0].x;
+        ny = pos[0].y;
+        nz = pos[0].z;
+        if (total > Acc(0)) {
             const float safe = total > 1.0e-20f ? total : 1.0e-20f;
             nx = __fdiv_rn(wx, safe);
             ny = __fdiv_rn(wy, safe);
             nz = __fdiv_rn(wz, safe);
         }
-        const int m = __shfl_sync(kFull, moved ? 1 : 0, gbase);
-        const float ny1 = __shfl_sync(kFull, ny, gbase);
-        const float nz2 = __shfl_sync(kFull, nz, gbase);
-        if (m) value = glane == 0 ? nx : (glane == 1 ? ny1 : nz2);
     }
-    __syncwarp();  // every lane is done with `pos` before the next update overwrites it
-    if (v >= 0 && glane < 3) st_word(pub + 4LL * v + glane, make_word(value, s));
-    if (__any_sync(kFull, proj_out != nullptr && v >= 0)) {
-        // sweep s ends a projection epoch: publish the projected point too (T::project_p3 of
-        // the float32 values just published, as the separate projection pass computed it)
-        const float px = __shfl_sync(kFull, value, gbase), py = __shfl_sync(kFull, value, gbase + 1),
-                    pz = __shfl_sync(kFull, value, gbase + 2);
-        if (proj_out != nullptr && v >= 0 && glane < 3) {
-            const P3 q = T::project_p3(P3{px, py, pz}, p.radius);
-            st_word(proj_out + 4LL * v + glane, make_word(glane == 0 ? q.x : (glane == 1 ? q.y : q.z), s));
+    if (v >= 0 && glane == 0) {
+        Quad* word = words + static_cast<long long>(kWordPitch) * v;
+        st_quad(word, make_quad(nx, ny, nz, s));
+        if (at_end) {
+            // T::project_p3 of the float32 values just published, as a separate projection pass computes it
+            const P3 q = T::project_p3(P3{nx, ny, nz}, p.radius);
+            st_quad(word + kProjected, make_quad(q.x, q.y, q.z, s));
         }
     }
+    __syncwarp();  // every lane is done with `pos` and `stage` before the next update overwrites them
     return true;
 }
 
 template <int MODE, int G>
 __global__ void __launch_bounds__(512) areal_dataflow_kernel(ArealParams p) {
-    using T = Traits<MODE>;
-    using P3 = typename T::P3;
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ double stage_all[512 / 32][4][32];
-    double (*stage)[32] = stage_all[threadIdx.x >> 5];
-    unsigned long long* pub = static_cast<unsigned long long*>(p.work);
+    Quad* words = static_cast<Quad*>(p.work);
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
     const int nthreads = gridDim.x * blockDim.x;
     const int c = blockIdx.x;
@@ -660,22 +704,28 @@ __global__ void __launch_bounds__(512) areal_dataflow_kernel(ArealParams p) {
     const int nloc = owned_below(p.n, c, nc);
     const int L = p.n_levels;
     const int D = p.stride;
-    // shared-memory image: per warp, kRingMax staged positions per group; per
-    // owned vertex its ring, ring size, face codes, id, degree and level; per
-    // level the owned range; per residue the top level
-    float3* wpos = reinterpret_cast<float3*>(smem) + (threadIdx.x >> 5) * (32 / G) * kRingMax;
-    float3* pos = wpos + my_group * kRingMax;
-    int* lring = reinterpret_cast<int*>(reinterpret_cast<float3*>(smem) + (blockDim.x / 32) * (32 / G) * kRingMax);
-    int* lcode = lring + p.nloc_max * kRingMax;
-    int* lnring = lcode + p.nloc_max * p.max_degree;
-    int* lvid = lnring + p.nloc_max;
-    int* ldeg = lvid + p.nloc_max;
-    int* llev = ldeg + p.nloc_max;
-    int* lbeg = llev + p.nloc_max;
+    const int cap = dataflow_ring_capacity(p.max_degree, G);
+    // shared-memory image: per warp the staged face terms; per group `cap` staged
+    // positions; per owned vertex its description (id, degree | ring size << 8,
+    // level / D), ring and face codes; per level the owned range; per residue the
+    // top level
+    double (*stage)[kStagePitch] = reinterpret_cast<double (*)[kStagePitch]>(smem) + 4 * (threadIdx.x >> 5);
+    float4* pos0 = reinterpret_cast<float4*>(smem + (blockDim.x / 32) * 4 * kStagePitch * sizeof(double));
+    float4* pos = pos0 + (threadIdx.x / G) * cap;
+    int4* lmeta = reinterpret_cast<int4*>(pos0 + (blockDim.x / G) * cap);
+    int* lring = reinterpret_cast<int*>(lmeta + p.nloc_max);
+    int* lcode = lring + p.nloc_max * cap;
+    int* lbeg = lcode + p.nloc_max * p.max_degree;
     int* lend = lbeg + L;
     int* hitop = lend + L;
     unsigned int phase = 0;
     int barrier_id = 0;
+    for (int l = threadIdx.x; l < L; l += blockDim.x) {
+        const int b = owned_below(__ldg(p.level_begin + l), c, nc), e = owned_below(__ldg(p.level_end + l), c, nc);
+        lbeg[l] = b;
+        lend[l] = e;
+        for (int i = b; i < e; ++i) lmeta[i].z = l / D;
+    }
     for (int i = threadIdx.x; i < nloc; i += blockDim.x) {
         const int v = __ldg(p.order + c + i * nc);
         const int s0 = __ldg(p.slot_off + v);
@@ -684,7 +734,7 @@ __global__ void __launch_bounds__(512) areal_dataflow_kernel(ArealParams p) {
             if (atomicCAS(&p.ctl->status, CSG_OK, CSG_ERR_ARG) == CSG_OK) p.ctl->where = -3;
             d = 0;
         }
-        int* ring = lring + i * kRingMax;
+        int* ring = lring + i * cap;
         int nr = 1;
         ring[0] = v;
         for (int j = 0; j < d; ++j) {
@@ -695,7 +745,7 @@ __global__ void __launch_bounds__(512) areal_dataflow_kernel(ArealParams p) {
                 int at = 0;
                 while (at < nr && ring[at] != u[k]) ++at;
                 if (at == nr) {
-                    if (nr == kRingMax) {  // the host sized kRingMax from max_degree; report, stay inside
+                    if (nr == cap) {  // cannot be with at most max_degree faces round v; report, stay inside
                         if (atomicCAS(&p.ctl->status, CSG_OK, CSG_ERR_ARG) == CSG_OK) p.ctl->where = -1;
                         at = 0;
                     } else {
@@ -706,23 +756,17 @@ __global__ void __launch_bounds__(512) areal_dataflow_kernel(ArealParams p) {
             }
             lcode[i * p.max_degree + j] = cd;
         }
-        lnring[i] = nr;
-        lvid[i] = v;
-        ldeg[i] = d;
-    }
-    for (int l = threadIdx.x; l < L; l += blockDim.x) {
-        const int b = owned_below(__ldg(p.level_begin + l), c, nc), e = owned_below(__ldg(p.level_end + l), c, nc);
-        lbeg[l] = b;
-        lend[l] = e;
-        for (int i = b; i < e; ++i) llev[i] = l;
+        lmeta[i].x = v;
+        lmeta[i].y = d | (nr << 8);
     }
     for (int r = threadIdx.x; r < D; r += blockDim.x) hitop[r] = (L - 1) - ((L - 1 - r) % D + D) % D;
     for (int v = tid; v < p.n; v += nthreads) {
         const float* q = static_cast<const float*>(p.points) + 3LL * v;
-        for (int k = 0; k < 3; ++k) st_word(pub + 4LL * v + k, make_word(q[k], 0u));
+        Quad* word = words + static_cast<long long>(kWordPitch) * v;
+        st_quad(word, make_quad(q[0], q[1], q[2], 0u));
         // projected words start at version 0, below any epoch's end: a word left
         // from an earlier call on the same scratch never satisfies a poll
-        for (int k = 0; k < 3; ++k) st_word(pub + 4LL * p.n + 4LL * v + k, make_word(0.0f, 0u));
+        st_quad(word + kProjected, make_quad(0.0f, 0.0f, 0.0f, 0u));
     }
     if (csg::grid_barrier(p.ctl, phase, p.timeout_ns, barrier_id++)) return;
     // a ring overflow or a degree over max_degree: the same answer in every CTA
@@ -730,54 +774,50 @@ __global__ void __launch_bounds__(512) areal_dataflow_kernel(ArealParams p) {
 
     // One wavefront over every sweep.  The projection after sweep b (b a multiple of
     // project_every) is applied by each vertex's group as it publishes sweep b, into
-    // the second word array `proj`; the updates of sweep b + 1 read their
-    // previous-sweep members (higher neighbours and the vertex itself) from there,
-    // the updates of sweep b read the unprojected words.  The wavefront therefore
+    // its projected word; the updates of sweep b + 1 read their previous-sweep
+    // members (higher neighbours and the vertex itself) from there, the updates of
+    // sweep b read the unprojected words.  The wavefront therefore
     // never drains at a projection.
     const int last = p.iterations - 1;
-    unsigned long long* proj = pub + 4LL * p.n;
     if (last >= 1) {
         const int span = (last - 1) * D;  // host guarantees span + L < 2^31
         const int nsteps = span + L;
-        int r = 0;
-        for (int t = 0; t < nsteps; ++t, r = (r + 1 == D) ? 0 : r + 1) {
+        int r = 0, tq = 0;                // t mod D, t / D
+        for (int t = 0; t < nsteps; ++t) {
             int lo = t - span;
             if (lo < r) lo = r;
             const int hi = t < L ? t : hitop[r];
-            if (hi < lo) continue;
-            const int i0 = lbeg[lo], i1 = lend[hi];
-            for (int base = i0 + warp_first_group; base < i1; base += groups) {
-                const int i = base + my_group;
-                int v = -1, deg = 0, nring = 0;
-                unsigned int sweep = 0;
-                const int* ring = nullptr;
-                const int* code = nullptr;
-                if (i < i1) {
-                    v = lvid[i];
-                    deg = ldeg[i];
-                    nring = lnring[i];
-                    ring = lring + i * kRingMax;
-                    code = lcode + i * p.max_degree;
-                    sweep = static_cast<unsigned int>(1 + (t - llev[i]) / D);
+            if (hi >= lo) {
+                const int i0 = lbeg[lo], i1 = lend[hi];
+                for (int base = i0 + warp_first_group; base < i1; base += groups) {
+                    const int i = base + my_group;
+                    int4 m = make_int4(-1, 0, 0, 0);
+                    if (i < i1) m = lmeta[i];
+                    const unsigned int sweep = static_cast<unsigned int>(1 + tq - m.z);  // t and the level agree mod D
+                    if (!update_vertex_df<MODE, G>(p, words, m.x, lring + i * cap, m.y >> 8,
+                                                   lcode + i * p.max_degree, m.y & 255, sweep, stage, pos))
+                        return;
                 }
-                const bool after = p.project_every > 0 && sweep > 1 && (sweep - 1) % p.project_every == 0;
-                const bool at = p.project_every > 0 && sweep > 0 && sweep % p.project_every == 0;
-                if (!update_vertex_df<MODE, G>(p, pub, after ? proj : pub, at ? proj : nullptr, v, ring, nring, code,
-                                               deg, sweep, stage, pos))
-                    return;
+            }
+            if (++r == D) {
+                r = 0;
+                ++tq;
             }
         }
     }
     if (csg::grid_barrier(p.ctl, phase, p.timeout_ns, barrier_id++)) return;
-    const unsigned long long* result =
-        (p.project_every > 0 && last >= 1 && last % p.project_every == 0) ? proj : pub;
+    const int result = (p.project_every > 0 && last >= 1 && last % p.project_every == 0) ? kProjected : 0;
     for (int v = tid; v < p.n; v += nthreads) {
         float* q = static_cast<float*>(p.points) + 3LL * v;
-        for (int k = 0; k < 3; ++k) q[k] = word_value(ld_word(result + 4LL * v + k));
+        const float4 x = quad_point(ld_quad(words + static_cast<long long>(kWordPitch) * v + result));
+        q[0] = x.x;
+        q[1] = x.y;
+        q[2] = x.z;
     }
 }
 
 constexpr size_t kMaxTopologySmem = 200 * 1024;
+constexpr size_t kMaxDataflowSmem = 216 * 1024;  // the staged face terms are part of it
 
 template <int MODE, int G, bool SMEM>
 int launch_variant(ArealParams params, int n_ctas, int threads, size_t smem, cudaStream_t stream) {
@@ -825,10 +865,15 @@ int launch(ArealParams params, int n_ctas, int threads, cudaStream_t stream) {
     if constexpr (MODE != CSG_ARITH_FP64) {
         // a ring has at most 2 max_degree + 1 vertices
         if (params.allow_dataflow && params.max_degree > 0 && 2 * params.max_degree + 1 <= kRingMax) {
-            const size_t smem = sizeof(float3) * (threads / 32) * (32 / G) * kRingMax +
-                                static_cast<size_t>(params.nloc_max) * sizeof(int) * (kRingMax + params.max_degree + 4) +
+            const long long pe = params.project_every;
+            params.epoch_magic = pe > 1 && pe * params.iterations < (1LL << 32)
+                                     ? static_cast<unsigned int>(((1LL << 32) + pe - 1) / pe)
+                                     : 0u;
+            const size_t cap = dataflow_ring_capacity(params.max_degree, G);
+            const size_t smem = (threads / 32) * 4 * kStagePitch * sizeof(double) + sizeof(float4) * (threads / G) * cap +
+                                static_cast<size_t>(params.nloc_max) * sizeof(int) * (cap + params.max_degree + 4) +
                                 sizeof(int) * (2 * static_cast<size_t>(params.n_levels) + params.stride);
-            if (smem <= kMaxTopologySmem) return launch_dataflow<MODE, G>(params, n_ctas, threads, smem, stream);
+            if (smem <= kMaxDataflowSmem) return launch_dataflow<MODE, G>(params, n_ctas, threads, smem, stream);
         }
     }
     const size_t smem = static_cast<size_t>(params.nloc_max) * (params.max_degree * sizeof(int4) + 2 * sizeof(int)) +
@@ -872,9 +917,8 @@ extern "C" {
 size_t csg_areal_scratch_bytes(int n_vertices, int arithmetic) {
     if (n_vertices < 1 || (arithmetic != CSG_ARITH_CAT && arithmetic != CSG_ARITH_FP32 && arithmetic != CSG_ARITH_FP64))
         return 0;
-    // float64: a double4 working copy; float32 modes: four published 8-byte
-    // words per vertex and four projected ones (the dataflow form; the barrier
-    // form uses the first 16 bytes per vertex)
+    // float64: a double4 working copy; float32 modes: the dataflow form's kWordPitch
+    // quads per vertex (the barrier form uses the first 16 bytes per vertex)
     return sizeof(csg::Control) + align256(64 * static_cast<size_t>(n_vertices));
 }
 

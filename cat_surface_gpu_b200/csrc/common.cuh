@@ -117,6 +117,37 @@ __device__ __forceinline__ unsigned long long make_word(float x, unsigned int ve
 __device__ __forceinline__ float word_value(unsigned long long w) { return __uint_as_float(static_cast<unsigned>(w)); }
 __device__ __forceinline__ unsigned int word_version(unsigned long long w) { return static_cast<unsigned>(w >> 32); }
 
+// The same in one 16-byte word: two 8-byte halves, of which the last four bytes
+// are the version.  A .b128 access with .relaxed is one scalar memory operation
+// (PTX ISA 8.3, sm_70 and later), so the three coordinates of a point and its
+// version are read and written together: one load per polled member and one
+// store per update where separate words take three of each.
+struct alignas(16) Quad {
+    unsigned long long lo, hi;
+};
+__device__ __forceinline__ Quad ld_quad(const Quad* p) {
+    Quad q;
+    asm volatile("{\n\t.reg .b128 w;\n\tld.relaxed.gpu.global.b128 w, [%2];\n\tmov.b128 {%0, %1}, w;\n\t}"
+                 : "=l"(q.lo), "=l"(q.hi)
+                 : "l"(p)
+                 : "memory");
+    return q;
+}
+__device__ __forceinline__ void st_quad(Quad* p, const Quad& q) {
+    asm volatile("{\n\t.reg .b128 w;\n\tmov.b128 w, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], w;\n\t}" ::"l"(p),
+                 "l"(q.lo), "l"(q.hi)
+                 : "memory");
+}
+__device__ __forceinline__ Quad make_quad(float x, float y, float z, unsigned int version) {
+    return {(static_cast<unsigned long long>(__float_as_uint(y)) << 32) | __float_as_uint(x),
+            (static_cast<unsigned long long>(version) << 32) | __float_as_uint(z)};
+}
+__device__ __forceinline__ unsigned int quad_version(const Quad& q) { return static_cast<unsigned>(q.hi >> 32); }
+__device__ __forceinline__ float4 quad_point(const Quad& q) {
+    return make_float4(__uint_as_float(static_cast<unsigned>(q.lo)), __uint_as_float(static_cast<unsigned>(q.lo >> 32)),
+                       __uint_as_float(static_cast<unsigned>(q.hi)), 0.0f);
+}
+
 // Work distribution of a dataflow kernel with few items per step (the
 // coloured SOR): the items of successive wavefront steps are dealt to a CTA's
 // groups round-robin without restarting at group 0 each step: item k of a
@@ -130,13 +161,15 @@ __device__ __forceinline__ int dealt_first(int rot, int warp_first_group, int gr
     return -(((rot - warp_first_group) % groups + groups) % groups);
 }
 
-// Bounded wait of one warp in a dataflow kernel: lane 0 checks the clock and
-// the status word every 64 polls; true (the same in every lane) means give up
-// -- the status is CSG_ERR_TIMEOUT (recorded here) or another CTA's error.
+// Bounded wait of one warp in a dataflow kernel: every 64 polls (`polls` is the
+// same in every lane) lane 0 checks the clock and the status word; true (the
+// same in every lane) means give up -- the status is CSG_ERR_TIMEOUT (recorded
+// here) or another CTA's error.
 __device__ __forceinline__ bool warp_wait_expired(Control* ctl, unsigned long long timeout_ns, unsigned int& polls,
                                                   unsigned long long& start) {
+    if (((++polls) & 63u) != 0u) return false;
     int expired = 0;
-    if ((threadIdx.x & 31) == 0 && ((++polls) & 63u) == 0u) {
+    if ((threadIdx.x & 31) == 0) {
         const unsigned long long now = global_timer_ns();
         if (start == 0) start = now;
         if (ld_relaxed_gpu(&ctl->status) != CSG_OK) {

@@ -230,11 +230,12 @@ def _resolve_dtype(dtype: str | torch.dtype) -> torch.dtype:
 def sweep_launch_default(device, arithmetic: str = "cat") -> dict:
     """Launch shape of the sweep kernel: 2 CTAs x 384 threads per SM, 8 lanes per vertex (float32 modes).
 
-    Measured on the 61,442-vertex hull (4,999 sweeps, dataflow form): 76.1 ms,
-    against 97.5 ms at 1 x 512 and 78.6 ms at 3 x 256; every shape gives
-    identical results (``launch="auto"`` times the candidates instead).  The
-    plain float32 mode (more registers per thread) and the float64 mode
-    (barrier form) keep 1 x 512.
+    Measured on the 61,442-vertex hull (999 sweeps, dataflow form): 10.33 ms,
+    against 16.15 ms at 1 x 512 (a step's vertices need a second round of its
+    groups) and 10.40 ms at 3 x 256; at 10,242 vertices every shape lies within
+    8.3-8.9 ms.  Every shape gives identical results (``launch="auto"`` times the
+    candidates instead).  The plain float32 mode and the float64 mode (barrier
+    form) keep 1 x 512.
     """
 
     from .autotune import sm_count

@@ -1,0 +1,54 @@
+"""The dataflow sweeps' published words at the sizes where their paths change.
+
+Meshes whose vertices have more ring members or more faces than a group has
+lanes, projection periods that take each form of the epoch test, and every
+lane count: all bit-identical to the oracle's sequential restatement.
+"""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+import torch
+
+from cat_surface_gpu_b200 import synthetic
+from oracle import areal as oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def _mesh(kind):
+    """(vertices, faces): closed, with an apex of nine faces, or with faces listed more than once."""
+
+    vertices, faces = synthetic.folded_icosphere(2, seed=5)
+    if kind == "apex":  # a vertex of nine faces (ten ring members): a fan over a nine-sided hole
+        angle = 2 * np.pi * np.arange(9) / 9
+        rim = np.stack((np.cos(angle), np.sin(angle), 0.1 * np.sin(3 * angle)), 1)
+        vertices = np.concatenate(([[0.1, 0.0, 1.0], [0.0, 0.1, -1.0]], rim)) * 40.0
+        turn = np.arange(9)
+        up = np.stack((np.zeros(9), 2 + turn, 2 + (turn + 1) % 9), 1)
+        down = np.stack((np.ones(9), 2 + (turn + 1) % 9, 2 + turn), 1)
+        faces = np.concatenate((up, down))
+    elif kind == "repeated":  # nine faces round vertices with seven ring members
+        at = int(np.bincount(faces.reshape(-1)).argmax())
+        faces = np.concatenate((faces, faces[(faces == at).any(axis=1)][:3]))
+    return np.asarray(vertices, dtype=np.float32), np.ascontiguousarray(faces, dtype=np.int32)
+
+
+@pytest.mark.parametrize("kind", ["closed", "apex", "repeated"])
+@pytest.mark.parametrize("lanes", [4, 8, 16])
+@pytest.mark.parametrize("arithmetic", ["cat", "fp32"])
+@pytest.mark.parametrize("project_every", [0, 1, 2, 7, 2**27])
+def test_sweeps_equal_the_oracle(native_library, kind, lanes, arithmetic, project_every):
+    from cat_surface_gpu_b200.gifti import GiftiMesh
+    from cat_surface_gpu_b200.surf2sphere import Surf2SphereTopology, run_areal_smoothing_cuda
+
+    vertices, faces = _mesh(kind)
+    radius = float(np.sqrt(np.max(np.sum(vertices.astype(np.float64) ** 2, axis=1))))
+    topology = Surf2SphereTopology.plan_only(GiftiMesh(vertices, faces))
+    launch = {"n_ctas": 3, "threads_per_cta": 64, "lanes_per_vertex": lanes}
+    got, _ = run_areal_smoothing_cuda(vertices, faces, topology, iterations=35, project_every=project_every,
+                                      radius=radius, arithmetic=arithmetic, launch=launch)
+    want = oracle.areal_sweeps(vertices, faces, iterations=35, project_every=project_every, radius=radius,
+                               arithmetic=arithmetic)
+    np.testing.assert_array_equal(got, want)
