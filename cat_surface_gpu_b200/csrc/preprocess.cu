@@ -82,7 +82,7 @@ struct Segment {
 
 struct PassParams {
     float4* work;
-    unsigned long long* pub;  // dataflow form: 4 versioned words per vertex
+    csg::Quad* pub;  // dataflow form: a published word per vertex
     const int* nb_off;
     const int* nb;
     const unsigned char* selected;
@@ -278,101 +278,140 @@ __global__ void __launch_bounds__(512) smooth_passes_kernel(PassParams p) {
 
 // ---------------------------------------------------------------- dataflow form
 //
-// The same passes without a grid barrier per wavefront step: each coordinate
-// is published as a versioned word (csg::make_word; version = passes the
-// vertex has completed in this launch).  Pass k of vertex v needs its
-// lower-index neighbours at version k + 1, its higher-index neighbours and
-// itself at version k, and none of them can be further ahead (a neighbour's
-// next pass needs v's pass k), so the words that show those versions hold
-// exactly the values the sequential order reads.  A group polls the ring (v
-// and its 1-ring, one round trip per poll), stages the positions in shared
-// memory and applies the segment's update; every vertex publishes every pass
-// (unchanged when it does not move).  Grid barriers remain at the start (the
-// words are written from `work`) and at the end (`work` is written back).
+// The same passes without a grid barrier per wavefront step: each vertex is
+// published as one 16-byte word (csg::make_quad; version = passes the vertex has
+// completed in this launch), the words kWordPitch quads apart (see the sweeps:
+// no two share 64 bytes).  Pass k of vertex v needs its lower-index neighbours at
+// version k + 1, its higher-index neighbours and itself at version k, and none of
+// them can be further ahead (a neighbour's next pass needs v's pass k), so the
+// words that show those versions hold exactly the values the sequential order
+// reads.  A group polls the ring (v and its 1-ring, one round trip per poll; a
+// lane that has its member's version stops loading) and applies the segment's
+// update; every vertex publishes every pass (unchanged when it does not move).
+// Grid barriers remain at the start (the words are written from `work`) and at
+// the end (`work` is written back).
+
+using csg::Quad;
 
 constexpr int kPRing = 17;  // the vertex and at most 16 neighbours
+constexpr int kWordPitch = 4;
+constexpr int kStagePitch = 34;  // doubles per staged row: the four rows of a warp start on different banks
 
+// Load this lane's MEMBERS ring members (k = glane, glane + G, ...; `first` is the first
+// one's vertex, -1 for none) until each shows the version the pass needs.
+template <int MEMBERS, int G>
+__device__ __forceinline__ bool poll_ring(const PassParams& p, int v, int first, const int* ring, int nring,
+                                          unsigned int pass, Quad (&w)[MEMBERS]) {
+    const int glane = threadIdx.x & (G - 1);
+    const Quad* from[MEMBERS];
+    unsigned int need[MEMBERS];
+#pragma unroll
+    for (int q = 0; q < MEMBERS; ++q) {
+        const int u = q == 0 ? first : (glane + q * G < nring ? ring[glane + q * G] : -1);
+        need[q] = u < v ? pass + 1 : pass;  // the vertex itself: pass
+        w[q] = Quad{0, static_cast<unsigned long long>(need[q]) << 32};
+        from[q] = p.pub + static_cast<long long>(kWordPitch) * u;
+        if (u >= 0) w[q] = csg::ld_quad(from[q]);
+    }
+    unsigned int polls = 0;
+    unsigned long long start = 0;
+    while (true) {
+        bool want = false;
+#pragma unroll
+        for (int q = 0; q < MEMBERS; ++q) want = want || csg::quad_version(w[q]) != need[q];
+        if (!__any_sync(kFull, want)) return true;
+        if (csg::warp_wait_expired(p.ctl, p.timeout_ns, polls, start)) return false;
+#pragma unroll
+        for (int q = 0; q < MEMBERS; ++q)
+            if (csg::quad_version(w[q]) != need[q]) w[q] = csg::ld_quad(from[q]);
+    }
+}
+
+// Stage one neighbour's terms (L1 distance d, d q when d > 0; zeros without a neighbour).
+__device__ __forceinline__ void stage_neighbour(bool has, const float4& q, const double o[3], int lane,
+                                                double (*stage)[kStagePitch]) {
+    double d = 0.0, dx = 0.0, dy = 0.0, dz = 0.0;
+    if (has) {
+        const double qx = q.x, qy = q.y, qz = q.z;
+        d = __dadd_rn(__dadd_rn(fabs(__dsub_rn(qx, o[0])), fabs(__dsub_rn(qy, o[1]))), fabs(__dsub_rn(qz, o[2])));
+        if (d > 0.0) {
+            dx = __dmul_rn(d, qx);
+            dy = __dmul_rn(d, qy);
+            dz = __dmul_rn(d, qz);
+        }
+    }
+    stage[0][lane] = d;
+    stage[1][lane] = dx;
+    stage[2][lane] = dy;
+    stage[3][lane] = dz;
+    __syncwarp();
+}
+
+// The total distance and one coordinate's weighted sum of G staged terms, in lane order.
+// Lanes without a neighbour staged +0, which leaves sums that started from +0 unchanged.
 template <int G>
-__device__ __forceinline__ bool pass_vertex_df(const PassParams& p, int v, const int* ring, int nring, int sg,
-                                               unsigned int pass, double (*stage)[32], float3* pos) {
-    constexpr int kQ = (kPRing + G - 1) / G;
+__device__ __forceinline__ void add_neighbours(const double (*stage)[kStagePitch], int comp, int gbase, double& total,
+                                               double& wsum) {
+    const double2* ta = reinterpret_cast<const double2*>(&stage[0][gbase]);
+    const double2* tm = reinterpret_cast<const double2*>(&stage[1 + comp][gbase]);
+#pragma unroll
+    for (int q = 0; q < G / 2; ++q) {
+        const double2 x = ta[q], y = tm[q];
+        total = __dadd_rn(__dadd_rn(total, x.x), x.y);
+        wsum = __dadd_rn(__dadd_rn(wsum, y.x), y.y);
+    }
+}
+
+// One pass of vertex v (groups without one: v < 0, nring 0) by a group of G lanes; all 32
+// lanes call it.  Rings of at most G members, the vertex's own first, stay in the lanes'
+// registers; longer ones go through `pos`.
+template <int G>
+__device__ __forceinline__ bool pass_vertex_df(const PassParams& p, int v, const int* ring, int nring, bool selected,
+                                               unsigned int pass, double (*stage)[kStagePitch], float4* pos) {
     const int lane = threadIdx.x & 31;
     const int glane = lane & (G - 1);
     const int gbase = lane & ~(G - 1);
+    const int first = glane < nring ? ring[glane] : -1;
+    int sg = 0;  // the segment this pass lies in
+    for (int k = 1; k < p.n_segments; ++k) sg += pass >= static_cast<unsigned int>(p.seg[k].first_pass);
     const int kind = p.seg[sg].kind;
     const double strength = p.seg[sg].value;
-    if (v < 0) nring = 0;
-    unsigned int polls = 0;
-    unsigned long long start = 0;
-    int who[kQ];
-#pragma unroll
-    for (int q = 0; q < kQ; ++q) {
-        const int k = glane + q * G;
-        who[q] = k < nring ? ring[k] : -1;
-    }
-    while (true) {
-        unsigned long long w[kQ][3];
-#pragma unroll
-        for (int q = 0; q < kQ; ++q)
-            if (who[q] >= 0)
-#pragma unroll
-                for (int k = 0; k < 3; ++k) w[q][k] = csg::ld_word(p.pub + 4LL * who[q] + k);
-        bool ok = true;
-#pragma unroll
-        for (int q = 0; q < kQ; ++q)
-            if (who[q] >= 0) {
-                const unsigned int need = who[q] < v ? pass + 1 : pass;  // the vertex itself: pass
-                ok = ok && csg::word_version(w[q][0]) == need && csg::word_version(w[q][1]) == need &&
-                     csg::word_version(w[q][2]) == need;
-                pos[glane + q * G] = make_float3(csg::word_value(w[q][0]), csg::word_value(w[q][1]),
-                                                 csg::word_value(w[q][2]));
-            }
-        if (__all_sync(kFull, ok)) break;
-        if (csg::warp_wait_expired(p.ctl, p.timeout_ns, polls, start)) return false;
-    }
-    __syncwarp();
-    int deg = nring > 0 ? nring - 1 : 0;
-    const bool active = v >= 0 && kind != kInflate && deg > 1 && (kind == kSmoothAll || p.selected[v]);
-    if (!active) deg = 0;
-    const int wdeg = __reduce_max_sync(kFull, deg);
-    double o[3] = {0.0, 0.0, 0.0};
-    if (v >= 0) {
-        o[0] = pos[0].x;
-        o[1] = pos[0].y;
-        o[2] = pos[0].z;
-    }
-    double total = 0.0, wsum = 0.0;
+    const bool active = kind != kInflate && nring > 2 && (kind == kSmoothAll || selected);
     const int comp = glane < 3 ? glane : 0;
-    for (int c0 = 0; c0 < wdeg; c0 += G) {
-        const int j = c0 + glane;
-        double d = 0.0, dx = 0.0, dy = 0.0, dz = 0.0;
-        if (j < deg) {
-            const float3 q = pos[1 + j];
-            const double qx = q.x, qy = q.y, qz = q.z;
-            d = __dadd_rn(__dadd_rn(fabs(__dsub_rn(qx, o[0])), fabs(__dsub_rn(qy, o[1]))), fabs(__dsub_rn(qz, o[2])));
-            if (d > 0.0) {
-                dx = __dmul_rn(d, qx);
-                dy = __dmul_rn(d, qy);
-                dz = __dmul_rn(d, qz);
-            }
+    double total = 0.0, wsum = 0.0;
+    double o[3];
+    if (!__any_sync(kFull, nring > G)) {
+        Quad w[1];
+        if (!poll_ring<1, G>(p, v, first, ring, nring, pass, w)) return false;
+        const float4 q = csg::quad_point(w[0]);
+        o[0] = __shfl_sync(kFull, q.x, gbase);
+        o[1] = __shfl_sync(kFull, q.y, gbase);
+        o[2] = __shfl_sync(kFull, q.z, gbase);
+        if (__any_sync(kFull, active)) {
+            stage_neighbour(active && glane > 0 && glane < nring, q, o, lane, stage);
+            if (glane < 3) add_neighbours<G>(stage, comp, gbase, total, wsum);
         }
-        stage[0][lane] = d;
-        stage[1][lane] = dx;
-        stage[2][lane] = dy;
-        stage[3][lane] = dz;
-        __syncwarp();
-        if (glane < 3) {
-            const int m = min(G, deg - c0);
+    } else {
+        constexpr int kQ = (kPRing + G - 1) / G;
+        Quad w[kQ];
+        if (!poll_ring<kQ, G>(p, v, first, ring, nring, pass, w)) return false;
 #pragma unroll
-            for (int q = 0; q < G; ++q) {
-                if (q < m) {
-                    total = __dadd_rn(total, stage[0][gbase + q]);
-                    // the reference adds d q only for d > 0; the staged term is 0 otherwise
-                    if (stage[0][gbase + q] > 0.0) wsum = __dadd_rn(wsum, stage[1 + comp][gbase + q]);
-                }
-            }
-        }
+        for (int q = 0; q < kQ; ++q)
+            if (glane + q * G < nring) pos[glane + q * G] = csg::quad_point(w[q]);
         __syncwarp();
+        o[0] = o[1] = o[2] = 0.0;
+        if (v >= 0) {
+            o[0] = pos[0].x;
+            o[1] = pos[0].y;
+            o[2] = pos[0].z;
+        }
+        const int deg = active ? nring - 1 : 0;
+        for (int c0 = 0; __any_sync(kFull, c0 < deg); c0 += G) {
+            const bool has = c0 + glane < deg;
+            stage_neighbour(has, has ? pos[1 + c0 + glane] : make_float4(0.0f, 0.0f, 0.0f, 0.0f), o, lane, stage);
+            if (glane < 3) add_neighbours<G>(stage, comp, gbase, total, wsum);
+            __syncwarp();
+        }
     }
     float value = 0.0f;
     if (v >= 0 && glane < 3) {
@@ -390,58 +429,58 @@ __device__ __forceinline__ bool pass_vertex_df(const PassParams& p, int v, const
             value = static_cast<float>(o[comp]);
         }
     }
-    __syncwarp();  // every lane is done with `pos` before the next update overwrites it
-    if (v >= 0 && glane < 3) csg::st_word(p.pub + 4LL * v + glane, csg::make_word(value, pass + 1));
+    const float vy = __shfl_sync(kFull, value, gbase + 1), vz = __shfl_sync(kFull, value, gbase + 2);
+    if (v >= 0 && glane == 0)
+        csg::st_quad(p.pub + static_cast<long long>(kWordPitch) * v, csg::make_quad(value, vy, vz, pass + 1));
+    __syncwarp();  // every lane is done with `pos` and `stage` before the next pass overwrites them
     return true;
 }
 
 template <int G>
 __global__ void __launch_bounds__(512) smooth_passes_df(PassParams p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ double stage_all[512 / 32][4][32];
-    double (*stage)[32] = stage_all[threadIdx.x >> 5];
     const int c = blockIdx.x, nc = gridDim.x;
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
     const int groups = blockDim.x / G;
     const int warp_first_group = (threadIdx.x >> 5) * (32 / G);
     const int my_group = (threadIdx.x & 31) / G;
     const int L = p.n_levels, D = p.stride;
-    // shared-memory image: per warp, kPRing staged positions per group; per
-    // owned vertex its ring (itself, then its 1-ring), ring size, id and level;
-    // per level the owned range
-    float3* pos = reinterpret_cast<float3*>(smem_raw) + ((threadIdx.x >> 5) * (32 / G) + my_group) * kPRing;
-    int* lring = reinterpret_cast<int*>(reinterpret_cast<float3*>(smem_raw) + (blockDim.x / G) * kPRing);
-    int* lnring = lring + p.nloc_max * kPRing;
-    int* lvid = lnring + p.nloc_max;
-    int* llev = lvid + p.nloc_max;
-    int* lbeg = llev + p.nloc_max;
+    const int cap = p.max_degree + 1;
+    // shared-memory image: per warp the staged terms; per group `cap` staged
+    // positions; per owned vertex its description (id, ring size, level / D,
+    // selected) and ring (itself, then its 1-ring); per level the owned range
+    double (*stage)[kStagePitch] = reinterpret_cast<double (*)[kStagePitch]>(smem_raw) + 4 * (threadIdx.x >> 5);
+    float4* pos0 = reinterpret_cast<float4*>(smem_raw + (blockDim.x / 32) * 4 * kStagePitch * sizeof(double));
+    float4* pos = pos0 + (threadIdx.x / G) * cap;
+    int4* lmeta = reinterpret_cast<int4*>(pos0 + (blockDim.x / G) * cap);
+    int* lring = reinterpret_cast<int*>(lmeta + p.nloc_max);
+    int* lbeg = lring + p.nloc_max * cap;
     int* lend = lbeg + L;
     const int nloc = owned_below(p.n, c, nc);
     for (int i = threadIdx.x; i < nloc; i += blockDim.x) {
         const int v = __ldg(p.order + c + i * nc);
         const int b = __ldg(p.nb_off + v);
         int d = __ldg(p.nb_off + v + 1) - b;
-        if (d > p.max_degree || d + 1 > kPRing) {  // a ring longer than the caller's max_degree: report it
+        if (d > p.max_degree) {  // a ring longer than the caller's max_degree: report it
             if (atomicCAS(&p.ctl->status, CSG_OK, CSG_ERR_ARG) == CSG_OK) p.ctl->where = -1;
-            d = min(d, kPRing - 1);
+            d = p.max_degree;
         }
-        int* ring = lring + i * kPRing;
+        int* ring = lring + i * cap;
         ring[0] = v;
         for (int j = 0; j < d; ++j) ring[1 + j] = __ldg(p.nb + b + j);
-        lnring[i] = d + 1;
-        lvid[i] = v;
+        lmeta[i].x = v;
+        lmeta[i].y = d + 1;
+        lmeta[i].w = p.selected[v];  // written before this launch, or not read by its segments
     }
     for (int l = threadIdx.x; l < L; l += blockDim.x) {
         const int lb = owned_below(__ldg(p.level_begin + l), c, nc), le = owned_below(__ldg(p.level_end + l), c, nc);
         lbeg[l] = lb;
         lend[l] = le;
-        for (int i = lb; i < le; ++i) llev[i] = l;
+        for (int i = lb; i < le; ++i) lmeta[i].z = l / D;
     }
     for (int v = tid; v < p.n; v += nthreads) {
         const float4 q = ld4(p.work, v);
-        csg::st_word(p.pub + 4LL * v, csg::make_word(q.x, 0u));
-        csg::st_word(p.pub + 4LL * v + 1, csg::make_word(q.y, 0u));
-        csg::st_word(p.pub + 4LL * v + 2, csg::make_word(q.z, 0u));
+        csg::st_quad(p.pub + static_cast<long long>(kWordPitch) * v, csg::make_quad(q.x, q.y, q.z, 0u));
     }
     unsigned int phase = 0;
     int barrier_id = 0;
@@ -449,44 +488,30 @@ __global__ void __launch_bounds__(512) smooth_passes_df(PassParams p) {
     if (csg::ld_relaxed_gpu(&p.ctl->status) != CSG_OK) return;  // a ring overflow: same answer in every CTA
     const int span = (p.passes - 1) * D;  // host guarantees span + L < 2^31
     const int nsteps = span + L;
-    int r = 0;
-    for (int t = 0; t < nsteps; ++t, r = (r + 1 == D) ? 0 : r + 1) {
+    const int top = (L - 1) % D;
+    int r = 0, tq = 0;  // t mod D, t / D
+    for (int t = 0; t < nsteps; ++t) {
         int lo = t - span;
         if (lo < r) lo = r;
-        const int hi = t < L ? t : (L - 1) - ((L - 1 - r) % D + D) % D;
-        if (hi < lo) continue;
-        const int i0 = lbeg[lo], i1 = lend[hi];
-        int ib[kMaxSegments];
-#pragma unroll
-        for (int k = 1; k < kMaxSegments; ++k) {
-            ib[k] = 0;
-            if (k < p.n_segments) {
-                const int m = t - p.seg[k].first_pass * D;
-                ib[k] = m < lo ? i0 : (m >= hi ? i1 : lend[m]);
+        const int hi = t < L ? t : L - 1 - (top - r + (r > top ? D : 0));  // the top level of t's residue
+        if (hi >= lo) {
+            const int i0 = lbeg[lo], i1 = lend[hi];
+            for (int base = i0 + warp_first_group; base < i1; base += groups) {
+                const int i = base + my_group;
+                int4 m = make_int4(-1, 0, 0, 0);
+                if (i < i1) m = lmeta[i];
+                const unsigned int pass = static_cast<unsigned int>(tq - m.z);  // t and the level agree mod D
+                if (!pass_vertex_df<G>(p, m.x, lring + i * cap, m.y, m.w != 0, pass, stage, pos)) return;
             }
         }
-        for (int base = i0 + warp_first_group; base < i1; base += groups) {
-            const int i = base + my_group;
-            int v = -1, nring = 0, sg = 0;
-            unsigned int pass = 0;
-            const int* ring = nullptr;
-            if (i < i1) {
-                v = lvid[i];
-                nring = lnring[i];
-                ring = lring + i * kPRing;
-                pass = static_cast<unsigned int>((t - llev[i]) / D);
-#pragma unroll
-                for (int k = 1; k < kMaxSegments; ++k) sg += i < ib[k];
-            }
-            if (!pass_vertex_df<G>(p, v, ring, nring, sg, pass, stage, pos)) return;
+        if (++r == D) {
+            r = 0;
+            ++tq;
         }
     }
     if (csg::grid_barrier(p.ctl, phase, p.timeout_ns, barrier_id++)) return;
-    for (int v = tid; v < p.n; v += nthreads) {
-        const unsigned long long* w = p.pub + 4LL * v;
-        __stcg(p.work + v, make_float4(csg::word_value(csg::ld_word(w)), csg::word_value(csg::ld_word(w + 1)),
-                                       csg::word_value(csg::ld_word(w + 2)), 0.0f));
-    }
+    for (int v = tid; v < p.n; v += nthreads)
+        __stcg(p.work + v, csg::quad_point(csg::ld_quad(p.pub + static_cast<long long>(kWordPitch) * v)));
 }
 
 // ---------------------------------------------------------------- per-stage steps
@@ -709,7 +734,7 @@ Layout layout(int n, int nf) {
     const size_t runs = (static_cast<size_t>(n > nf ? n : nf) + kBlockSum - 1) / kBlockSum;
     L.ctl = take(sizeof(csg::Control));
     L.work = take(16ULL * n);
-    L.pub = take(32ULL * n);
+    L.pub = take(64ULL * n);  // kWordPitch quads per vertex
     L.ref = take(16ULL * n);
     L.area = take(8ULL * nf);
     L.va_ref = take(8ULL * n);
@@ -723,6 +748,7 @@ Layout layout(int n, int nf) {
 }
 
 constexpr size_t kMaxTopologySmem = 160 * 1024;
+constexpr size_t kMaxDataflowSmem = 176 * 1024;  // the staged terms are part of it
 
 template <int G, bool SMEM>
 int launch_variant(const PassParams& params, int n_ctas, int threads, size_t smem, cudaStream_t s) {
@@ -770,10 +796,11 @@ int launch_passes(PassParams params, int n_ctas, int threads, cudaStream_t s) {
     if (n_ctas <= 0) n_ctas = sms;
     params.nloc_max = (params.n + n_ctas - 1) / n_ctas;
     if (params.max_degree > 0 && params.max_degree + 1 <= kPRing) {
-        const size_t smem = sizeof(float3) * (threads / G) * kPRing +
-                            sizeof(int) * (static_cast<size_t>(params.nloc_max) * (kPRing + 3) +
+        const size_t cap = static_cast<size_t>(params.max_degree) + 1;
+        const size_t smem = (threads / 32) * 4 * kStagePitch * sizeof(double) + sizeof(float4) * (threads / G) * cap +
+                            sizeof(int) * (static_cast<size_t>(params.nloc_max) * (cap + 4) +
                                            2 * static_cast<size_t>(params.n_levels));
-        if (smem <= kMaxTopologySmem) return launch_dataflow<G>(params, n_ctas, threads, smem, s);
+        if (smem <= kMaxDataflowSmem) return launch_dataflow<G>(params, n_ctas, threads, smem, s);
     }
     const size_t smem = sizeof(int) * (static_cast<size_t>(params.nloc_max) * (params.max_degree + 2) +
                                        2 * static_cast<size_t>(params.n_levels));
@@ -878,7 +905,7 @@ int csg_surf2sphere_preprocess(float* points, int n, const int32_t* faces, int n
     (csg::note_launch(), k_pack<<<blocks(n, kThreads), kThreads, 0, s>>>(points, work, n));
     PassQueue q{};
     q.p.work = work;
-    q.p.pub = reinterpret_cast<unsigned long long*>(base + L.pub);
+    q.p.pub = reinterpret_cast<csg::Quad*>(base + L.pub);
     q.p.nb_off = nb_off;
     q.p.nb = nb;
     q.p.selected = sel;

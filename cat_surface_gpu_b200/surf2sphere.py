@@ -444,9 +444,9 @@ def run_areal_smoothing_cuda(
 def preprocess_launch_default(device) -> dict:
     """Launch shape of the stages 1-5 pass kernel: 2 CTAs x 384 threads per SM, 8 lanes per vertex.
 
-    Measured on the 61,442-vertex hull (stages 1-5, dataflow form): 49.2 ms,
-    against 52.0 ms at 1 x 512 and 49.5 ms at 3 x 256; every shape gives
-    identical results.
+    Measured on the 61,442-vertex hull (stages 1-5, dataflow form): 31.1 ms,
+    against 34.2 ms at 1 x 512, 31.0 ms at 3 x 256 and 30.4 ms at 4 x 192;
+    every shape gives identical results.
     """
 
     from .autotune import sm_count

@@ -52,3 +52,22 @@ def test_sweeps_equal_the_oracle(native_library, kind, lanes, arithmetic, projec
     want = oracle.areal_sweeps(vertices, faces, iterations=35, project_every=project_every, radius=radius,
                                arithmetic=arithmetic)
     np.testing.assert_array_equal(got, want)
+
+
+@pytest.mark.parametrize("kind", ["closed", "apex"])
+@pytest.mark.parametrize("lanes", [4, 8, 16])
+@pytest.mark.parametrize("stop_at", [1, 2, 3])
+def test_stage_passes_equal_the_oracle(native_library, kind, lanes, stop_at):
+    """Rings of at most and of more members than lanes, through smoothing, inflation and selected passes."""
+
+    from cat_surface_gpu_b200.gifti import GiftiMesh
+    from cat_surface_gpu_b200.surf2sphere import Surf2SphereTopology, run_surf2sphere_preprocess_cuda
+    from oracle import preprocess as oracle_pre
+
+    vertices, faces = _mesh(kind)
+    topology = Surf2SphereTopology.plan_only(GiftiMesh(vertices, faces))
+    launch = {"n_ctas": 3, "threads_per_cta": 64, "lanes_per_vertex": lanes}
+    got, _ = run_surf2sphere_preprocess_cuda(vertices, faces, topology, stop_at=stop_at, desired_surface_area=1.0,
+                                             launch=launch)
+    want = oracle_pre.preprocess(vertices, faces, stop_at=stop_at)
+    np.testing.assert_array_equal(got, want)
