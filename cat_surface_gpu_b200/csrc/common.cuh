@@ -148,6 +148,31 @@ __device__ __forceinline__ float4 quad_point(const Quad& q) {
                        __uint_as_float(static_cast<unsigned>(q.hi)), 0.0f);
 }
 
+// x[0] + x[1] + ... + x[n - 1] in that order, starting from 0 (the blocked sums fold their
+// partials so, whatever the launch shape), by one CTA of kOrderedThreads; the sum is valid
+// in thread 0.  `buf` holds kOrderedChunk elements.  One thread reading global memory pays
+// a round trip every few elements (960 partials: 37 us); here the CTA brings a chunk into
+// shared memory at once and the chain of additions runs from there (960: 8 us).
+constexpr int kOrderedThreads = 256, kOrderedChunk = 1024;
+template <typename T>
+__device__ __forceinline__ T ordered_sum(const T* __restrict__ x, int n, T* buf) {
+    T sum = T(0);
+    for (int base = 0; base < n; base += kOrderedChunk) {
+        const int m = min(kOrderedChunk, n - base);
+        __syncthreads();
+        for (int i = threadIdx.x; i < m; i += blockDim.x) buf[i] = x[base + i];
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            int i = 0;
+            for (; i + 8 <= m; i += 8)
+#pragma unroll
+                for (int k = 0; k < 8; ++k) sum = sum + buf[i + k];
+            for (; i < m; ++i) sum = sum + buf[i];
+        }
+    }
+    return sum;
+}
+
 // Work distribution of a dataflow kernel with few items per step (the
 // coloured SOR): the items of successive wavefront steps are dealt to a CTA's
 // groups round-robin without restarting at group 0 each step: item k of a

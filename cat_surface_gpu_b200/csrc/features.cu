@@ -99,10 +99,9 @@ __global__ void k_edge_sum(const T* __restrict__ v, const int* __restrict__ face
 }
 
 __global__ void k_sum_partials(const double* __restrict__ partial, int n, double* __restrict__ out) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    double s = 0.0;
-    for (int i = 0; i < n; ++i) s = s + partial[i];
-    out[0] = s;
+    __shared__ double buf[csg::kOrderedChunk];
+    const double s = csg::ordered_sum(partial, n, buf);
+    if (threadIdx.x == 0) out[0] = s;
 }
 
 // smooth_geometry (372-388), every iteration in one cooperative launch:
@@ -366,17 +365,29 @@ __global__ void k_minmax_apply(const double* __restrict__ v, int n, const double
                                double* __restrict__ out) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const long long base = static_cast<long long>(blockIdx.y) * n;
-    __shared__ double lo, hi;
-    if (threadIdx.x == 0) {
-        double a = INFINITY, b = -INFINITY;
-        for (int k = 0; k < nblocks; ++k) {
-            a = fmin(a, partial[2 * (static_cast<long long>(blockIdx.y) * nblocks + k)]);
-            b = fmax(b, partial[2 * (static_cast<long long>(blockIdx.y) * nblocks + k) + 1]);
-        }
-        lo = a;
-        hi = b;
+    // every CTA folds the row's partials itself, all threads at once (the extremes do not depend on the order)
+    __shared__ double mn[kThreads / 32], mx[kThreads / 32];
+    const double* row = partial + 2 * static_cast<long long>(blockIdx.y) * nblocks;
+    double a = INFINITY, b = -INFINITY;
+    for (int k = threadIdx.x; k < nblocks; k += blockDim.x) {
+        a = fmin(a, row[2 * k]);
+        b = fmax(b, row[2 * k + 1]);
+    }
+    for (int off = 16; off >= 1; off >>= 1) {
+        a = fmin(a, __shfl_xor_sync(0xffffffffu, a, off));
+        b = fmax(b, __shfl_xor_sync(0xffffffffu, b, off));
+    }
+    if ((threadIdx.x & 31) == 0) {
+        mn[threadIdx.x >> 5] = a;
+        mx[threadIdx.x >> 5] = b;
     }
     __syncthreads();
+    double lo = mn[0], hi = mx[0];
+#pragma unroll
+    for (int k = 1; k < kThreads / 32; ++k) {
+        lo = fmin(lo, mn[k]);
+        hi = fmax(hi, mx[k]);
+    }
     if (i < n) out[base + i] = (v[base + i] - lo) / (hi - lo);
 }
 
@@ -442,7 +453,7 @@ int csg_feature_edge_sum(int dtype, int n_faces, const int32_t* faces, const voi
         (csg::note_launch(), k_edge_sum<float><<<nb, kThreads, 0, s>>>(static_cast<const float*>(vertices), faces, n_faces, partial));
     else
         (csg::note_launch(), k_edge_sum<double><<<nb, kThreads, 0, s>>>(static_cast<const double*>(vertices), faces, n_faces, partial));
-    (csg::note_launch(), k_sum_partials<<<1, 32, 0, s>>>(partial, static_cast<int>(nb), out_sum));
+    (csg::note_launch(), k_sum_partials<<<1, csg::kOrderedThreads, 0, s>>>(partial, static_cast<int>(nb), out_sum));
     CSG_CUDA_CHECK(cudaGetLastError());
     return CSG_OK;
 }
