@@ -533,7 +533,7 @@ __global__ void k_unpack(const float4* __restrict__ work, float* __restrict__ po
 // A run's terms are brought into shared memory by a warp (coalesced, all in flight) and
 // added from there in order by one lane per sum: a thread that walks its run in global
 // memory pays the round trips one after another (61,442 vertices, per call: sums of face
-// areas 43 -> 4 us, stage partials 95 -> 7 us, their fold 60 -> 6 us).
+// areas 43 -> 5 us, stage partials 95 -> 17 us, their fold 60 -> 11 us).
 constexpr int kRunWarps = 4;  // runs (one warp each) of a CTA
 
 // ref = work; per run of kBlockSum vertices: coordinate sums, min, max.
