@@ -99,29 +99,11 @@ __device__ __forceinline__ bool grid_barrier(Control* ctl, unsigned int& phase, 
     return s_abort != 0;
 }
 
-// Versioned words of the dataflow kernels: a float32 value and the number of
-// updates it belongs to in one 8-byte word.  Aligned 8-byte accesses are
-// single-copy atomic, so a relaxed load returns a value together with its own
-// version and needs no acquire ordering.
-__device__ __forceinline__ unsigned long long ld_word(const unsigned long long* p) {
-    unsigned long long v;
-    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void st_word(unsigned long long* p, unsigned long long v) {
-    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-__device__ __forceinline__ unsigned long long make_word(float x, unsigned int version) {
-    return (static_cast<unsigned long long>(version) << 32) | __float_as_uint(x);
-}
-__device__ __forceinline__ float word_value(unsigned long long w) { return __uint_as_float(static_cast<unsigned>(w)); }
-__device__ __forceinline__ unsigned int word_version(unsigned long long w) { return static_cast<unsigned>(w >> 32); }
-
-// The same in one 16-byte word: two 8-byte halves, of which the last four bytes
-// are the version.  A .b128 access with .relaxed is one scalar memory operation
-// (PTX ISA 8.3, sm_70 and later), so the three coordinates of a point and its
-// version are read and written together: one load per polled member and one
-// store per update where separate words take three of each.
+// Published words of the dataflow kernels: 16 bytes that hold a value (three
+// float32 coordinates, or a float64) and the number of updates it belongs to.  A
+// .b128 access with .relaxed is one scalar memory operation (PTX ISA 8.3, sm_70
+// and later), so a load returns a value together with its own version and needs
+// no acquire ordering.
 struct alignas(16) Quad {
     unsigned long long lo, hi;
 };
@@ -171,19 +153,6 @@ __device__ __forceinline__ T ordered_sum(const T* __restrict__ x, int n, T* buf)
         }
     }
     return sum;
-}
-
-// Work distribution of a dataflow kernel with few items per step (the
-// coloured SOR): the items of successive wavefront steps are dealt to a CTA's
-// groups round-robin without restarting at group 0 each step: item k of a
-// step goes to group (rot + k) mod groups, rot = items dealt in earlier steps
-// mod groups.  Each group still takes its items in step order (progress is
-// guaranteed as in the step-by-step form), and groups without an item in this
-// step take the next steps' items, so several steps are in flight in a CTA.
-// Returns the first item index of this warp's first group (<= 0); the warp's
-// groups then take k = first + g + j * groups, valid while 0 <= k < count.
-__device__ __forceinline__ int dealt_first(int rot, int warp_first_group, int groups) {
-    return -(((rot - warp_first_group) % groups + groups) % groups);
 }
 
 // Bounded wait of one warp in a dataflow kernel: every 64 polls (`polls` is the

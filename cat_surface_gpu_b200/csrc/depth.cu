@@ -279,7 +279,7 @@ struct SorParams {
     int max_row, nloc_max;  // shared-memory image (0: rows read from global memory)
     double relaxation;
     unsigned long long timeout_ns;
-    unsigned long long* pub;  // dataflow form: x as versioned words, 2 per (surface, vertex)
+    csg::Quad* pub;           // dataflow form: x as published words, one per (surface, vertex)
     int* level_of;            // dataflow form: the schedule level of every vertex
 };
 
@@ -426,16 +426,24 @@ __global__ void __launch_bounds__(512) k_depth_sor(SorParams p) {
 // ---------------------------------------------------------------- SOR, dataflow form
 //
 // The sweeps without a grid barrier per step, as the Surf2Sphere dataflow
-// kernels do it: x[b][v] is published as two versioned words (the low and the
-// high 32 bits of the double, each with the number of sweeps completed).  In
-// colour-major Gauss-Seidel order a neighbour u comes before v exactly when
-// level(u) < level(v) (the schedule's potential grows along that order), so
-// sweep s of v needs earlier neighbours at version s and later neighbours and
-// v itself at version s - 1, and none can be further ahead.  A group polls the
-// row's distinct columns (its ring), stages their x in shared memory, forms
-// the row sum in entry order and publishes the update.
+// kernels do it: x[b][v] is published as one 16-byte word (the double and the
+// number of sweeps completed).  In colour-major Gauss-Seidel order a neighbour u
+// comes before v exactly when level(u) < level(v) (the schedule's potential grows
+// along that order), so sweep s of v needs earlier neighbours at version s and
+// later neighbours and v itself at version s - 1, and none can be further ahead.
+// A group polls the row's distinct columns (its ring), stages their x in shared
+// memory, forms the row sum in entry order and publishes the update.
+//
+// A step has few rows per CTA (one colour of both surfaces: 92 of 40,962 x 2), so
+// the rows of successive steps are dealt to a CTA's groups round-robin without
+// restarting at group 0 each step: item k of a step goes to group (rot + k) mod
+// groups, rot = items dealt in earlier steps mod groups.  Each group still takes its
+// items in step order (the earliest unfinished row's inputs are always finished), and
+// groups without an item in this step take the next steps', so several steps are in
+// flight in a CTA.
 
-constexpr int kSRing = 16;  // the vertex and at most 15 distinct neighbours
+constexpr int kSRing = 16;    // the vertex and at most 15 distinct neighbours
+constexpr int kSRowMax = 22;  // the longest row whose columns are sure to fit the ring (seven incidences)
 
 __global__ void k_level_of(const int* __restrict__ order, const int* __restrict__ level_begin,
                            const int* __restrict__ level_end, int* __restrict__ level_of) {
@@ -445,80 +453,104 @@ __global__ void k_level_of(const int* __restrict__ order, const int* __restrict_
         level_of[order[pos]] = l;
 }
 
-__device__ __forceinline__ double words_value(unsigned long long lo, unsigned long long hi) {
-    return __hiloint2double(static_cast<int>(static_cast<unsigned>(hi)), static_cast<int>(static_cast<unsigned>(lo)));
+// The published word of x[b][v]: the double's bits and, in the other half, its version.
+// Words sit kWordPitch quads (32 bytes, a sector) apart, so polls of one row do not queue
+// behind the publication of another (two surfaces of 40,962, 1,000 sweeps: 12.2 ms; 12.5 at
+// 64 bytes; 18.3 with two 8-byte words per value, re-read until the last member arrived).
+constexpr int kWordPitch = 2;
+__device__ __forceinline__ csg::Quad make_word(double x, unsigned int version) {
+    return {static_cast<unsigned long long>(__double_as_longlong(x)), static_cast<unsigned long long>(version)};
 }
+__device__ __forceinline__ double word_value(const csg::Quad& q) { return __longlong_as_double(static_cast<long long>(q.lo)); }
 
-template <int G>
-__device__ __forceinline__ bool sor_row_df(const SorParams& p, int b, int v, const int* ring, int nring,
-                                           const unsigned char* code, const double* rval, int len, double rhs,
-                                           double diag, unsigned int s, double* ringx) {
-    constexpr int kQ = (kSRing + G - 1) / G;
-    constexpr int kE = 32 / G;  // entries per lane and block of 32
-    const int lane = threadIdx.x & 31;
-    const int glane = lane & (G - 1);
-    const int gbase = lane & ~(G - 1);
-    const unsigned long long* pub = p.pub + 2LL * p.n * b;
-    if (v < 0) {
-        nring = 0;
-        len = 0;
+// A row: vertex (-1: none), ring (sign bit: the neighbour comes first), entry codes and values.
+struct SorRow {
+    int v, nring, len;
+    unsigned int sweep;
+    const int* ring;
+    const unsigned char* code;
+    const double* val;
+    double rhs, diag;
+};
+
+// Load this lane's MEMBERS ring members until each shows the version sweep s needs, then
+// stage them.  A lane that has a member's version stops loading it.
+template <int MEMBERS, int G>
+__device__ __forceinline__ bool poll_ring(const SorParams& p, const csg::Quad* words, const SorRow& row, double* ringx) {
+    const int glane = threadIdx.x & (G - 1);
+    const csg::Quad* from[MEMBERS];
+    unsigned int need[MEMBERS];
+    csg::Quad w[MEMBERS];
+#pragma unroll
+    for (int q = 0; q < MEMBERS; ++q) {
+        const int k = glane + q * G;
+        need[q] = row.sweep - 1;
+        w[q] = csg::Quad{0, need[q]};
+        if (k < row.nring) {
+            const int u = row.ring[k];
+            if (u < 0) need[q] = row.sweep;
+            from[q] = words + static_cast<long long>(kWordPitch) * (u & 0x7fffffff);
+            w[q] = csg::ld_quad(from[q]);
+        }
     }
     unsigned int polls = 0;
     unsigned long long start = 0;
-    int who[kQ];
-    unsigned int need[kQ];
-#pragma unroll
-    for (int q = 0; q < kQ; ++q) {
-        const int k = glane + q * G;
-        who[q] = k < nring ? (ring[k] & 0x7fffffff) : -1;
-        need[q] = (k < nring && (ring[k] < 0)) ? s : s - 1;  // sign bit: the neighbour comes first
-    }
     while (true) {
-        unsigned long long w[kQ][2];
+        bool want = false;
 #pragma unroll
-        for (int q = 0; q < kQ; ++q)
-            if (who[q] >= 0) {
-                w[q][0] = csg::ld_word(pub + 2LL * who[q]);
-                w[q][1] = csg::ld_word(pub + 2LL * who[q] + 1);
-            }
-        bool ok = true;
-#pragma unroll
-        for (int q = 0; q < kQ; ++q)
-            if (who[q] >= 0) {
-                ok = ok && csg::word_version(w[q][0]) == need[q] && csg::word_version(w[q][1]) == need[q];
-                ringx[glane + q * G] = words_value(w[q][0], w[q][1]);
-            }
-        if (__all_sync(kFull, ok)) break;
+        for (int q = 0; q < MEMBERS; ++q) want = want || static_cast<unsigned int>(w[q].hi) != need[q];
+        if (!__any_sync(kFull, want)) break;
         if (csg::warp_wait_expired(p.ctl, p.timeout_ns, polls, start)) return false;
+#pragma unroll
+        for (int q = 0; q < MEMBERS; ++q)
+            if (static_cast<unsigned int>(w[q].hi) != need[q]) w[q] = csg::ld_quad(from[q]);
+    }
+#pragma unroll
+    for (int q = 0; q < MEMBERS; ++q)
+        if (glane + q * G < row.nring) ringx[glane + q * G] = word_value(w[q]);
+    return true;
+}
+
+// One row of one sweep by a group of G lanes (all 32 lanes call it).  The lanes poll the
+// row's distinct columns, multiply the entries, stage the products where the ring stood
+// and add them in entry order; entries past the row's last are staged as +0, which leaves
+// a sum that started from +0 unchanged, so the additions need no test.
+template <int G>
+__device__ __forceinline__ bool sor_row_df(const SorParams& p, csg::Quad* words, const SorRow& row, double* buf) {
+    constexpr int kNarrow = G == 4 ? 2 : 1;               // members per lane of a ring of at most eight
+    constexpr int kE = (kSRowMax + G - 1) / G;            // entries per lane
+    const int glane = threadIdx.x & (G - 1);
+    if (!__any_sync(kFull, row.nring > kNarrow * G)) {
+        if (!poll_ring<kNarrow, G>(p, words, row, buf)) return false;
+    } else {
+        if (!poll_ring<(kSRing + G - 1) / G, G>(p, words, row, buf)) return false;
     }
     __syncwarp();
-    const int wlen = __reduce_max_sync(kFull, len);
+    double prod[kE];
+#pragma unroll
+    for (int q = 0; q < kE; ++q) {
+        const int j = q * G + glane;
+        prod[q] = j < row.len ? row.val[j] * buf[row.code[j]] : 0.0;
+    }
+    const double xv = row.v >= 0 ? buf[0] : 0.0;
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < kE; ++q)
+        if (q * G + glane < kSRowMax) buf[q * G + glane] = prod[q];
+    __syncwarp();
     double sum = 0.0;
-    for (int base = 0; base < wlen; base += G * kE) {
-        double prod[kE];
+    const double2* terms = reinterpret_cast<const double2*>(buf);
 #pragma unroll
-        for (int q = 0; q < kE; ++q) {
-            const int j = base + q * G + glane;
-            prod[q] = j < len ? rval[j] * ringx[code[j]] : 0.0;
-        }
-#pragma unroll
-        for (int q = 0; q < kE; ++q) {
-            if (base + q * G >= wlen) break;  // warp-uniform
-#pragma unroll
-            for (int i = 0; i < G; ++i) {
-                const double t = __shfl_sync(kFull, prod[q], gbase + i);
-                if (base + q * G + i < len) sum = sum + t;
-            }
-        }
+    for (int j = 0; j < kSRowMax; j += 2) {
+        if (j >= p.max_row) break;  // the launch's longest row
+        const double2 t = terms[j / 2];
+        sum = (sum + t.x) + t.y;
     }
-    const double xv = v >= 0 ? ringx[0] : 0.0;
-    __syncwarp();  // every lane is done with `ringx` before the next row overwrites it
-    if (v >= 0 && glane < 2) {
-        const double nx = xv + p.relaxation * (rhs - sum) / diag;
-        const unsigned int half = glane == 0 ? static_cast<unsigned>(__double2loint(nx))
-                                             : static_cast<unsigned>(__double2hiint(nx));
-        csg::st_word(p.pub + 2LL * p.n * b + 2LL * v + glane, csg::make_word(__uint_as_float(half), s));
+    if (row.v >= 0 && glane == 0) {
+        const double nx = xv + p.relaxation * (row.rhs - sum) / row.diag;
+        csg::st_quad(words + static_cast<long long>(kWordPitch) * row.v, make_word(nx, row.sweep));
     }
+    __syncwarp();  // every lane is done with `buf` before the next row overwrites it
     return true;
 }
 
@@ -532,21 +564,18 @@ __global__ void __launch_bounds__(512) k_depth_sor_df(SorParams p) {
     const int warp_first_group = (threadIdx.x >> 5) * (32 / G);
     const int my_group = (threadIdx.x & 31) / G;
     const int L = p.n_levels, D = p.stride;
-    // shared-memory image: per group kSRing staged x; values [batch][nloc][max_row];
-    // rhs and diagonal [batch][nloc]; rings [nloc][kSRing] (sign bit: the neighbour
-    // comes first); entry codes [nloc][max_row]; ids, ring sizes, row lengths,
-    // levels; per-level owned ranges
+    // shared-memory image: per group kSRowMax staged values; per owned vertex its
+    // description (id, ring size | row length << 8, level / D); values
+    // [batch][nloc][max_row]; rhs and diagonal [batch][nloc]; rings [nloc][kSRing] (sign
+    // bit: the neighbour comes first); per-level owned ranges; entry codes [nloc][max_row]
     const long long nb = static_cast<long long>(p.batch) * p.nloc_max;
-    double* ringx = reinterpret_cast<double*>(smem_raw) + (threadIdx.x / G) * kSRing;
-    double* sval = reinterpret_cast<double*>(smem_raw) + (blockDim.x / G) * kSRing;
+    double* buf = reinterpret_cast<double*>(smem_raw) + (threadIdx.x / G) * kSRowMax;
+    int4* smeta = reinterpret_cast<int4*>(reinterpret_cast<double*>(smem_raw) + (blockDim.x / G) * kSRowMax);
+    double* sval = reinterpret_cast<double*>(smeta + p.nloc_max);
     double* srhs = sval + nb * p.max_row;
     double* sdiag = srhs + nb;
     int* sring = reinterpret_cast<int*>(sdiag + nb);
-    int* svid = sring + p.nloc_max * kSRing;
-    int* snring = svid + p.nloc_max;
-    int* slen = snring + p.nloc_max;
-    int* slev = slen + p.nloc_max;
-    int* lbeg = slev + p.nloc_max;
+    int* lbeg = sring + p.nloc_max * kSRing;
     int* lend = lbeg + L;
     unsigned char* scode = reinterpret_cast<unsigned char*>(lend + L);
     const int nloc = owned_below(p.n, c, nc);
@@ -575,10 +604,7 @@ __global__ void __launch_bounds__(512) k_depth_sor_df(SorParams p) {
             scode[static_cast<long long>(i) * p.max_row + j] = static_cast<unsigned char>(at);
         }
         if (bad && atomicCAS(&p.ctl->status, CSG_OK, CSG_ERR_ARG) == CSG_OK) p.ctl->where = -1;
-        snring[i] = nr;
-        svid[i] = v;
-        slen[i] = len;
-        slev[i] = lv;
+        smeta[i] = make_int4(v, nr | (len << 8), lv / D, 0);
         for (int b = 0; b < p.batch; ++b) {
             const long long slot = static_cast<long long>(b) * p.nloc_max + i;
             for (int j = 0; j < len; ++j) sval[slot * p.max_row + j] = p.val[b * p.nnz + row + j];
@@ -591,54 +617,60 @@ __global__ void __launch_bounds__(512) k_depth_sor_df(SorParams p) {
         lbeg[l] = owned_below(p.level_begin[l], c, nc);
         lend[l] = owned_below(p.level_end[l], c, nc);
     }
-    for (long long q = tid; q < static_cast<long long>(p.batch) * p.n; q += nthreads) {
-        const double x = p.x[q];
-        csg::st_word(p.pub + 2 * q, csg::make_word(__uint_as_float(static_cast<unsigned>(__double2loint(x))), 0u));
-        csg::st_word(p.pub + 2 * q + 1, csg::make_word(__uint_as_float(static_cast<unsigned>(__double2hiint(x))), 0u));
-    }
+    for (long long q = tid; q < static_cast<long long>(p.batch) * p.n; q += nthreads)
+        csg::st_quad(p.pub + kWordPitch * q, make_word(p.x[q], 0u));
     unsigned int phase = 0;
     int barrier_id = 0;
     if (csg::grid_barrier(p.ctl, phase, p.timeout_ns, barrier_id++)) return;
     if (csg::ld_relaxed_gpu(&p.ctl->status) != CSG_OK) return;  // an oversized row: same answer in every CTA
     const int span = (p.sweeps - 1) * D;  // host guarantees span + L < 2^31
     const int nsteps = span + L;
-    int r = 0, rot = 0;
-    for (int t = 0; t < nsteps; ++t, r = (r + 1 == D) ? 0 : r + 1) {
+    const int top = (L - 1) % D;
+    int r = 0, tq = 0, rot = 0;  // t mod D, t / D, items dealt so far mod groups
+    for (int t = 0; t < nsteps; ++t) {
         int lo = t - span;
         if (lo < r) lo = r;
-        const int hi = t < L ? t : (L - 1) - ((L - 1 - r) % D + D) % D;
-        if (hi < lo) continue;
-        const int i0 = lbeg[lo], i1 = lend[hi];
-        const int count = i1 - i0;
-        for (int k0 = csg::dealt_first(rot, warp_first_group, groups); k0 < count * p.batch; k0 += groups) {
-            const int w = k0 + my_group;
-            int b = 0, i = 0, v = -1, nring = 0, len = 0;
-            unsigned int sweep = 0;
-            const int* ring = nullptr;
-            const unsigned char* code = nullptr;
-            const double* rval = nullptr;
-            double rhs = 0.0, diag = 1.0;
-            if (w >= 0 && w < count * p.batch) {
-                b = w / count;
-                i = i0 + w % count;
-                const long long slot = static_cast<long long>(b) * p.nloc_max + i;
-                v = svid[i];
-                nring = snring[i];
-                len = slen[i];
-                ring = sring + i * kSRing;
-                code = scode + static_cast<long long>(i) * p.max_row;
-                rval = sval + slot * p.max_row;
-                rhs = srhs[slot];
-                diag = sdiag[slot];
-                sweep = static_cast<unsigned int>(1 + (t - slev[i]) / D);
+        const int hi = t < L ? t : L - 1 - (top - r + (r > top ? D : 0));  // the top level of t's residue
+        if (hi >= lo) {
+            const int i0 = lbeg[lo];
+            const int count = lend[hi] - i0, items = count * p.batch;
+            const int ahead = rot - warp_first_group;  // the warp's first group takes k = -ahead mod groups first
+            for (int k0 = ahead >= 0 ? -ahead : -(ahead + groups); k0 < items; k0 += groups) {
+                const int w = k0 + my_group;
+                SorRow row{-1, 0, 0, 1u, nullptr, nullptr, nullptr, 0.0, 1.0};
+                csg::Quad* words = p.pub;
+                if (w >= 0 && w < items) {
+                    int b = 0, i = i0 + w;
+                    while (i - i0 >= count) {  // surface b's items follow surface b - 1's
+                        i -= count;
+                        ++b;
+                    }
+                    const long long slot = static_cast<long long>(b) * p.nloc_max + i;
+                    const int4 m = smeta[i];
+                    row.v = m.x;
+                    row.nring = m.y & 255;
+                    row.len = m.y >> 8;
+                    row.sweep = static_cast<unsigned int>(1 + tq - m.z);  // t and the level agree mod D
+                    row.ring = sring + i * kSRing;
+                    row.code = scode + static_cast<long long>(i) * p.max_row;
+                    row.val = sval + slot * p.max_row;
+                    row.rhs = srhs[slot];
+                    row.diag = sdiag[slot];
+                    words += static_cast<long long>(kWordPitch) * p.n * b;
+                }
+                if (!sor_row_df<G>(p, words, row, buf)) return;
             }
-            if (!sor_row_df<G>(p, b, v, ring, nring, code, rval, len, rhs, diag, sweep, ringx)) return;
+            rot += items;
+            while (rot >= groups) rot -= groups;
         }
-        rot = (rot + count * p.batch) % groups;
+        if (++r == D) {
+            r = 0;
+            ++tq;
+        }
     }
     if (csg::grid_barrier(p.ctl, phase, p.timeout_ns, barrier_id++)) return;
     for (long long q = tid; q < static_cast<long long>(p.batch) * p.n; q += nthreads)
-        p.x[q] = words_value(csg::ld_word(p.pub + 2 * q), csg::ld_word(p.pub + 2 * q + 1));
+        p.x[q] = word_value(csg::ld_quad(p.pub + kWordPitch * q));
 }
 
 // residual terms (rhs - A x)^2 per vertex (also the matrix-vector product of CG's start)
@@ -867,7 +899,7 @@ Layout layout(int n, int nf, int batch, long long nnz) {
     L.z = take(8 * nb);
     L.pv = take(8 * nb);
     L.ap = take(8 * nb);
-    L.pub = take(16 * nb);
+    L.pub = L.r;  // the SOR's published words (kWordPitch quads per value) lie over the CG's four vectors
     L.level_of = take(4 * static_cast<size_t>(n));
     L.total = at;
     return L;
@@ -876,6 +908,7 @@ Layout layout(int n, int nf, int batch, long long nnz) {
 inline unsigned blocks(long long n, int threads) { return static_cast<unsigned>((n + threads - 1) / threads); }
 
 constexpr size_t kMaxRowSmem = 200 * 1024;
+constexpr size_t kMaxDataflowSmem = 206 * 1024;  // its staged rows are longer than the 16-entry rings they lie over
 
 template <int G, bool SMEM>
 int launch_sor(const SorParams& params, int n_ctas, int threads, size_t smem, cudaStream_t s) {
@@ -919,12 +952,12 @@ template <int G>
 int dispatch_sor(SorParams p, int n_ctas, int threads, cudaStream_t s) {
     p.nloc_max = (p.n + n_ctas - 1) / n_ctas;
     // dataflow form: a row's distinct columns (at most 2 max_incidences + 1) fit the ring
-    if (p.pub && p.max_row > 0 && p.max_row <= 255 && 2 * ((p.max_row - 1) / 3) + 1 <= kSRing) {
+    if (p.pub && p.max_row > 0 && p.max_row <= kSRowMax && 2 * ((p.max_row - 1) / 3) + 1 <= kSRing) {
         const long long nb = static_cast<long long>(p.batch) * p.nloc_max;
-        const size_t smem = sizeof(double) * (static_cast<size_t>(threads / G) * kSRing + nb * (p.max_row + 2)) +
-                            sizeof(int) * (static_cast<size_t>(p.nloc_max) * (kSRing + 5) + 2 * static_cast<size_t>(p.n_levels)) +
+        const size_t smem = sizeof(double) * (static_cast<size_t>(threads / G) * kSRowMax + nb * (p.max_row + 2)) +
+                            sizeof(int) * (static_cast<size_t>(p.nloc_max) * (kSRing + 4) + 2 * static_cast<size_t>(p.n_levels)) +
                             static_cast<size_t>(p.nloc_max) * p.max_row;
-        if (smem <= kMaxRowSmem) return launch_sor_df<G>(p, n_ctas, threads, smem, s);
+        if (smem <= kMaxDataflowSmem) return launch_sor_df<G>(p, n_ctas, threads, smem, s);
     }
     const size_t ints = static_cast<size_t>(p.nloc_max) * (p.max_row + 2) + 2 * static_cast<size_t>(p.n_levels);
     const size_t smem = sizeof(double) * static_cast<size_t>(p.batch) * p.nloc_max * (p.max_row + 3) + sizeof(int) * ints;
@@ -1029,7 +1062,7 @@ int csg_depth_potential(const float* geometry, int batch, int n, const int32_t* 
             p.max_row = 3 * max_incidences + 1;
             p.relaxation = relaxation;
             p.timeout_ns = timeout_ns;
-            p.pub = reinterpret_cast<unsigned long long*>(base + L.pub);
+            p.pub = reinterpret_cast<csg::Quad*>(base + L.pub);
             p.level_of = reinterpret_cast<int*>(base + L.level_of);
             (csg::note_launch(), k_level_of<<<dim3(blocks(n, kThreads) > 64 ? 64 : blocks(n, kThreads), n_levels),
                                               kThreads, 0, s>>>(order, level_begin, level_end, p.level_of));

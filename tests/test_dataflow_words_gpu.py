@@ -71,3 +71,24 @@ def test_stage_passes_equal_the_oracle(native_library, kind, lanes, stop_at):
                                              launch=launch)
     want = oracle_pre.preprocess(vertices, faces, stop_at=stop_at)
     np.testing.assert_array_equal(got, want)
+
+
+@pytest.mark.parametrize("n, seed", [(60, 0), (150, 1), (300, 3)])  # rings of at most eight members, and of nine
+@pytest.mark.parametrize("lanes", [4, 8, 16])
+@pytest.mark.parametrize("batch", [1, 3])
+def test_depth_sor_equals_the_oracle(native_library, n, seed, lanes, batch):
+    from cat_surface_gpu_b200.rotation_feature import DepthTopology, depth_potential
+    from oracle import depth as oracle_depth
+
+    vertices, faces = synthetic.folded_hull(n, seed)
+    surfaces = np.stack([vertices * np.float32(1.0 + 0.25 * b) for b in range(batch)])
+    topology = DepthTopology.build(faces, n, torch.device("cuda:0"))
+    groups = oracle_depth.colour_groups(faces, n)
+    launch = {"n_ctas": 3, "threads_per_cta": 64, "lanes_per_row": lanes}
+    for sweeps in (1, 40):
+        got, _, residual = depth_potential(torch.as_tensor(surfaces, device="cuda:0"), topology, max_iter=sweeps,
+                                           launch=launch)
+        for b in range(batch):
+            want, _, want_residual = oracle_depth.System(surfaces[b], faces).sor(groups, sweeps)
+            np.testing.assert_array_equal(got[b].cpu().numpy(), want)
+            assert residual[b] == want_residual
