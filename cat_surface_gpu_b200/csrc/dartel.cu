@@ -21,8 +21,10 @@
 #include <cmath>
 #include <cstdint>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include "../../include/catsurf_b200.h"
@@ -472,24 +474,6 @@ __device__ __forceinline__ Nbr4 neighbours(int x, int y, int nx, int ny) {
     return {nb(x, y, -1, 0, nx, ny), nb(x, y, 1, 0, nx, ny), nb(x, y, 0, -1, nx, ny), nb(x, y, 0, 1, nx, ny)};
 }
 
-// membrane_apply_at (rtype 1) with the neighbour offsets given, for one batch element's fields.
-template <typename T>
-__device__ __forceinline__ void membrane_core(const T* __restrict__ H, const T* __restrict__ ux,
-                                              const T* __restrict__ b, T* __restrict__ o, int P, int i, const Nbr4& n,
-                                              const RegWeights& rw) {
-    const T w00 = T(rw.w[0]), w01 = T(rw.w[1]), w10 = T(rw.w[2]);
-    T reg[2];
-    for (int c = 0; c < 2; ++c) {
-        const T* f = ux + c * P;
-        reg[c] = w00 * f[i] + w01 * (f[n.ym] + f[n.yp]) + w10 * (f[n.xm] + f[n.xp]);
-    }
-    const T u0 = ux[i], u1 = ux[P + i];
-    const T a0 = reg[0] + H[i] * u0 + H[2 * P + i] * u1;
-    const T a1 = reg[1] + H[2 * P + i] * u0 + H[P + i] * u1;
-    o[i] = b[i] - a0;
-    o[P + i] = b[P + i] - a1;
-}
-
 template <typename T>
 __device__ __forceinline__ void membrane_apply_at(const T* __restrict__ hess, const T* __restrict__ u,
                                                   const T* __restrict__ b, T* __restrict__ out, int nx, int ny,
@@ -656,233 +640,759 @@ __global__ void k_resize(const T* __restrict__ src, T* __restrict__ dst, int snx
     resize_at(src, dst, snx, sny, tnx, tny, accumulate, static_cast<int>(blockIdx.y), i);
 }
 
-// ------------------------------------------------ fused coarse multigrid cycle
+// ------------------------------------------------ resident V-cycles (one cluster per grid)
 //
-// The levels of a V-cycle at or below kCoarsePoints points per grid run as one
-// launch with one CTA per batch element: the same per-point operations as the
-// separate kernels (relax_at, membrane_apply_at, resize_at) in the same
-// order, phases separated by __syncthreads.  A coarse level's work is a few
-// thousand points, so one CTA covers it, and ~100 small launches per cycle
-// become one.  Every level's Hessian, right-hand side, solution and residual
-// live in shared memory for the whole cycle (at most ~1,100 points over all
-// levels, 9 words each): the CTA reads the Hessians and the first level's
-// right-hand side and solution once, and writes back the first level's
-// solution, the only field read after the cycle.  Each point's neighbour
-// offsets and each level pair's resize taps (per target row and column) are
-// tabled once per launch, so the ~90 barrier-separated phases do no index or
-// weight arithmetic (the values are the ones relax_at, membrane_apply_at and
-// resize_at form).
+// From the finest level whose grid fits the shared memory and registers of one
+// thread-block cluster (256 x 128 in float64) on, a whole V-cycle -- all cycles of
+// a solve when that is level 0 -- is one launch with one cluster per batch element.
+// What bounds a V-cycle here is its chain of ~100 half-sweeps and ~40 residuals and
+// transfers, each a few hundred cycles of dependent arithmetic: as separate
+// launches, or as tiles that recompute their halos, each link cost 2-4 us.  Inside a
+// cluster the neighbours' edge rows are written straight into each other's shared memory and
+// a link costs 250-550 ns.  Per V-cycle, against legs of 2-D tiles over one CTA for the
+// coarse levels: two 256 x 128 grids 129 -> 56 us in float64 and 123 -> 57 in float32, 64 x 32
+// 71 -> 27 us, 32 x 16 47 -> 17 us; 32 float32 grids of 256 x 128 369 -> 243 us, 64 float64 grids
+// 731 -> 561 us.  Of the 56 us the first level takes 20, the other split levels 20, the levels of
+// CTA 0 17.
+//
+// Levels above kCoarsePoints points are split by rows over the cluster's CTAs, each
+// holding its rows of u with a halo row above and below.  The first such level's system
+// and right-hand side are read from global memory at each visit, the others' are in
+// shared memory; during a visit they are in registers.  The levels below run on CTA 0
+// alone, in teams of 256 and 64 threads and one warp as they shrink.  256 threads of up to
+// 255 registers, not 512 of 128: the eight points of a thread (float64: 112 registers) must
+// not spill, since shared memory leaves the L1 too small for it (70 us per V-cycle with spills).
+// Every point sees the operations of relax_core, membrane_apply_at and
+// resize_value in their order, so results equal the separate kernels' bit for bit.
 
-constexpr int kCoarsePoints = 512;  // measured: 512 beats 0, 2048 and 8192 at 256 x 128
+constexpr int kCoarsePoints = 512;  // levels of at most this many points run on one CTA, a unit of two points per thread
 constexpr int kMaxLevels = 16;
-constexpr int kCoarseThreads = 1024;
-constexpr int kCoarseCycleThreads = 512;
+constexpr int kResidentThreads = 256;
+constexpr int kResidentSlots = 4;   // units a thread holds of a split level at most
+constexpr int kResidentPoints = 2 * kResidentSlots * kResidentThreads;  // of a CTA's rows of it
+constexpr int kMaxCluster = 16;     // 16 CTAs is the largest cluster of the architecture (8 is the portable bound)
+// A launch of more CTAs than the device's 148 SMs hold as clusters of 16 uses as few CTAs per grid
+// as hold it (64 float64 grids of 128 x 64 per V-cycle: 354 us with 16 CTAs each, 95 with 4; two
+// of them: 36 and 55), and in float32 the kernel of 128 registers, two CTAs to an SM (32 grids of
+// 256 x 128: 286 -> 243 us; two: 57 and 71).
+constexpr int kPairedCtas = 128;
+
+// Both components of a field at a point, moved together.
+template <typename T>
+struct alignas(2 * sizeof(T)) Pair {
+    T x, y;
+};
+
+// A point's 2 x 2 system: the Hessian, the determinant relax_core divides by, and its
+// correctly rounded reciprocal (0: divide).
+template <typename T>
+struct PointSystem {
+    T h0, h1, h2, det, inv;
+};
 
 template <typename T>
-struct CoarseLevel {
-    const T* A;  // Hessian [batch][3][ny][nx]
-    T* B;        // right-hand side [batch][2][ny][nx]
-    T* U;        // solution [batch][2][ny][nx]
-    T* R;        // residual [batch][2][ny][nx]
-    int nx, ny;
+__device__ __forceinline__ PointSystem<T> point_system(T h0, T h1, T h2, T w00) {
+    PointSystem<T> s{h0, h1, h2, T(0), T(0)};
+    const T dxx = h0 + w00, dyy = h1 + w00;
+    s.det = dxx * dyy * T(1.0000000001) - h2 * h2;
+    if constexpr (sizeof(T) == 8) {
+        const unsigned e = (static_cast<unsigned>(__double2hiint(s.det)) >> 20) & 0x7ffu;
+        if (e - 623u <= 800u) s.inv = __drcp_rn(s.det);  // 2^-400 <= |det| <= 2^400
+    }
+    return s;
+}
+
+// (a.x / s.det, a.y / s.det).  float64: with y = RN(1 / d) and q within an ulp of a / d,
+// RN(q + RN(a - d q) y) is the correctly rounded quotient (P. Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34(1),
+// 1990); q0 = RN(a y) is refined once to come within an ulp.  The exponent bounds
+// (2^-500 <= |a| < 2^500 here, s.inv = 0 for an extreme determinant) keep every remainder
+// and quotient normal; outside them, and for a = 0, the division itself runs.  Both
+// quotients share one test, off their dependency chain: a half-sweep of one warp takes 243
+// cycles without a test, 365 with one per quotient, as with the divisions.
+template <typename T>
+__device__ __forceinline__ Pair<T> quotients(T a0, T a1, const PointSystem<T>& s) {
+    if constexpr (sizeof(T) == 8) {
+        // biased exponents 523 .. 1522, the sign shifted out
+        const unsigned e0 = 2u * static_cast<unsigned>(__double2hiint(a0)) - (523u << 21);
+        const unsigned e1 = 2u * static_cast<unsigned>(__double2hiint(a1)) - (523u << 21);
+        const double p0 = __dmul_rn(a0, s.inv), p1 = __dmul_rn(a1, s.inv);
+        const double q0 = __fma_rn(__fma_rn(-s.det, p0, a0), s.inv, p0);
+        const double q1 = __fma_rn(__fma_rn(-s.det, p1, a1), s.inv, p1);
+        Pair<T> r{__fma_rn(__fma_rn(-s.det, q0, a0), s.inv, q0), __fma_rn(__fma_rn(-s.det, q1, a1), s.inv, q1)};
+        if (e0 >= (1000u << 21) || e1 >= (1000u << 21) || __double2hiint(s.inv) == 0) r = {a0 / s.det, a1 / s.det};
+        return r;
+    } else {
+        return {a0 / s.det, a1 / s.det};
+    }
+}
+
+template <typename T>
+struct Weights {
     T w00, w01, w10;
-    RegWeights rw;
-    int off;  // offset of the level's [A 3 | B 2 | U 2 | R 2] x nx x ny block in shared memory (elements)
 };
 
 template <typename T>
-struct CoarseCycle {
-    CoarseLevel<T> lv[kMaxLevels];
-    int first, last, nit;
+struct ResidentLevel {
+    const T* A;  // Hessian [batch][3][ny][nx]
+    T* B;        // right-hand side [batch][2][ny][nx] (the first level's is read)
+    T* U;        // solution [batch][2][ny][nx] (the first level's is read and written)
+    int nx, ny, lg;   // lg: log2(nx), a power of two on every level
+    int rows;         // rows of a CTA's slab at most (0: a level of CTA 0 alone)
+    int own;          // points in a CTA's memory (of a slab at most)
+    int u, b, r;      // byte offsets in shared memory: solution, right-hand side, residual (a split level's
+                      // solution and residual have a halo row above and below)
+    int a;            // and systems: pairs (h0, h1) [own], pairs (h2, det) [own], inv [own]
+    int down, up;     // and row taps of the restriction to the next level / the prolongation to this one
+    int team;         // threads of CTA 0 that run a whole level
+    int near;         // a split level: every row a CTA's transfers read is one of its own or next to them
+    Weights<T> w, g;  // relaxation weights (mem_weights) and operator weights (reg_weights)
 };
 
-// Resize of one batch element's two planes with the target rows' and columns' taps tabled.
-// The threads that work a phase of the coarse cycle and their barrier: the whole CTA,
-// or (levels of at most 32 points) warp 0 alone with a warp barrier.
-template <bool WARP>
-struct Team {
-    static __device__ __forceinline__ int rank() { return WARP ? (threadIdx.x & 31) : threadIdx.x; }
-    static __device__ __forceinline__ int size() { return WARP ? 32 : blockDim.x; }
-    static __device__ __forceinline__ void sync() {
-        if (WARP) __syncwarp();
-        else __syncthreads();
-    }
-};
-
-// Resize of one batch element's two planes with the target rows' and columns' taps tabled.
-template <bool WARP, typename T>
-__device__ __forceinline__ void taps_resize(const T* src, int snx, int sny, T* dst, int tnx, int tny,
-                                            const AxisTaps<T>* rows, const AxisTaps<T>* cols, int accumulate) {
-    const int P = tnx * tny;
-    for (int j = Team<WARP>::rank(); j < 2 * P; j += Team<WARP>::size()) {
-        const int c = j >= P ? 1 : 0, i = j - c * P;
-        const T r = resize_value(src + static_cast<size_t>(c) * snx * sny, rows[i / tnx], cols[i % tnx]);
-        T* o = dst + static_cast<size_t>(c) * P;
-        o[i] = accumulate ? o[i] + r : r;
-    }
-    Team<WARP>::sync();
-}
-
-// The shared-memory image of level L (one batch element, batch index 0).
 template <typename T>
-__device__ __forceinline__ CoarseLevel<T> shared_level(const CoarseLevel<T>& L, T* base) {
-    CoarseLevel<T> S = L;
-    const int P = L.nx * L.ny;
-    T* a = base + L.off;
-    S.A = a;
-    S.B = a + 3 * P;
-    S.U = a + 5 * P;
-    S.R = a + 7 * P;
-    return S;
+struct ResidentCycle {
+    ResidentLevel<T> lv[kMaxLevels];
+    int first, local, last;  // levels first .. local - 1 are split over the cluster, local .. last run on CTA 0
+    int nit, cycles;
+    int lgsize;              // log2 of the cluster's CTAs
+};
+
+// The start of a CTA's shared memory; the levels' fields and the row taps follow.  What
+// follows addresses them by 32-bit byte offsets from the shared array itself: through pointers
+// every access would need 64-bit address arithmetic or go through the generic address window.
+// The plan is read from the kernel's parameters, which makes its values uniform to the
+// compiler: a half-sweep is ~60 instructions of one chain, and every branch that might
+// diverge adds 20-40 cycles to it (227 cycles with none, 440 with five).  So inner branches
+// are on uniform values, and what depends on the lane is computed by all and stored under a
+// predicate.
+struct ResidentHead {
+    alignas(8) unsigned long long barriers[2];
+    int lost;
+};
+constexpr int kHead = 32;
+static_assert(sizeof(ResidentHead) <= kHead);
+
+extern __shared__ __align__(16) unsigned char resident_smem[];
+__device__ __forceinline__ ResidentHead& resident_head() { return *reinterpret_cast<ResidentHead*>(resident_smem); }
+template <typename T>
+__device__ __forceinline__ Pair<T>& pair_at(int offset) {
+    return *reinterpret_cast<Pair<T>*>(resident_smem + offset);
+}
+template <typename T>
+__device__ __forceinline__ const AxisTaps<T>& taps_at(int offset, int k) {
+    return *reinterpret_cast<const AxisTaps<T>*>(resident_smem + offset + k * static_cast<int>(sizeof(AxisTaps<T>)));
+}
+template <typename T>
+__device__ __forceinline__ PointSystem<T> load_system(int a, int own, int i) {
+    constexpr int kPair = sizeof(Pair<T>);
+    const Pair<T> p = pair_at<T>(a + i * kPair), q = pair_at<T>(a + (own + i) * kPair);
+    T inv = T(0);
+    if constexpr (sizeof(T) == 8) inv = *reinterpret_cast<const T*>(resident_smem + a + 2 * own * kPair + i * sizeof(T));
+    return {p.x, p.y, q.x, q.y, inv};
+}
+template <typename T>
+__device__ __forceinline__ void store_system(int a, int own, int i, const PointSystem<T>& s) {
+    constexpr int kPair = sizeof(Pair<T>);
+    pair_at<T>(a + i * kPair) = {s.h0, s.h1};
+    pair_at<T>(a + (own + i) * kPair) = {s.h2, s.det};
+    if constexpr (sizeof(T) == 8) *reinterpret_cast<T*>(resident_smem + a + 2 * own * kPair + i * sizeof(T)) = s.inv;
 }
 
-// Red-black relaxation of a shared-memory level with tabled neighbour offsets.
-template <bool WARP, typename T>
-__device__ __forceinline__ void table_relax(const CoarseLevel<T>& L, const int4* tab, int nit) {
-    const int P = L.nx * L.ny;
-    for (int it = 0; it < 2 * nit; ++it) {
-        const int colour = it % 2 == 0 ? 1 : 0;
-        for (int i = Team<WARP>::rank(); i < P; i += Team<WARP>::size()) {
-            const int4 t = tab[i];
-            if (((i % L.nx + i / L.nx) & 1) == colour)
-                relax_core(L.A, L.B, L.U, P, 0, i, Nbr4{t.x, t.y, t.z, t.w}, L.w00, L.w01, L.w10);
+// Every field of a level is an image of rows of nx pairs, a row holding its points of colour 0
+// ((x + y) even) by ascending x, then those of colour 1: the points of one colour that the
+// lanes of a warp hold, and each kind of neighbour of theirs, are consecutive in shared memory.
+__device__ __forceinline__ int image_column(int y, int x, int nx) { return ((x + y) & 1) * (nx >> 1) + (x >> 1); }
+
+// A point a thread holds in registers: its system and right-hand side.
+template <typename T>
+struct Point {
+    PointSystem<T> s;
+    Pair<T> b;
+};
+
+// The points (2 j, y) and (2 j + 1, y), one of each colour, as byte offsets in the image of u whose
+// row y starts at `row`; each is the other's x neighbour on one side.  nx = 1: the row's one
+// point, its own x neighbour.  At the grid's edges the y neighbour is the point itself.
+struct Unit {
+    int q[2];              // the points of colour 0 and 1
+    int side[2];           // their other x neighbours
+    int above[2], below[2];
+    bool odd;              // the point of colour 0 is (2 j + 1, y)
+};
+template <typename T>
+__device__ __forceinline__ Unit make_unit(int row, int y, int j, int nx, int ny) {
+    constexpr int kPair = sizeof(Pair<T>);
+    const int h = nx >> 1, mask = h > 0 ? h - 1 : 0, next = (j + 1) & mask, previous = (j - 1) & mask;
+    Unit m;
+    m.odd = (y & 1) != 0 && nx > 1;
+    m.q[0] = row + j * kPair;
+    m.q[1] = m.q[0] + h * kPair;
+    m.side[0] = row + (h + (m.odd ? next : previous)) * kPair;
+    m.side[1] = row + (m.odd ? previous : next) * kPair;
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+        m.above[c] = y == 0 ? m.q[c] : m.q[1 - c] - nx * kPair;
+        m.below[c] = y == ny - 1 ? m.q[c] : m.q[1 - c] + nx * kPair;
+    }
+    return m;
+}
+
+// Sums of the y and of the x neighbours of a unit's point.
+template <int COLOUR, typename T>
+__device__ __forceinline__ void neighbour_sums(const Unit& m, Pair<T>& ys, Pair<T>& xs) {
+    const Pair<T> a = pair_at<T>(m.above[COLOUR]), b = pair_at<T>(m.below[COLOUR]);
+    const Pair<T> c = pair_at<T>(m.q[1 - COLOUR]), d = pair_at<T>(m.side[COLOUR]);
+    ys = {a.x + b.x, a.y + b.y};
+    xs = {c.x + d.x, c.y + d.y};
+}
+
+// relax_core at a held point.
+template <int COLOUR, typename T>
+__device__ __forceinline__ Pair<T> relaxed(const Unit& m, const Point<T>& p, const Weights<T>& w) {
+    Pair<T> ys, xs;
+    neighbour_sums<COLOUR>(m, ys, xs);
+    const T rx = p.b.x - w.w01 * ys.x - w.w10 * xs.x;
+    const T ry = p.b.y - w.w01 * ys.y - w.w10 * xs.y;
+    const T dxx = p.s.h0 + w.w00, dyy = p.s.h1 + w.w00;
+    return quotients(dyy * rx - p.s.h2 * ry, -p.s.h2 * rx + dxx * ry, p.s);
+}
+
+// membrane_apply_at's residual at a held point (w: the operator weights).
+template <int COLOUR, typename T>
+__device__ __forceinline__ Pair<T> residual(const Unit& m, const Point<T>& p, const Weights<T>& w) {
+    Pair<T> ys, xs;
+    neighbour_sums<COLOUR>(m, ys, xs);
+    const Pair<T> v = pair_at<T>(m.q[COLOUR]);
+    const T reg0 = w.w00 * v.x + w.w01 * ys.x + w.w10 * xs.x;
+    const T reg1 = w.w00 * v.y + w.w01 * ys.y + w.w10 * xs.y;
+    return {p.b.x - (reg0 + p.s.h0 * v.x + p.s.h2 * v.y), p.b.y - (reg1 + p.s.h2 * v.x + p.s.h1 * v.y)};
+}
+
+// ---- transfers between levels whose x sizes are powers of two: resize_value of both
+// components, the inner sums down the three source rows first.  The column weights are exact
+// values of col_taps.  Halving reads columns 2 X .. 2 X + 2, doubling x / 2 - 1 .. x / 2 + 1 by the
+// parity of x; between levels of one column it is that column three times.
+
+template <typename T>
+__device__ __forceinline__ void add_row(Pair<T> (&v)[3], int r, T w, const Pair<T>& p0, const Pair<T>& p1, const Pair<T>& p2) {
+    const Pair<T> p[3] = {p0, p1, p2};
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const Pair<T> d{w * p[k].x, w * p[k].y};
+        v[k] = r == 0 ? d : Pair<T>{v[k].x + d.x, v[k].y + d.y};
+    }
+}
+template <typename T>
+__device__ __forceinline__ Pair<T> column_sum(const Pair<T> (&v)[3], T w0, T w1, T w2) {
+    return {w0 * v[0].x + w1 * v[1].x + w2 * v[2].x, w0 * v[0].y + w1 * v[1].y + w2 * v[2].y};
+}
+template <typename T>
+__device__ __forceinline__ Pair<T> halved(const Pair<T> (&v)[3], bool same) {
+    return column_sum<T>(v, same ? T(0.125) : T(0.5), same ? T(0.75) : T(0.5), same ? T(0.125) : T(0));
+}
+template <typename T>
+__device__ __forceinline__ Pair<T> doubled(const Pair<T> (&v)[3], bool same, bool odd) {
+    return column_sum<T>(v, same ? T(0.125) : (odd ? T(0.03125) : T(0.28125)), same ? T(0.75) : T(0.6875),
+                         same ? T(0.125) : (odd ? T(0.28125) : T(0.03125)));
+}
+// The sums down the rows t.o of the image at byte offset f (its row `lo` first) of columns x - 1,
+// x, x + 1 (periodic).
+template <typename T>
+__device__ __forceinline__ void row_sums(int f, int lo, const AxisTaps<T>& t, int x, int nx, Pair<T> (&v)[3]) {
+    constexpr int kPair = sizeof(Pair<T>);
+    const int half = (nx >> 1) * kPair, mask = nx - 1;
+    const int before = (((x - 1) & mask) >> 1) * kPair, centre = (x >> 1) * kPair, after = (((x + 1) & mask) >> 1) * kPair;
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+        const int g = t.o[r], row = f + (g - lo) * nx * kPair, shift = ((x + g) & 1) * half;
+        const int own = row + shift, other = row + half - shift;
+        add_row(v, r, t.w[r], pair_at<T>(other + before), pair_at<T>(own + centre), pair_at<T>(other + after));
+    }
+}
+
+// ---- levels of CTA 0.  A thread holds one unit.  A level's team is as many threads as it has
+// units, rounded up to 32, 64 or 256; a smaller team synchronises in fewer cycles.
+
+// (a branch by team to __syncwarp or an immediate barrier costs 30 cycles more)
+__device__ __forceinline__ void team_sync(int id, int team) {
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(team) : "memory");
+}
+__device__ __forceinline__ int team_barrier(int team) { return team == 32 ? 1 : team == 64 ? 2 : 4; }
+
+// One visit of a level of CTA 0 in a V-cycle by its team.  up: prolongation of level
+// l + 1's solution, then relaxation.  Else relaxation and, unless l is the last level, the
+// residual and its restriction to level l + 1, whose solution is zeroed.
+template <typename T>
+__device__ __forceinline__ void local_visit(const ResidentCycle<T>& c, int l, bool up) {
+    constexpr int kPair = sizeof(Pair<T>);
+    const ResidentLevel<T>& L = c.lv[l];
+    const ResidentLevel<T>& N = c.lv[l + 1 <= c.last ? l + 1 : l];
+    const int nx = L.nx, ny = L.ny, team = L.team, id = team_barrier(team), h = nx >> 1, thread = threadIdx.x;
+    const int row = thread >> (L.lg > 0 ? L.lg - 1 : 0), j = h > 0 ? thread & (h - 1) : 0;
+    const bool same = nx == 1, in = row < ny;
+    const int y = in ? row : ny - 1;  // (a thread without a unit computes the last row's again)
+    const bool has0 = in && (!same || (y & 1) == 0), has1 = in && (!same || (y & 1) != 0);
+    const int u = L.u, i = y * nx + j;
+    const Unit m = make_unit<T>(u + y * nx * kPair, y, j, nx, ny);
+    const Point<T> p0{load_system<T>(L.a, L.own, i), pair_at<T>(L.b + i * kPair)};
+    const Point<T> p1{load_system<T>(L.a, L.own, i + h), pair_at<T>(L.b + (i + h) * kPair)};
+    if (up) {
+        Pair<T> v[3];
+        row_sums(N.u, 0, taps_at<T>(L.up, y), j, N.nx, v);
+        const Pair<T> d0 = doubled(v, same, m.odd), d1 = doubled(v, same, !m.odd), v0 = pair_at<T>(m.q[0]),
+                      v1 = pair_at<T>(m.q[1]);
+        if (in) pair_at<T>(m.q[0]) = {v0.x + d0.x, v0.y + d0.y};
+        if (in && !same) pair_at<T>(m.q[1]) = {v1.x + d1.x, v1.y + d1.y};
+        team_sync(id, team);
+    }
+    const Weights<T> w = L.w;
+    const int nit = c.nit;
+#pragma unroll 1
+    for (int it = 0; it < nit; ++it) {
+        const Pair<T> v1 = relaxed<1>(m, p1, w);
+        if (has1) pair_at<T>(m.q[1]) = v1;
+        team_sync(id, team);
+        const Pair<T> v0 = relaxed<0>(m, p0, w);
+        if (has0) pair_at<T>(m.q[0]) = v0;
+        team_sync(id, team);
+    }
+    if (up || l == c.last) return;
+    const int r = L.r - u;
+    const Weights<T> g = L.g;
+    const Pair<T> r1 = residual<1>(m, p1, g), r0 = residual<0>(m, p0, g);
+    if (has1) pair_at<T>(m.q[1] + r) = r1;
+    if (has0) pair_at<T>(m.q[0] + r) = r0;
+    team_sync(id, team);
+    const int snx = N.nx;
+    for (int k = thread; k < N.own; k += team) {
+        const int X = k & (snx - 1), Y = k >> N.lg;
+        Pair<T> v[3];
+        row_sums(L.r, 0, taps_at<T>(L.down, Y), same ? 0 : 2 * X + 1, nx, v);
+        pair_at<T>(N.b + (Y * snx + image_column(Y, X, snx)) * kPair) = halved(v, same);
+        pair_at<T>(N.u + k * kPair) = Pair<T>{T(0), T(0)};
+    }
+    team_sync(id, team);
+}
+
+// The V-cycle's levels local .. last on CTA 0; a thread takes part while the level's team includes
+// it, and on the way up waits for the smaller team of the level below.
+template <typename T>
+__device__ __forceinline__ void local_cycle(const ResidentCycle<T>& c) {
+    const int thread = threadIdx.x, local = c.local, last = c.last;
+    // (visits in one uniform sequence, down then up)
+    const int visits = 2 * (last - local) + 1;
+#pragma unroll 1
+    for (int k = 0; k < visits; ++k) {
+        const bool up = k > last - local;
+        const int l = up ? 2 * last - local - k : local + k, team = c.lv[l].team;
+        if (thread >= team) continue;
+        if (up && c.lv[l + 1].team != team) team_sync(team_barrier(team), team);  // the smaller team is done with l + 1
+        local_visit<T>(c, l, up);
+    }
+    __syncthreads();
+}
+
+// ---- levels split over the cluster
+
+__device__ __forceinline__ unsigned shared_address(const void* p) {
+    return static_cast<unsigned>(__cvta_generic_to_shared(p));
+}
+// The address, in the cluster's shared window, of byte offset `offset` of CTA `rank`'s shared memory.
+__device__ __forceinline__ unsigned cluster_address(int offset, int rank) {
+    unsigned a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(shared_address(resident_smem + offset)), "r"(rank));
+    return a;
+}
+// Where `on`, store a pair in another CTA's shared memory and count its bytes on a barrier there.
+__device__ __forceinline__ void send(bool on, unsigned to, unsigned barrier, const Pair<double>& v) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %0, 0;\n\t@p st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%1], {%2, %3}, [%4];\n\t}" ::"r"(static_cast<unsigned>(on)),
+                 "r"(to), "l"(__double_as_longlong(v.x)), "l"(__double_as_longlong(v.y)), "r"(barrier)
+                 : "memory");
+}
+__device__ __forceinline__ void send(bool on, unsigned to, unsigned barrier, const Pair<float>& v) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %0, 0;\n\t@p st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%1], {%2, %3}, [%4];\n\t}" ::"r"(static_cast<unsigned>(on)),
+                 "r"(to), "r"(__float_as_uint(v.x)), "r"(__float_as_uint(v.y)), "r"(barrier)
+                 : "memory");
+}
+// Plain stores (where `on`) and loads of another CTA's shared memory; cluster barriers order them.
+__device__ __forceinline__ void put(bool on, unsigned to, const Pair<double>& v) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %0, 0;\n\t@p st.shared::cluster.v2.f64 [%1], {%2, %3};\n\t}" ::"r"(static_cast<unsigned>(on)),
+                 "r"(to), "d"(v.x), "d"(v.y)
+                 : "memory");
+}
+__device__ __forceinline__ void put(bool on, unsigned to, const Pair<float>& v) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %0, 0;\n\t@p st.shared::cluster.v2.f32 [%1], {%2, %3};\n\t}" ::"r"(static_cast<unsigned>(on)),
+                 "r"(to), "f"(v.x), "f"(v.y)
+                 : "memory");
+}
+__device__ __forceinline__ void get(unsigned from, Pair<double>& v) {
+    asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(from) : "memory");
+}
+__device__ __forceinline__ void get(unsigned from, Pair<float>& v) {
+    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(from) : "memory");
+}
+
+// The edge-row exchange of the half-sweeps.  Half-sweep e sends each updated edge point to
+// the neighbour's halo, counted on the neighbour's barrier e & 1, which completes when
+// both neighbours' bytes have come and this CTA has announced them.  Half-sweep e waits for
+// half-sweep e - 1; a neighbour can run at most one half-sweep ahead (its e + 1 needs this
+// CTA's e), so two barriers do, and what it then writes is of the colour that no edge point
+// reads in half-sweep e.  An exchange of 16 CTAs in a chain takes 434 cycles from wait to wait.
+// (A cluster barrier with its release and acquire takes 570, 770-980 with remote stores before
+// it; remote stores with one remote arrival per warp 1,120; bulk copies of the rows 470-480.)
+// Every wait is bounded; one that runs out sets `lost`: the CTA waits no more and its results
+// are replaced by NaN.
+__device__ __forceinline__ void await_exchange(unsigned at, unsigned parity, int* lost) {
+    for (int tries = 0;; ++tries) {
+        unsigned done;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(done)
+            : "r"(at), "r"(parity)
+            : "memory");
+        if (done) return;
+        if (tries > (1 << 16) || *reinterpret_cast<volatile int*>(lost)) {
+            *reinterpret_cast<volatile int*>(lost) = 1;
+            return;
         }
-        Team<WARP>::sync();
     }
 }
 
-// The down half of the V-cycle at level l: relaxation, residual, its restriction to
-// level l + 1 and that level's zero solution.
-template <bool WARP, typename T>
-__device__ __forceinline__ void coarse_down(const CoarseCycle<T>& c, int l, T* base, const int4* tab,
-                                            const AxisTaps<T>* rows, const AxisTaps<T>* cols) {
-    const CoarseLevel<T> L = shared_level(c.lv[l], base);
-    table_relax<WARP>(L, tab, c.nit);
-    const int P = L.nx * L.ny;
-    for (int i = Team<WARP>::rank(); i < P; i += Team<WARP>::size()) {
-        const int4 t = tab[i];
-        membrane_core(L.A, L.U, L.B, L.R, P, i, Nbr4{t.x, t.y, t.z, t.w}, L.rw);
+// A CTA's rows of a split level.
+struct Slab {
+    int lo, n;  // its rows
+    int lg, nx, ny;
+    int rank, lgsize;
+    __device__ __forceinline__ Slab(int lg_, int nx_, int ny_, int rank_, int lgsize_)
+        : lg(lg_), nx(nx_), ny(ny_), rank(rank_), lgsize(lgsize_) {
+        lo = begin(rank);
+        n = begin(rank + 1) - lo;
     }
-    Team<WARP>::sync();
-    const CoarseLevel<T> N = shared_level(c.lv[l + 1], base);
-    taps_resize<WARP>(L.R, L.nx, L.ny, N.B, N.nx, N.ny, rows, cols, 0);
-    const int Pn = N.nx * N.ny;
-    for (int j = Team<WARP>::rank(); j < 2 * Pn; j += Team<WARP>::size()) N.U[j] = T(0);
-    Team<WARP>::sync();
-}
-
-// The up half at level l: prolongation of level l + 1's solution, then relaxation.
-template <bool WARP, typename T>
-__device__ __forceinline__ void coarse_up(const CoarseCycle<T>& c, int l, T* base, const int4* tab,
-                                          const AxisTaps<T>* rows, const AxisTaps<T>* cols) {
-    const CoarseLevel<T> L = shared_level(c.lv[l], base);
-    const CoarseLevel<T> N = shared_level(c.lv[l + 1], base);
-    taps_resize<WARP>(N.U, N.nx, N.ny, L.U, L.nx, L.ny, rows, cols, 1);
-    table_relax<WARP>(L, tab, c.nit);
-}
-
-// cycle(first) of Fmg (host side) restricted to levels first..last, for batch element blockIdx.x.
+    __device__ __forceinline__ int begin(int r) const { return (r * ny) >> lgsize; }
+    __device__ __forceinline__ bool above() const { return rank > 0; }
+    __device__ __forceinline__ bool below() const { return rank + 1 < (1 << lgsize); }
+};
 template <typename T>
-__global__ void __launch_bounds__(kCoarseCycleThreads) k_fmg_coarse_cycle(CoarseCycle<T> c) {
+__device__ __forceinline__ Slab slab_of(const ResidentCycle<T>& c, int l) {
+    return Slab(c.lv[l].lg, c.lv[l].nx, c.lv[l].ny, static_cast<int>(blockIdx.x), c.lgsize);
+}
+
+// row_sums over a field at byte offset f whose CTAs hold their rows between two halo rows.  near: the
+// three rows are the CTA's own or its halo rows, else each is read from the CTA that holds it.
+template <typename T>
+__device__ __forceinline__ void slab_sums(const Slab& V, int f, bool near, const AxisTaps<T>& t, int x, Pair<T> (&v)[3]) {
+    if (near) {
+        row_sums(f, V.lo - 1, t, x, V.nx, v);
+        return;
+    }
+#pragma unroll 1
+    for (int r = 0; r < 3; ++r) {
+        const int g = t.o[r];
+        int owner = V.rank;
+        while (g < V.begin(owner)) --owner;
+        while (g >= V.begin(owner + 1)) ++owner;
+        const unsigned row = cluster_address(f, owner) + (((g - V.begin(owner) + 1) << V.lg)) * static_cast<unsigned>(sizeof(Pair<T>));
+        Pair<T> p[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+            get(row + image_column(g, (x - 1 + k) & (V.nx - 1), V.nx) * static_cast<unsigned>(sizeof(Pair<T>)), p[k]);
+        add_row(v, r, t.w[r], p[0], p[1], p[2]);
+    }
+}
+
+// Two consecutive elements, in one read when the field is aligned for it.
+template <typename T>
+__device__ __forceinline__ Pair<T> load_two(const T* p, bool aligned) {
+    if (aligned) return *reinterpret_cast<const Pair<T>*>(p);
+    return {p[0], p[1]};
+}
+
+// The units of a CTA's first and last row come first: their points are sent early in a half-sweep and
+// arrive while the others are updated.
+__device__ __forceinline__ int unit_row(int k, int n) { return k == 0 ? 0 : (k == 1 ? n - 1 : k - 1); }
+
+// One visit of a split level in a V-cycle.  up: prolongation of level l + 1's solution and
+// relaxation; down: relaxation, the residual and its restriction to level l + 1, whose
+// solution is zeroed.  Both: the end of one cycle and the start of the next on the first
+// level, whose systems stay in registers in between.  A thread holds up to kResidentSlots
+// units; e: iterations exchanged before.
+template <typename T>
+__device__ __forceinline__ void split_visit(const ResidentCycle<T>& c, int l, int e, bool up, bool down) {
+    constexpr int kPair = sizeof(Pair<T>);
+    ResidentHead& S = resident_head();
+    const ResidentLevel<T>& L = c.lv[l];
+    const ResidentLevel<T>& N = c.lv[l + 1];
+    const Slab V = slab_of<T>(c, l), W = slab_of<T>(c, l + 1);
+    const int nx = V.nx, lg = V.lg, h = nx >> 1, thread = threadIdx.x, rank = V.rank, u = L.u;
+    const bool whole = N.rows == 0, near = L.near != 0;
+    // the thread's units; the first level's systems come from global memory
+    const int count = V.n << (lg - 1);
+    const int active = min(kResidentThreads, (count + 31) & ~31);  // threads with units, rounded to warps
+    const int slots = (count + kResidentThreads - 1) / kResidentThreads;
+    Unit m[kResidentSlots];
+    Point<T> p[2][kResidentSlots];
+    bool in[kResidentSlots], top[kResidentSlots], bottom[kResidentSlots];  // a unit in the slot; in the first, the last own
+                                                                           // row with a CTA beyond it
+#pragma unroll
+    for (int s = 0; s < kResidentSlots; ++s) {
+        if (s >= slots) break;
+        int k = thread + s * kResidentThreads;
+        in[s] = k < count;
+        k = min(k, count - 1);  // (a thread without a unit computes the last one's again)
+        const int row = unit_row(k >> (lg - 1), V.n), j = k & (h - 1);
+        m[s] = make_unit<T>(u + ((row + 1) << lg) * kPair, V.lo + row, j, nx, V.ny);
+        top[s] = in[s] && row == 0 && V.above();
+        bottom[s] = in[s] && row == V.n - 1 && V.below();
+        if (l == c.first) {
+            const int P = nx * V.ny, at = ((V.lo + row) << lg) + 2 * j;
+            const T* A = L.A + 3 * static_cast<size_t>(blockIdx.y) * P;
+            const T* B = L.B + 2 * static_cast<size_t>(blockIdx.y) * P;
+            const bool wide = ((reinterpret_cast<size_t>(A) | reinterpret_cast<size_t>(B)) & (2 * sizeof(T) - 1)) == 0;
+            A += at;
+            B += at;
+            const Pair<T> h0 = load_two(A, wide), h1 = load_two(A + P, wide), h2 = load_two(A + 2 * P, wide);
+            const Pair<T> bx = load_two(B, wide), by = load_two(B + P, wide);
+            const bool odd = m[s].odd;
+            p[0][s] = {point_system(odd ? h0.y : h0.x, odd ? h1.y : h1.x, odd ? h2.y : h2.x, L.w.w00),
+                       {odd ? bx.y : bx.x, odd ? by.y : by.x}};
+            p[1][s] = {point_system(odd ? h0.x : h0.y, odd ? h1.x : h1.y, odd ? h2.x : h2.y, L.w.w00),
+                       {odd ? bx.x : bx.y, odd ? by.x : by.y}};
+        } else {
+            const int i = (row << lg) + j;
+            p[0][s] = {load_system<T>(L.a, L.own, i), pair_at<T>(L.b + i * kPair)};
+            p[1][s] = {load_system<T>(L.a, L.own, i + h), pair_at<T>(L.b + (i + h) * kPair)};
+        }
+    }
+    // offset of the halo row of the CTA above that copies the first own row, minus that row's here;
+    // the same for the last own row and the CTA below
+    const unsigned above = (V.above() ? cluster_address(0, rank - 1) : 0) + (V.lo - V.begin(rank - 1)) * nx * kPair;
+    const unsigned below = (V.below() ? cluster_address(0, rank + 1) : 0) - V.n * nx * kPair;
+    if (up) {
+        if (whole) {
+            // CTA 0's solution: this CTA's rows need its rows lowest .. highest
+            if (rank > 0) {
+                const unsigned source = cluster_address(N.u, 0);
+                const int lowest = taps_at<T>(L.up, 0).o[0] << N.lg, highest = (taps_at<T>(L.up, V.n - 1).o[2] + 1) << N.lg;
+                for (int i = lowest + thread; i < highest; i += kResidentThreads)
+                    get(source + i * kPair, pair_at<T>(N.u + i * kPair));
+            }
+            __syncthreads();
+        }
+#pragma unroll
+        for (int s = 0; s < kResidentSlots; ++s) {
+            if (s >= slots) break;
+            const int k = min(thread + s * kResidentThreads, count - 1);
+            const int row = unit_row(k >> (lg - 1), V.n), j = k & (h - 1);
+            Pair<T> v[3];
+            if (whole) row_sums(N.u, 0, taps_at<T>(L.up, row), j, N.nx, v);
+            else slab_sums(W, N.u, near, taps_at<T>(L.up, row), j, v);
+#pragma unroll
+            for (int colour = 0; colour < 2; ++colour) {
+                const int q = m[s].q[colour];
+                const Pair<T> d = doubled(v, false, m[s].odd == (colour == 0)), b = pair_at<T>(q), z{b.x + d.x, b.y + d.y};
+                if (in[s]) pair_at<T>(q) = z;
+                put(top[s], above + q, z);
+                put(bottom[s], below + q, z);
+            }
+        }
+        cooperative_groups::this_cluster().sync();
+    }
+    if (thread < active) {
+        // the half-sweeps of colour 1 use barrier 0, those of colour 0 barrier 1
+        const unsigned barrier = shared_address(S.barriers);
+        const int bytes = nx * static_cast<int>(sizeof(T)) * ((V.above() ? 1 : 0) + (V.below() ? 1 : 0));
+        unsigned above_barrier = 0, below_barrier = 0;
+        if (V.above()) above_barrier = cluster_address(0, rank - 1);
+        if (V.below()) below_barrier = cluster_address(0, rank + 1);
+        const Weights<T> w = L.w;
+        const int end = e + c.nit * ((up ? 1 : 0) + (down ? 1 : 0));
+        auto half_sweep = [&](auto colour_) {
+            constexpr int colour = decltype(colour_)::value, mine = colour ? 0 : 8, theirs = 8 - mine;
+            asm volatile(
+                "{\n\t.reg .pred p;\n\tsetp.eq.u32 p, %0, 0;\n\t"
+                "@p mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 _, [%1], %2;\n\t}" ::"r"(thread),
+                "r"(barrier + mine), "r"(bytes)
+                : "memory");
+            await_exchange(barrier + theirs, (colour ? e - 1 : e) & 1, &S.lost);
+#pragma unroll
+            for (int s = 0; s < kResidentSlots; ++s) {
+                if (s >= slots) break;
+                // (as if h0 and h1 changed: the sums h + w00 of eight points would not fit the registers)
+                if constexpr (sizeof(T) == 8) asm volatile("" : "+d"(p[colour][s].s.h0), "+d"(p[colour][s].s.h1));
+                const int q = m[s].q[colour];
+                const Pair<T> v = relaxed<colour>(m[s], p[colour][s], w);
+                if (in[s]) pair_at<T>(q) = v;
+                if (s * kResidentThreads < nx) {  // the units of the first and the last row
+                    send(top[s], above + q, above_barrier + mine, v);
+                    send(bottom[s], below + q, below_barrier + mine, v);
+                }
+            }
+            asm volatile("bar.sync 3, %0;" ::"r"(active) : "memory");
+        };
+#pragma unroll 1
+        for (; e < end; ++e) {
+            half_sweep(std::integral_constant<int, 1>{});
+            half_sweep(std::integral_constant<int, 0>{});
+        }
+        await_exchange(barrier + 8, (e - 1) & 1, &S.lost);
+        if (down) {
+            const Weights<T> g = L.g;
+            const int r = L.r - u;
+#pragma unroll
+            for (int s = 0; s < kResidentSlots; ++s) {
+                if (s >= slots) break;
+#pragma unroll
+                for (int colour = 0; colour < 2; ++colour) {
+                    const int q = m[s].q[colour] + r;
+                    const Pair<T> z = colour ? residual<1>(m[s], p[1][s], g) : residual<0>(m[s], p[0][s], g);
+                    if (in[s]) pair_at<T>(q) = z;
+                    if (s * kResidentThreads < nx) {
+                        put(top[s], above + q, z);
+                        put(bottom[s], below + q, z);
+                    }
+                }
+            }
+        }
+    }
+    if (!down) {
+        // the next prolongation reads this CTA's rows and halo rows only, unless they are not near
+        if (l > c.first && c.lv[l - 1].near != 0) __syncthreads();
+        else cooperative_groups::this_cluster().sync();
+        return;
+    }
+    // the next level's solution starts from zero (a neighbour writes its halo rows only after the barrier)
+    if (!whole || rank == 0) {
+        const int n = whole ? N.own : (N.rows + 2) << N.lg;
+        for (int i = thread; i < n; i += kResidentThreads) pair_at<T>(N.u + i * kPair) = Pair<T>{T(0), T(0)};
+    }
+    cooperative_groups::this_cluster().sync();
+    const unsigned home = whole ? cluster_address(N.b + (W.lo << N.lg) * kPair, 0) : 0;  // the rows of a whole level go to CTA 0
+    for (int i = thread; i < (W.n << N.lg); i += kResidentThreads) {
+        const int X = i & (N.nx - 1), row = i >> N.lg, at = (row * N.nx + image_column(W.lo + row, X, N.nx)) * kPair;
+        Pair<T> v[3];
+        slab_sums(V, L.r, near, taps_at<T>(L.down, row), 2 * X + 1, v);
+        if (whole) put(true, home + at, halved(v, false));
+        else pair_at<T>(N.b + at) = halved(v, false);
+    }
+    if (whole || !near) cooperative_groups::this_cluster().sync();
+    else __syncthreads();
+}
+
+// c.cycles V-cycles from level c.first on, one cluster per batch element (blockIdx.y).
+template <typename T, int CTAS>
+__global__ void __launch_bounds__(kResidentThreads, CTAS) k_resident_cycles(const __grid_constant__ ResidentCycle<T> c) {
+    constexpr int kPair = sizeof(Pair<T>);
     csg::pdl_begin();
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    T* base = reinterpret_cast<T*>(smem_raw);
-    const int bi = blockIdx.x;
-    int words = 0;
-    for (int l = c.first; l <= c.last; ++l) {
-        words += 9 * c.lv[l].nx * c.lv[l].ny;
+    ResidentHead& S = resident_head();
+    const int rank = blockIdx.x;  // the grid's x dimension is one cluster
+    const size_t bi = blockIdx.y;
+    const bool split = c.local > c.first;
+    if (threadIdx.x == 0) {
+        S.lost = 0;
+        const unsigned barrier = shared_address(S.barriers);
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(barrier) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(barrier + 8) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    // neighbour offsets of every point of every level, after the fields (16-byte aligned)
-    int4* table = reinterpret_cast<int4*>(smem_raw + ((static_cast<size_t>(words) * sizeof(T) + 15) & ~size_t(15)));
-    for (int l = c.first, toff = 0; l <= c.last; ++l) {
-        const CoarseLevel<T>& L = c.lv[l];
-        const CoarseLevel<T> S = shared_level(L, base);
+    // systems of every level (the first split level's are read when it is visited) and the
+    // first level's b and u
+    for (int l = c.first; l <= c.last; ++l) {
+        const ResidentLevel<T>& L = c.lv[l];
         const int P = L.nx * L.ny;
-        for (int j = threadIdx.x; j < 3 * P; j += blockDim.x)
-            const_cast<T*>(S.A)[j] = L.A[3 * static_cast<size_t>(bi) * P + j];
-        if (l == c.first)
-            for (int j = threadIdx.x; j < 2 * P; j += blockDim.x) {
-                S.B[j] = L.B[2 * static_cast<size_t>(bi) * P + j];
-                S.U[j] = L.U[2 * static_cast<size_t>(bi) * P + j];
+        const T* A = L.A + 3 * bi * P;
+        const Slab V(L.lg, L.nx, L.ny, rank, c.lgsize);
+        if (L.rows > 0) {
+            const int g0 = V.lo << L.lg;
+            if (l == c.first) {
+                // the image of u with its halo rows (rows outside the grid are never read)
+                const T* U = L.U + 2 * bi * P;
+                for (int j = threadIdx.x; j < (V.n + 2) << L.lg; j += kResidentThreads) {
+                    const int row = j >> L.lg, g = V.lo - 1 + row, x = j & (L.nx - 1), i = (g << L.lg) + x;
+                    if (g >= 0 && g < L.ny)
+                        pair_at<T>(L.u + ((row << L.lg) + image_column(g, x, L.nx)) * kPair) = Pair<T>{U[i], U[P + i]};
+                }
+            } else {
+                for (int j = threadIdx.x; j < V.n << L.lg; j += kResidentThreads) {
+                    const int row = j >> L.lg, i = g0 + j;
+                    store_system(L.a, L.own, (row << L.lg) + image_column(V.lo + row, j & (L.nx - 1), L.nx),
+                                 point_system(A[i], A[P + i], A[2 * P + i], L.w.w00));
+                }
             }
-        for (int i = threadIdx.x; i < P; i += blockDim.x) {
-            const Nbr4 n = neighbours(i % L.nx, i / L.nx, L.nx, L.ny);
-            table[toff + i] = make_int4(n.xm, n.xp, n.ym, n.yp);
+        } else if (rank == 0) {
+            for (int i = threadIdx.x; i < P; i += kResidentThreads) {
+                const int y = i >> L.lg, q = (y << L.lg) + image_column(y, i & (L.nx - 1), L.nx);
+                store_system(L.a, L.own, q, point_system(A[i], A[P + i], A[2 * P + i], L.w.w00));
+                if (l == c.first) {
+                    const T* B = L.B + 2 * bi * P;
+                    const T* U = L.U + 2 * bi * P;
+                    pair_at<T>(L.b + q * kPair) = Pair<T>{B[i], B[P + i]};
+                    pair_at<T>(L.u + q * kPair) = Pair<T>{U[i], U[P + i]};
+                }
+            }
         }
-        toff += P;
-    }
-    __syncthreads();
-    int toff = 0;
-    int level_toff[kMaxLevels];
-    for (int l = c.first; l <= c.last; ++l) {
-        level_toff[l] = toff;
-        toff += c.lv[l].nx * c.lv[l].ny;
-    }
-    // resize taps per level pair: restriction rows/columns of level l + 1, prolongation rows/columns of l
-    AxisTaps<T>* taps = reinterpret_cast<AxisTaps<T>*>(table + toff);
-    int down_rows[kMaxLevels], down_cols[kMaxLevels], up_rows[kMaxLevels], up_cols[kMaxLevels];
-    {
-        int at = 0;
-        for (int l = c.first; l < c.last; ++l) {
-            const CoarseLevel<T>& L = c.lv[l];
-            const CoarseLevel<T>& N = c.lv[l + 1];
-            down_rows[l] = at;
-            at += N.ny;
-            down_cols[l] = at;
-            at += N.nx;
-            up_rows[l] = at;
-            at += L.ny;
-            up_cols[l] = at;
-            at += L.nx;
-            for (int k = threadIdx.x; k < N.ny + N.nx + L.ny + L.nx; k += blockDim.x) {
-                AxisTaps<T> t;
-                if (k < N.ny) t = row_taps<T>(k, L.ny, N.ny, L.nx);
-                else if (k < N.ny + N.nx) t = col_taps<T>(k - N.ny, L.nx, N.nx);
-                else if (k < N.ny + N.nx + L.ny) t = row_taps<T>(k - N.ny - N.nx, N.ny, L.ny, N.nx);
-                else t = col_taps<T>(k - N.ny - N.nx - L.ny, N.nx, L.nx);
-                taps[down_rows[l] + k] = t;
+        // row taps (row numbers and weights) of the rows this CTA restricts to and prolongates to
+        if (l < c.last) {
+            const ResidentLevel<T>& N = c.lv[l + 1];
+            const bool whole = L.rows == 0;
+            const Slab W(N.lg, N.nx, N.ny, rank, c.lgsize);
+            const int nlo = whole ? 0 : W.lo, nn = whole ? N.ny : W.n, lo = whole ? 0 : V.lo, n = whole ? L.ny : V.n;
+            for (int k = threadIdx.x; k < nn + n; k += kResidentThreads) {
+                AxisTaps<T>* taps = reinterpret_cast<AxisTaps<T>*>(resident_smem + (k < nn ? L.down : L.up));
+                if (k < nn) taps[k] = row_taps<T>(nlo + k, L.ny, N.ny, 1);
+                else taps[k - nn] = row_taps<T>(lo + k - nn, N.ny, L.ny, 1);
             }
         }
     }
-    __syncthreads();
-    // levels from `tail` on hold at most 32 points: warp 0 runs them with warp barriers
-    int tail = c.last;
-    while (tail > c.first && c.lv[tail - 1].nx * c.lv[tail - 1].ny <= 32) --tail;
-    for (int l = c.first; l < tail; ++l)
-        coarse_down<false>(c, l, base, table + level_toff[l], taps + down_rows[l], taps + down_cols[l]);
-    if (threadIdx.x < 32) {
-        for (int l = tail; l < c.last; ++l)
-            coarse_down<true>(c, l, base, table + level_toff[l], taps + down_rows[l], taps + down_cols[l]);
-        table_relax<true>(shared_level(c.lv[c.last], base), table + level_toff[c.last], c.nit);
-        for (int l = c.last; l-- > tail;)
-            coarse_up<true>(c, l, base, table + level_toff[l], taps + up_rows[l], taps + up_cols[l]);
+    if (split) cooperative_groups::this_cluster().sync();
+    else __syncthreads();
+    // Down the split levels, the levels of CTA 0, up again; on the first level the end of a cycle
+    // and the start of the next are one visit.  (One call of each visit, as they are inlined:
+    // behind a call every half-sweep takes 160 cycles more.)
+    int e = 0, l = c.first, cycle = 0;  // e: iterations exchanged
+    bool up = false;
+#pragma unroll 1
+    while (true) {
+        if (l == c.local) {
+            if (rank == 0) local_cycle<T>(c);
+            if (!split) {
+                if (++cycle == c.cycles) break;
+                continue;
+            }
+            cooperative_groups::this_cluster().sync();
+            up = true;
+            --l;
+        }
+        if (l == c.first && up) ++cycle;
+        const bool down = !up || (l == c.first && cycle < c.cycles);
+        split_visit<T>(c, l, e, up, down);
+        e += c.nit * ((up ? 1 : 0) + (down ? 1 : 0));
+        if (l == c.first && cycle == c.cycles) break;
+        if (down) {
+            up = false;
+            ++l;
+        } else {
+            --l;
+        }
     }
-    __syncthreads();
-    for (int l = tail; l-- > c.first;)
-        coarse_up<false>(c, l, base, table + level_toff[l], taps + up_rows[l], taps + up_cols[l]);
-    const CoarseLevel<T>& F = c.lv[c.first];
-    const int P = F.nx * F.ny;
-    const T* su = base + F.off + 5 * P;
-    for (int j = threadIdx.x; j < 2 * P; j += blockDim.x) F.U[2 * static_cast<size_t>(bi) * P + j] = su[j];
-}
-
-// Shared memory of the coarse cycle over levels first..last (specs: (nx, ny) per level).
-template <typename T>
-size_t coarse_cycle_smem(const std::vector<std::pair<int, int>>& specs, size_t first) {
-    size_t words = 0, points = 0;
-    for (size_t l = first; l < specs.size(); ++l) {
-        words += 9 * static_cast<size_t>(specs[l].first) * specs[l].second;
-        points += static_cast<size_t>(specs[l].first) * specs[l].second;
+    const ResidentLevel<T>& F = c.lv[c.first];
+    const int P = F.nx * F.ny, halo = split ? 1 : 0;
+    T* U = F.U + 2 * bi * P;
+    // every exchange has been waited for and the cluster has met: no CTA touches another's memory past here
+    const bool lost = *reinterpret_cast<volatile int*>(&S.lost) != 0;
+    const Slab V(F.lg, F.nx, F.ny, rank, c.lgsize);
+    for (int i = threadIdx.x; i < V.n << F.lg; i += kResidentThreads) {
+        const int row = i >> F.lg;
+        const Pair<T> v =
+            pair_at<T>(F.u + (((row + halo) << F.lg) + image_column(V.lo + row, i & (F.nx - 1), F.nx)) * kPair);
+        U[(V.lo << F.lg) + i] = lost ? T(NAN) : v.x;
+        U[P + (V.lo << F.lg) + i] = lost ? T(NAN) : v.y;
     }
-    size_t taps = 0;
-    for (size_t l = first; l + 1 < specs.size(); ++l)
-        taps += static_cast<size_t>(specs[l].first + specs[l].second + specs[l + 1].first + specs[l + 1].second);
-    return ((words * sizeof(T) + 15) & ~size_t(15)) + points * sizeof(int4) + taps * sizeof(AxisTaps<T>);
 }
 
 // ------------------------------------------------ fused fine-level V-cycle legs
 //
-// On the fine levels (above kCoarsePoints points) one V-cycle leg used to be
+// On the levels too fine for a resident V-cycle one leg used to be
 // 2 nit red-black half-sweep launches plus a residual and a restriction
 // launch going down, and a prolongation plus 2 nit half-sweeps going up.
 // Here each leg of each level is one launch: a CTA copies its tile of the
@@ -1210,6 +1720,7 @@ size_t leg_smem(int nx, int ny, int halo, bool down) {
 }
 
 constexpr size_t kLegSmemMax = 200 * 1024;
+constexpr size_t kResidentSmemMax = 226 * 1024;
 // Fused legs recompute their halos: past this many CTAs per level launch (tiles x
 // batch) the separate launches are faster.  Measured on 256 x 128 sheets: in
 // float64 a batch of 16 solves in 30.0 ms with the level-0 legs separate against
@@ -1225,6 +1736,7 @@ constexpr long long leg_max_ctas() {
 // level, with __syncthreads between levels.  Each restricted level is kept in
 // shared memory (at most ~700 points x channels over all levels) as the
 // source of the next one, and written to its field.
+constexpr int kChainThreads = 1024;
 constexpr int kChainPoints = 512;  // measured: 512 beats 2,048 (7.96 vs 8.14 ms per 256 x 128 solve) and matches 128
 
 template <typename T>
@@ -1236,7 +1748,7 @@ struct ResizeChain {
 };
 
 template <typename T>
-__global__ void __launch_bounds__(kCoarseThreads) k_resize_chain(ResizeChain<T> c) {
+__global__ void __launch_bounds__(kChainThreads) k_resize_chain(ResizeChain<T> c) {
     csg::pdl_begin();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T* base = reinterpret_cast<T*>(smem_raw);
@@ -1285,7 +1797,7 @@ size_t resize_chain_smem(const ResizeChain<T>& c) {
     return ((words * sizeof(T) + 15) & ~size_t(15)) + taps * sizeof(AxisTaps<T>);
 }
 
-// Opt the leg, coarse-cycle and chain kernels in to more than 48 KB of dynamic
+// Opt the leg, resident-cycle and chain kernels in to more than 48 KB of dynamic
 // shared memory, once per type and device (the first solve on a device runs eagerly, before any capture).
 template <typename T>
 void allow_big_smem() {
@@ -1298,11 +1810,46 @@ void allow_big_smem() {
                          static_cast<int>(kLegSmemMax));
     cudaFuncSetAttribute(reinterpret_cast<const void*>(k_vcycle_up<T>), cudaFuncAttributeMaxDynamicSharedMemorySize,
                          static_cast<int>(kLegSmemMax));
-    cudaFuncSetAttribute(reinterpret_cast<const void*>(k_fmg_coarse_cycle<T>),
-                         cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kLegSmemMax));
+    for (const void* kernel : {reinterpret_cast<const void*>(k_resident_cycles<T, 1>),
+                               reinterpret_cast<const void*>(k_resident_cycles<T, sizeof(T) == 4 ? 2 : 1>)}) {
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kResidentSmemMax));
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    }
     cudaFuncSetAttribute(reinterpret_cast<const void*>(k_resize_chain<T>), cudaFuncAttributeMaxDynamicSharedMemorySize,
                          static_cast<int>(kLegSmemMax));
     done.fetch_or(bit);
+}
+
+// Largest cluster (16, 8, 4, 2 or 1 CTAs) of the resident kernel this device can hold with
+// kResidentSmemMax of shared memory per CTA, found once per device.
+template <typename T>
+int largest_cluster() {
+    static std::atomic<int> known[64];
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return 1;
+    int size = known[device].load();
+    if (size > 0) return size;
+    allow_big_smem<T>();
+    for (size = kMaxCluster; size > 1; size >>= 1) {
+        cudaLaunchAttribute attr{};
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = static_cast<unsigned>(size);
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cudaLaunchConfig_t config{};
+        config.gridDim = dim3(static_cast<unsigned>(size), 1, 1);
+        config.blockDim = dim3(kResidentThreads, 1, 1);
+        config.dynamicSmemBytes = kResidentSmemMax;
+        config.attrs = &attr;
+        config.numAttrs = 1;
+        int clusters = 0;
+        if (cudaOccupancyMaxActiveClusters(&clusters, reinterpret_cast<const void*>(k_resident_cycles<T, 1>), &config) ==
+                cudaSuccess &&
+            clusters > 0)
+            break;
+        cudaGetLastError();  // a size the device refuses is not the caller's error
+    }
+    known[device].store(size);
+    return size;
 }
 
 template <typename T>
@@ -1466,36 +2013,97 @@ struct Fmg {
         (csg::note_launch(), csg::launch_pdl(k_resize<T>, grid_for(t.first * t.second, batch * channels), kThreads, 0, s, src, dst, f.first, f.second,
                                                                                      t.first, t.second, accumulate));
     }
-    // First level of the fused coarse part: the finest level of at most
-    // kCoarsePoints points (the whole cycle when the finest level is small).
-    size_t coarse_first() const {
-        size_t l = 0;
-        while (l + 1 < buf.specs.size() &&
-               static_cast<long long>(buf.specs[l].first) * buf.specs[l].second > kCoarsePoints)
-            ++l;
-        return l;
-    }
-    void coarse_cycle(size_t first) {
-        const size_t last = buf.specs.size() - 1;
-        CoarseCycle<T> c{};
+    // The resident launch of `count` V-cycles from level `first` on, or size 0 when the level
+    // does not fit one cluster: more than kResidentPoints points for a CTA of it (256 x 128
+    // fits 16 CTAs, 512 x 256 does not), too much shared memory, or an x size that is no power of
+    // two.  A cluster has a CTA per kCoarsePoints points and no more CTAs than any split level has rows.
+    struct Resident {
+        ResidentCycle<T> c{};
+        int size = 0;
+        size_t smem = 0;
+    };
+    Resident resident(size_t first, int count) const {
+        Resident none, plan;
+        const size_t L = buf.specs.size();
+        if (L > static_cast<size_t>(kMaxLevels) || nit < 1) return none;
+        auto points = [&](size_t l) { return static_cast<long long>(buf.specs[l].first) * buf.specs[l].second; };
+        size_t local = first;
+        while (points(local) > kCoarsePoints) ++local;  // the last level is one point
+        int size = 1;
+        if (local > first) {
+            const int most = largest_cluster<T>();
+            while (size < most && points(first) > static_cast<long long>(size) * kCoarsePoints) size *= 2;
+            for (size_t l = first; l < local; ++l) {
+                if (buf.specs[l].first < 2) return none;
+                while (buf.specs[l].second < size) size /= 2;
+            }
+            while (size > 2 && static_cast<long long>(size) * batch > kPairedCtas &&
+                   2 * points(first) <= static_cast<long long>(size) * kResidentPoints)
+                size /= 2;
+            if (size < 2) return none;
+        }
+        ResidentCycle<T>& c = plan.c;
         c.first = static_cast<int>(first);
-        c.last = static_cast<int>(last);
+        c.local = static_cast<int>(local);
+        c.last = static_cast<int>(L - 1);
         c.nit = nit;
-        int off = 0;
-        for (size_t l = first; l <= last; ++l) {
+        c.cycles = count;
+        while ((1 << c.lgsize) < size) ++c.lgsize;
+        long long at = kHead;
+        auto take = [&](long long elements) {  // a byte offset of that many elements, aligned for pairs
+            const long long here = at;
+            at += (elements * static_cast<long long>(sizeof(T)) + 15) / 16 * 16;
+            return static_cast<int>(here);
+        };
+        int residual = 0;
+        for (size_t l = first; l < L; ++l) {
             double pr[5];
             params_at(l, pr);
             const MemWeights w = mem_weights(pr);
-            c.lv[l] = CoarseLevel<T>{buf.A[l], buf.B[l], buf.U[l], buf.R[l], buf.specs[l].first, buf.specs[l].second,
-                                     T(w.w00), T(w.w01), T(w.w10), reg_weights(pr, 1), off};
-            off += 9 * buf.specs[l].first * buf.specs[l].second;
+            const RegWeights g = reg_weights(pr, 1);
+            ResidentLevel<T>& V = c.lv[l];
+            V.A = buf.A[l];
+            V.B = buf.B[l];
+            V.U = buf.U[l];
+            V.nx = buf.specs[l].first;
+            V.ny = buf.specs[l].second;
+            while ((1 << V.lg) < V.nx) ++V.lg;
+            if ((1 << V.lg) != V.nx) return none;
+            const bool split = l < local;
+            V.rows = split ? (V.ny + size - 1) / size : 0;
+            const long long own = split ? static_cast<long long>(V.rows) * V.nx : points(l);
+            if (split && own > kResidentPoints) return none;
+            V.own = static_cast<int>(own);
+            if (l == first && split) residual = take(2 * (own + 2LL * V.nx));
+            V.u = take(split ? 2 * (own + 2LL * V.nx) : 2 * own);
+            V.b = l == first && split ? 0 : take(2 * own);
+            V.r = split ? residual : take(2 * own);
+            V.a = l == first && split ? 0 : take((sizeof(T) == 8 ? 5 : 4) * own);
+            const int units = V.ny * std::max(1, V.nx / 2);
+            if (!split && units > kResidentThreads) return none;  // (a level one point wide)
+            V.team = units > 64 ? kResidentThreads : units > 32 ? 64 : 32;
+            V.w = {T(w.w00), T(w.w01), T(w.w10)};
+            V.g = {T(g.w[0]), T(g.w[1]), T(g.w[2])};
+            if (l + 1 < L) {
+                const int ny1 = buf.specs[l + 1].second;
+                const int kTaps = static_cast<int>(sizeof(AxisTaps<T>) / sizeof(T));
+                V.near = split && V.ny == 2 * ny1 && ny1 % size == 0;
+                V.down = take(kTaps * (split ? (ny1 + size - 1) / size : ny1));
+                V.up = take(kTaps * (split ? V.rows : V.ny));
+            }
         }
-        allow_big_smem<T>();
-        (csg::note_launch(), csg::launch_pdl(k_fmg_coarse_cycle<T>, batch, kCoarseCycleThreads,
-                                             coarse_cycle_smem<T>(buf.specs, first), s, c));
+        if (at > kResidentSmemMax) return none;
+        plan.smem = static_cast<size_t>(at);
+        plan.size = size;
+        return plan;
     }
-    // One launch per fine leg (k_vcycle_down / k_vcycle_up) when every fine
-    // level has an even x size and the tile regions fit in shared memory.
+    void launch_resident(const Resident& plan) {
+        allow_big_smem<T>();
+        auto kernel = k_resident_cycles<T, 1>;
+        if (sizeof(T) == 4 && plan.size * batch > kPairedCtas) kernel = k_resident_cycles<T, sizeof(T) == 4 ? 2 : 1>;
+        (csg::note_launch(), csg::launch_pdl_cluster(kernel, dim3(static_cast<unsigned>(plan.size), static_cast<unsigned>(batch)),
+                                                     static_cast<unsigned>(plan.size), kResidentThreads, plan.smem, s, plan.c));
+    }
     // Level l runs as one down and one up leg launch when its tile regions fit the
     // shared memory and the per-thread point slots, and its tiles over the batch
     // stay within kLegMaxCtas CTAs (beyond that the halo recomputation costs more
@@ -1534,16 +2142,26 @@ struct Fmg {
         return dim3(static_cast<unsigned>(((nx + kTileX - 1) / kTileX) * ((ny + kTileY - 1) / kTileY)),
                     static_cast<unsigned>(batch));
     }
-    void cycle(size_t start) {
+    // `count` V-cycles from level `start` on: resident from the first level that fits a cluster,
+    // the levels above it leg by leg in every cycle.
+    void run_cycles(size_t start, int count) {
+        if (count < 1) return;
         const size_t last = buf.specs.size() - 1;
-        const size_t fused = std::max(start, coarse_first());
-        if (buf.specs.size() <= static_cast<size_t>(kMaxLevels) && fused < last) {
-            allow_big_smem<T>();
+        size_t fit = start;
+        Resident plan = resident(start, count);
+        while (plan.size == 0 && fit < last) plan = resident(++fit, 1);
+        if (plan.size > 0 && fit == start) {
+            launch_resident(plan);
+            return;
+        }
+        if (plan.size == 0) fit = last;
+        for (int c = 0; c < count; ++c) {
             // down: relax, residual, restriction (a fused leg leaves the relaxed solution in R[l]);
             // up: prolongation, relax (a fused leg reads R[l] and writes U[l])
-            for (size_t l = start; l < fused; ++l) {
+            for (size_t l = start; l < fit; ++l) {
                 const int nx = buf.specs[l].first, ny = buf.specs[l].second;
                 if (fused_leg(l)) {
+                    allow_big_smem<T>();
                     (csg::note_launch(), csg::launch_pdl(k_vcycle_down<T>, leg_grid(l), kLegThreads,
                                                          leg_smem<T>(nx, ny, 2 * nit + 2, true), s,
                                                          leg(l, buf.U[l], buf.R[l])));
@@ -1558,8 +2176,9 @@ struct Fmg {
                 const size_t P1 = static_cast<size_t>(buf.specs[l + 1].first) * buf.specs[l + 1].second;
                 cudaMemsetAsync(buf.U[l + 1], 0, 2 * P1 * batch * sizeof(T), s);
             }
-            coarse_cycle(fused);
-            for (size_t l = fused; l-- > start;) {
+            if (plan.size > 0) launch_resident(plan);
+            else relax(last);
+            for (size_t l = fit; l-- > start;) {
                 const int nx = buf.specs[l].first, ny = buf.specs[l].second;
                 if (fused_leg(l)) {
                     (csg::note_launch(), csg::launch_pdl(k_vcycle_up<T>, leg_grid(l), kLegThreads,
@@ -1570,23 +2189,6 @@ struct Fmg {
                 resize(buf.U[l + 1], l + 1, buf.U[l], l, 2, true);
                 relax(l);
             }
-            return;
-        }
-        for (size_t l = start; l < last; ++l) {
-            relax(l);
-            const int nx = buf.specs[l].first, ny = buf.specs[l].second;
-            double pr[5];
-            params_at(l, pr);
-            (csg::note_launch(), csg::launch_pdl(k_membrane_apply<T>, grid_for(nx * ny, batch), kThreads, 0, s, buf.A[l], buf.U[l], buf.B[l], buf.R[l], nx,
-                                                                               ny, reg_weights(pr, 1)));
-            resize(buf.R[l], l, buf.B[l + 1], l + 1, 2, false);
-            const size_t P1 = static_cast<size_t>(buf.specs[l + 1].first) * buf.specs[l + 1].second;
-            cudaMemsetAsync(buf.U[l + 1], 0, 2 * P1 * batch * sizeof(T), s);
-        }
-        relax(last);
-        for (size_t l = last; l-- > start;) {
-            resize(buf.U[l + 1], l + 1, buf.U[l], l, 2, true);
-            relax(l);
         }
     }
     // Solves into buf.U[0]; U[0] must already hold the initial guess (or
@@ -1617,7 +2219,7 @@ struct Fmg {
             off += c.channels * c.nx[k] * c.ny[k];
         }
         allow_big_smem<T>();
-        (csg::note_launch(), csg::launch_pdl(k_resize_chain<T>, batch, kCoarseThreads, resize_chain_smem(c), s, c));
+        (csg::note_launch(), csg::launch_pdl(k_resize_chain<T>, batch, kChainThreads, resize_chain_smem(c), s, c));
     }
     void run(bool coarse_init) {
         const size_t L = buf.specs.size();
@@ -1625,7 +2227,7 @@ struct Fmg {
         if (!coarse_init) {
             // every V-cycle writes each coarser level's right-hand side and zeroes its
             // solution before reading them, so the warm start needs no clearing
-            for (int c = 0; c < cycles; ++c) cycle(0);
+            run_cycles(0, cycles);
             return;
         }
         for (size_t l = 1; l < L; ++l) resize(l == 1 ? buf.B[0] : buf.B0[l - 1], l - 1, buf.B0[l], l, 2, false);
@@ -1645,7 +2247,7 @@ struct Fmg {
                 const size_t P = static_cast<size_t>(buf.specs[l].first) * buf.specs[l].second;
                 cudaMemcpyAsync(buf.B[l], buf.B0[l], 2 * P * batch * sizeof(T), cudaMemcpyDeviceToDevice, s);
             }
-            for (int c = 0; c < cycles; ++c) cycle(l);
+            run_cycles(l, cycles);
         }
     }
 };

@@ -42,4 +42,28 @@ inline cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, 
     return cudaLaunchKernelEx(&config, kernel, std::forward<Args>(args)...);
 }
 
+// launch_pdl of a kernel in thread-block clusters of `size` CTAs along x.
+template <typename... Params, typename... Args>
+inline cudaError_t launch_pdl_cluster(void (*kernel)(Params...), dim3 grid, unsigned size, dim3 block, size_t smem,
+                                      cudaStream_t stream, Args&&... args) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    const cudaError_t query = cudaStreamIsCapturing(stream, &capture);
+    if (query != cudaSuccess) return query;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = size;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t config{};
+    config.gridDim = grid;
+    config.blockDim = block;
+    config.dynamicSmemBytes = smem;
+    config.stream = stream;
+    config.attrs = attr;
+    config.numAttrs = capture == cudaStreamCaptureStatusActive ? 2 : 1;
+    return cudaLaunchKernelEx(&config, kernel, std::forward<Args>(args)...);
+}
+
 }  // namespace csg

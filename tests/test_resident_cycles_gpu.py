@@ -1,0 +1,115 @@
+"""Resident V-cycles against the separate relaxation, residual and transfer kernels.
+
+Every point sees the operations of the separate kernels in their order, so a solve
+must equal, bit for bit, the same V-cycles composed of those kernels: at grids on
+either side of each size rule, slabs of unequal rows, batches that change the
+cluster size, and systems whose quotients need the plain division.
+"""
+
+from __future__ import annotations
+
+import ctypes
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+PARAMS = (1.0, 1.0, 0.3, 0.0, 1e-3)
+
+
+def _levels(nx, ny):
+    sizes = [(nx, ny)]
+    while sizes[-1] != (1, 1):
+        sizes.append(((sizes[-1][0] + 1) // 2, (sizes[-1][1] + 1) // 2))
+    return sizes
+
+
+def _problem(nx, ny, batch, dtype, kind):
+    generator = torch.Generator(device="cuda").manual_seed(1000 * nx + ny)
+    hess = 0.5 + 0.1 * torch.rand(batch, 3, ny, nx, dtype=dtype, device="cuda", generator=generator)
+    hess[:, 2] *= 0.1
+    rhs = torch.randn(batch, 2, ny, nx, dtype=dtype, device="cuda", generator=generator)
+    start = torch.randn(batch, 2, ny, nx, dtype=dtype, device="cuda", generator=generator)
+    if kind == "division":  # zero numerators, and determinants outside the reciprocal's range
+        start.zero_()
+        rhs[..., ::3, :] = 0
+        hess[:, :2, ny // 2 :] *= 1e70 if dtype == torch.float64 else 1e15
+    return hess, rhs, start
+
+
+def _params(level, full):
+    sx, sy, mu, lam, ident = PARAMS
+    return (ctypes.c_double * 5)(sx * level[0] / full[0], sy * level[1] / full[1], mu, lam, ident)
+
+
+def _separate(lib, code, hess, rhs, start, cycles, nit):
+    batch, _, ny, nx = hess.shape
+    sizes = _levels(nx, ny)
+    systems = [hess]
+    for (snx, sny), (tnx, tny) in zip(sizes, sizes[1:]):
+        coarse = torch.empty(batch, 3, tny, tnx, dtype=hess.dtype, device="cuda")
+        assert lib.csg_dartel_resize(code, 3 * batch, snx, sny, systems[-1].data_ptr(), tnx, tny, coarse.data_ptr(), 0, 0) == 0
+        systems.append(coarse)
+
+    def relax(level, b, u):
+        w, h = sizes[level]
+        assert lib.csg_dartel_relax(code, batch, w, h, systems[level].data_ptr(), b.data_ptr(), _params(sizes[level], sizes[0]),
+                                    nit, u.data_ptr(), 0) == 0
+
+    def cycle(level, b, u):
+        w, h = sizes[level]
+        relax(level, b, u)
+        if level + 1 == len(sizes):
+            return
+        applied, coarse_b = torch.empty_like(u), torch.empty(batch, 2, *sizes[level + 1][::-1], dtype=u.dtype, device="cuda")
+        assert lib.csg_dartel_membrane_apply(code, batch, w, h, systems[level].data_ptr(), u.data_ptr(),
+                                             _params(sizes[level], sizes[0]), applied.data_ptr(), 0) == 0
+        left = b - applied
+        cw, ch = sizes[level + 1]
+        assert lib.csg_dartel_resize(code, 2 * batch, w, h, left.data_ptr(), cw, ch, coarse_b.data_ptr(), 0, 0) == 0
+        coarse_u = torch.zeros_like(coarse_b)
+        cycle(level + 1, coarse_b, coarse_u)
+        assert lib.csg_dartel_resize(code, 2 * batch, cw, ch, coarse_u.data_ptr(), w, h, u.data_ptr(), 1, 0) == 0
+        relax(level, b, u)
+
+    u = start.clone()
+    for _ in range(cycles):
+        cycle(0, rhs, u)
+    return u
+
+
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+@pytest.mark.parametrize(
+    "nx, ny, batch, cycles, nit, kind",
+    [
+        (1, 1, 2, 2, 1, "plain"),
+        (2, 1, 1, 1, 3, "plain"),
+        (8, 5, 3, 2, 2, "division"),
+        (32, 16, 2, 3, 3, "plain"),  # the largest grid of one CTA
+        (32, 17, 1, 2, 3, "division"),  # two CTAs, unequal rows
+        (2, 300, 1, 2, 1, "plain"),
+        (1, 300, 1, 1, 2, "plain"),  # too many rows for one unit per thread
+        (64, 32, 1, 2, 3, "division"),
+        (64, 33, 3, 2, 1, "plain"),  # transfers that read other CTAs' rows
+        (64, 32, 40, 2, 2, "plain"),  # fewer CTAs per grid; float32 two to an SM
+        (128, 65, 1, 1, 2, "plain"),
+        (256, 100, 1, 2, 1, "plain"),
+        (256, 128, 2, 2, 3, "division"),  # the largest resident grid
+        (256, 128, 10, 1, 1, "plain"),
+        (512, 64, 1, 1, 2, "plain"),
+        (256, 130, 1, 1, 1, "plain"),  # the first level in separate launches
+        (512, 256, 1, 1, 3, "plain"),
+    ],
+)
+def test_resident_cycles_equal_the_separate_kernels(native_library, dtype, nx, ny, batch, cycles, nit, kind):
+    lib = native_library
+    code = 1 if dtype == torch.float64 else 0
+    hess, rhs, start = _problem(nx, ny, batch, dtype, kind)
+    scratch = torch.empty(lib.csg_dartel_scratch_bytes(code, batch, nx, ny), dtype=torch.uint8, device="cuda")
+    u = start.clone()
+    assert lib.csg_dartel_fmg(code, batch, nx, ny, hess.data_ptr(), rhs.data_ptr(), _params((nx, ny), (nx, ny)), cycles, nit,
+                              u.data_ptr(), 1, 1, scratch.data_ptr(), scratch.numel(), 0) == 0
+    torch.cuda.synchronize()
+    assert torch.isfinite(u).all()
+    assert torch.equal(u, _separate(lib, code, hess, rhs, start, cycles, nit))
