@@ -812,7 +812,7 @@ struct Point {
 
 // The points (2 j, y) and (2 j + 1, y), one of each colour, as byte offsets in the image of u whose
 // row y starts at `row`; each is the other's x neighbour on one side.  nx = 1: the row's one
-// point, its own x neighbour.  At the grid's edges the y neighbour is the point itself.
+// point, its own x neighbour.  At the image's top and bottom the y neighbour is the point itself.
 struct Unit {
     int q[2];              // the points of colour 0 and 1
     int side[2];           // their other x neighbours
@@ -820,9 +820,9 @@ struct Unit {
     bool odd;              // the point of colour 0 is (2 j + 1, y)
 };
 template <typename T>
-__device__ __forceinline__ Unit make_unit(int row, int y, int j, int nx, int ny) {
+__device__ __forceinline__ Unit make_unit(int row, int y, int j, int nx, bool top, bool bottom) {
     constexpr int kPair = sizeof(Pair<T>);
-    const int h = nx >> 1, mask = h > 0 ? h - 1 : 0, next = (j + 1) & mask, previous = (j - 1) & mask;
+    const int h = nx >> 1, next = j + 1 >= h ? 0 : j + 1, previous = j > 0 ? j - 1 : max(h - 1, 0);
     Unit m;
     m.odd = (y & 1) != 0 && nx > 1;
     m.q[0] = row + j * kPair;
@@ -831,8 +831,8 @@ __device__ __forceinline__ Unit make_unit(int row, int y, int j, int nx, int ny)
     m.side[1] = row + (m.odd ? previous : next) * kPair;
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
-        m.above[c] = y == 0 ? m.q[c] : m.q[1 - c] - nx * kPair;
-        m.below[c] = y == ny - 1 ? m.q[c] : m.q[1 - c] + nx * kPair;
+        m.above[c] = top ? m.q[c] : m.q[1 - c] - nx * kPair;
+        m.below[c] = bottom ? m.q[c] : m.q[1 - c] + nx * kPair;
     }
     return m;
 }
@@ -933,7 +933,7 @@ __device__ __forceinline__ void local_visit(const ResidentCycle<T>& c, int l, bo
     const int y = in ? row : ny - 1;  // (a thread without a unit computes the last row's again)
     const bool has0 = in && (!same || (y & 1) == 0), has1 = in && (!same || (y & 1) != 0);
     const int u = L.u, i = y * nx + j;
-    const Unit m = make_unit<T>(u + y * nx * kPair, y, j, nx, ny);
+    const Unit m = make_unit<T>(u + y * nx * kPair, y, j, nx, y == 0, y == ny - 1);
     const Point<T> p0{load_system<T>(L.a, L.own, i), pair_at<T>(L.b + i * kPair)};
     const Point<T> p1{load_system<T>(L.a, L.own, i + h), pair_at<T>(L.b + (i + h) * kPair)};
     if (up) {
@@ -1141,7 +1141,7 @@ __device__ __forceinline__ void split_visit(const ResidentCycle<T>& c, int l, in
         in[s] = k < count;
         k = min(k, count - 1);  // (a thread without a unit computes the last one's again)
         const int row = unit_row(k >> (lg - 1), V.n), j = k & (h - 1);
-        m[s] = make_unit<T>(u + ((row + 1) << lg) * kPair, V.lo + row, j, nx, V.ny);
+        m[s] = make_unit<T>(u + ((row + 1) << lg) * kPair, V.lo + row, j, nx, V.lo + row == 0, V.lo + row == V.ny - 1);
         top[s] = in[s] && row == 0 && V.above();
         bottom[s] = in[s] && row == V.n - 1 && V.below();
         if (l == c.first) {
@@ -1390,180 +1390,28 @@ __global__ void __launch_bounds__(kResidentThreads, CTAS) k_resident_cycles(cons
     }
 }
 
-// ------------------------------------------------ fused fine-level V-cycle legs
+// ------------------------------------------------ V-cycle legs of the levels above
 //
-// On the levels too fine for a resident V-cycle one leg used to be
-// 2 nit red-black half-sweep launches plus a residual and a restriction
-// launch going down, and a prolongation plus 2 nit half-sweeps going up.
-// Here each leg of each level is one launch: a CTA copies its tile of the
-// level and a halo into shared memory, runs all the leg's steps there and
-// writes back its tile.  A red-black half-sweep reads only neighbours one
-// step away, so after k half-sweeps the values are exact everywhere at
-// least k cells inside the copied region (the true y edges reflect onto
-// copied rows and x is periodic, so only the region's cut edges shrink);
-// with a halo of 2 nit + 2 the tile and one ring round it hold exact
-// residuals for the restriction taps.  Every point sees the same operands in
-// the same order as in the separate kernels (relax_at, membrane_apply_at,
-// resize_at), so results are bit-identical; halo points are recomputed by
-// neighbouring tiles instead of exchanged.
+// A level too fine for a resident V-cycle takes one launch down (2 nit half-sweeps, the
+// residual and its restriction) and one up (the prolongation and 2 nit half-sweeps): a CTA
+// holds a tile and a halo, runs the leg's steps on them and writes back its tile.  A
+// half-sweep reads only neighbours one step away, so after k of them the values are exact
+// at least k cells inside the region's cut edges; with a halo of 2 nit + 2 the tile and one
+// ring round it hold exact residuals for the restriction taps (2 nit going up).  What lies
+// outside is computed all the same, from whatever the region's wrapped rows give, and never used.
+// The points are held as in a resident level -- systems and right-hand sides in registers,
+// u in an image split by colour -- and see the operations of the separate kernels in their
+// order, so results are bit-identical.
+//
+// Separate launches are bound by reading 56 bytes per point for each half-sweep from L2: on two
+// 512 x 256 float64 grids 6.7 us each, 104 us a V-cycle for the level, where both legs take 52
+// although they update each point 2.5 times.  A V-cycle of the whole hierarchy: 178 -> 127 us
+// (eight grids 419 -> 335, two in float32 146 -> 109, one of 1024 x 512 290 -> 195); no batch
+// was found at which the separate launches are faster.
 
-constexpr int kTileX = 32, kTileY = 16;
-
-struct TileGeom {
-    int x0, x1, y0, y1;  // the tile's interior (global, half-open)
-    int gx0, wx;         // copied columns: gx0 .. gx0 + wx - 1 (unwrapped), or all nx when full_x
-    int gy0, wy;         // copied rows (clipped to the grid)
-    bool full_x;
-};
-
-__device__ __forceinline__ TileGeom tile_geom(int nx, int ny, int halo) {
-    const int tiles_x = (nx + kTileX - 1) / kTileX;
-    TileGeom g;
-    const int tx = static_cast<int>(blockIdx.x) % tiles_x, ty = static_cast<int>(blockIdx.x) / tiles_x;
-    g.x0 = tx * kTileX;
-    g.x1 = min(nx, g.x0 + kTileX);
-    g.y0 = ty * kTileY;
-    g.y1 = min(ny, g.y0 + kTileY);
-    g.full_x = (g.x1 - g.x0) + 2 * halo >= nx;
-    g.gx0 = g.full_x ? 0 : g.x0 - halo;
-    g.wx = g.full_x ? nx : (g.x1 - g.x0) + 2 * halo;
-    g.gy0 = max(0, g.y0 - halo);
-    g.wy = min(ny, g.y1 + halo) - g.gy0;
-    return g;
-}
-
-// Image coordinates of the x neighbour of image column ix (dx = -1 / +1).
-__device__ __forceinline__ int image_x(const TileGeom& g, int ix, int dx, int nx) {
-    return g.full_x ? wrap_x(ix + dx, nx) : ix + dx;
-}
-// Image row of the y neighbour of global row gy (reflected at the grid edges).
-__device__ __forceinline__ int image_y(const TileGeom& g, int gy, int dy, int ny) {
-    return reflect_y(gy + dy, ny) - g.gy0;
-}
-
-template <typename T>
-struct FineImage {
-    T* a;  // [3][wy][wx]
-    T* b;  // [2][wy][wx]
-    T* u;  // [2][wy][wx]
-    int n;  // wx * wy
-};
-
-// Copy A, B and U of batch element bi over the tile's region into shared memory.
-template <typename T>
-__device__ void load_image(const T* __restrict__ A, const T* __restrict__ B, const T* __restrict__ U,
-                           const TileGeom& g, int nx, int ny, int bi, FineImage<T>& im) {
-    const int P = nx * ny;
-    const size_t o1 = static_cast<size_t>(bi) * P;
-    for (int q = threadIdx.x; q < im.n; q += blockDim.x) {
-        const int ix = q % g.wx, iy = q / g.wx;
-        const int gi = (g.gy0 + iy) * nx + wrap_x(g.gx0 + ix, nx);
-        for (int c = 0; c < 3; ++c) im.a[c * im.n + q] = A[3 * o1 + c * P + gi];
-        for (int c = 0; c < 2; ++c) {
-            im.b[c * im.n + q] = B[2 * o1 + c * P + gi];
-            im.u[c * im.n + q] = U[2 * o1 + c * P + gi];
-        }
-    }
-}
-
-// The points of one colour a thread owns in a leg: the r-th point of that
-// colour in row-major image order for r = threadIdx.x + j * blockDim.x (an
-// image row has an even width, so it holds wx / 2 points of each colour).
-// Each carries its image index, its neighbours' image indices and its depth,
-// the number of steps (each reading one cell away) after which it is still
-// exact: its distance to the nearest cut edge of the region (x edges unless
-// the region spans the periodic x range, y edges inside the grid); all are
-// formed once per leg instead of once per half-sweep.
-// measured on 2 maps x 256 x 128 float64: 512 threads with two points of each colour
-// solve in 8.27 ms against 9.08 ms for 256 threads with three
-constexpr int kLegPts = 2;
-constexpr int kLegThreads = 512;
-
-struct LegPoint {
-    int q;  // image index, -1 for an empty slot
-    int depth;
-    int xm, xp, ym, yp;
-};
-
-__device__ __forceinline__ LegPoint leg_point(const TileGeom& g, int nx, int ny, int colour, int r) {
-    LegPoint p{-1, 0, 0, 0, 0, 0};
-    const int half = g.wx >> 1;
-    if (r >= half * g.wy) return p;
-    const int iy = r / half;
-    const int ix = 2 * (r - iy * half) + ((colour - g.gx0 - g.gy0 - iy) & 1);
-    p.q = iy * g.wx + ix;
-    int d = 1 << 30;
-    if (!g.full_x) d = min(d, min(ix, g.wx - 1 - ix));
-    if (g.gy0 > 0) d = min(d, iy);
-    if (g.gy0 + g.wy < ny) d = min(d, g.wy - 1 - iy);
-    p.depth = d;
-    if (d >= 1) {  // every neighbour lies inside the image
-        const int gy = g.gy0 + iy;
-        p.xm = iy * g.wx + image_x(g, ix, -1, nx);
-        p.xp = iy * g.wx + image_x(g, ix, 1, nx);
-        p.ym = image_y(g, gy, -1, ny) * g.wx + ix;
-        p.yp = image_y(g, gy, 1, ny) * g.wx + ix;
-    }
-    return p;
-}
-
-struct LegPoints {
-    LegPoint c[2][kLegPts];  // by colour
-};
-
-__device__ __forceinline__ void own_points(const TileGeom& g, int nx, int ny, LegPoints& own) {
-#pragma unroll
-    for (int c = 0; c < 2; ++c)
-#pragma unroll
-        for (int j = 0; j < kLegPts; ++j) own.c[c][j] = leg_point(g, nx, ny, c, threadIdx.x + j * blockDim.x);
-}
-
-// relax_at on the image: one half-sweep of `colour` over the owned points exact after `k` steps.
-template <int COLOUR, typename T>
-__device__ __forceinline__ void image_half_sweep(FineImage<T>& im, const LegPoints& own, int k, T w00, T w01,
-                                                 T w10) {
-    T* ux = im.u;
-    T* uy = im.u + im.n;
-#pragma unroll
-    for (int j = 0; j < kLegPts; ++j) {
-        const LegPoint& p = own.c[COLOUR][j];
-        if (p.q < 0 || p.depth < k) continue;
-        const int q = p.q;
-        const T rx = im.b[q] - w01 * (ux[p.ym] + ux[p.yp]) - w10 * (ux[p.xm] + ux[p.xp]);
-        const T ry = im.b[im.n + q] - w01 * (uy[p.ym] + uy[p.yp]) - w10 * (uy[p.xm] + uy[p.xp]);
-        const T dxx = im.a[q] + w00;
-        const T dyy = im.a[im.n + q] + w00;
-        const T cr = im.a[2 * im.n + q];
-        const T det = dxx * dyy * T(1.0000000001) - cr * cr;
-        const T nxv = (dyy * rx - cr * ry) / det;
-        const T nyv = (-cr * rx + dxx * ry) / det;
-        ux[q] = nxv;
-        uy[q] = nyv;
-    }
-    __syncthreads();
-}
-
-// 2 nit half-sweeps, colour 1 first (the order of the separate relax launches).
-template <typename T>
-__device__ void image_relax(FineImage<T>& im, const LegPoints& own, int nit, T w00, T w01, T w10) {
-    for (int it = 0; it < nit; ++it) {
-        image_half_sweep<1>(im, own, 2 * it + 1, w00, w01, w10);
-        image_half_sweep<0>(im, own, 2 * it + 2, w00, w01, w10);
-    }
-}
-
-template <typename T>
-__device__ void store_tile(const FineImage<T>& im, const TileGeom& g, int nx, int ny, int bi, T* __restrict__ U) {
-    const int P = nx * ny;
-    const size_t o1 = static_cast<size_t>(bi) * P;
-    const int tw = g.x1 - g.x0, th = g.y1 - g.y0;
-    for (int q = threadIdx.x; q < tw * th; q += blockDim.x) {
-        const int gx = g.x0 + q % tw, gy = g.y0 + q / tw;
-        const int iq = (gy - g.gy0) * g.wx + (g.full_x ? gx : gx - g.gx0);
-        U[2 * o1 + gy * nx + gx] = im.u[iq];
-        U[2 * o1 + P + gy * nx + gx] = im.u[im.n + iq];
-    }
-}
+constexpr int kLegUnits = kResidentSlots * kResidentThreads;  // of a region, one row of tap weights each at most 128
+constexpr int kLegWidth = 48;                                 // columns of a region (nx when fewer); 40-64 within 2%, 80 10% slower
+constexpr int kLegRows = 128;                                 // rows at most
 
 // A leg reads the level's solution from Uin and writes its tiles to Uout, a
 // different buffer: tiles of one launch read each other's halos, so none may
@@ -1575,161 +1423,153 @@ struct FineLeg {
     const T* B;    // right-hand side [batch][2][ny][nx]
     const T* Uin;  // solution before the leg [batch][2][ny][nx]
     T* Uout;       // solution after the leg
-    int nx, ny;
-    T w00, w01, w10;
-    RegWeights rw;
-    T* nB;  // down: the next coarser level's right-hand side (restricted residual)
-    T* nU;  // down: the next coarser level's solution (zeroed); up: the coarser solution to prolongate
-    int cnx, cny;
+    T* nB;         // down: the next coarser level's right-hand side (restricted residual)
+    T* nU;         // down: the next coarser level's solution (zeroed); up: the coarser solution to prolongate
+    int nx, ny, cnx, cny;
+    int width, halo, tw, th, tiles_x;  // region columns; tile size (tw = width = nx: whole rows)
     int nit;
+    int wide;      // the fields are aligned for pairs of elements
+    Weights<T> w, g;
 };
 
-// Down leg of level l: 2 nit half-sweeps, the residual b - (H + L) u and its
-// restriction to level l + 1, whose solution is zeroed.  Halo 2 nit + 2.
 template <typename T>
-__global__ void __launch_bounds__(kLegThreads) k_vcycle_down(FineLeg<T> L) {
+__device__ __forceinline__ void store_two(T* p, const Pair<T>& v, bool aligned) {
+    if (aligned) {
+        *reinterpret_cast<Pair<T>*>(p) = v;
+    } else {
+        p[0] = v.x;
+        p[1] = v.y;
+    }
+}
+
+template <typename T, bool DOWN>
+__global__ void __launch_bounds__(kResidentThreads, sizeof(T) == 4 ? 2 : 1)
+    k_vcycle_leg(const __grid_constant__ FineLeg<T> L) {
+    constexpr int kPair = sizeof(Pair<T>);
     csg::pdl_begin();
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int bi = blockIdx.y;
-    const TileGeom g = tile_geom(L.nx, L.ny, 2 * L.nit + 2);
-    FineImage<T> im;
-    im.n = g.wx * g.wy;
-    im.a = reinterpret_cast<T*>(smem_raw);
-    im.b = im.a + 3 * im.n;
-    im.u = im.b + 2 * im.n;
-    T* r = im.u + 2 * im.n;  // residual [2][wy][wx]
-    LegPoints own;
-    own_points(g, L.nx, L.ny, own);
-    load_image(L.A, L.B, L.Uin, g, L.nx, L.ny, bi, im);
-    __syncthreads();
-    image_relax(im, own, L.nit, L.w00, L.w01, L.w10);
-    // residual (membrane_apply_at on the image) where it is exact
-    const int kr = 2 * L.nit + 1;
-    const T w00 = T(L.rw.w[0]), w01 = T(L.rw.w[1]), w10 = T(L.rw.w[2]);
+    const int nx = L.nx, ny = L.ny, w = L.width, h = w >> 1, thread = threadIdx.x, P = nx * ny, cP = L.cnx * L.cny;
+    const int tx = static_cast<int>(blockIdx.x) % L.tiles_x, ty = static_cast<int>(blockIdx.x) / L.tiles_x;
+    const int x0 = tx * L.tw, x1 = min(nx, x0 + L.tw), y0 = ty * L.th, y1 = min(ny, y0 + L.th);
+    const int gx0 = w == nx ? 0 : x0 - L.halo, gy0 = max(0, y0 - L.halo), wy = min(ny, y1 + L.halo) - gy0;
+    const int count = h * wy, slots = (count + kResidentThreads - 1) / kResidentThreads;
+    const bool wide = L.wide != 0;
+    // shared memory: u, the residual (down), row taps
+    const int u = 0, image = wy * w * kPair, taps = DOWN ? 2 * image : image;
+    const size_t bi = blockIdx.y;
+    const T* A = L.A + 3 * bi * P;
+    const T* B = L.B + 2 * bi * P;
+    const T* Uin = L.Uin + 2 * bi * P;
+    // taps of the coarse rows whose centre tap may lie in the tile / of the region's rows
+    const int Y0 = DOWN ? max(0, (y0 - 2) * L.cny / ny - 1) : gy0;
+    const int rows = DOWN ? min(L.cny, (y1 + 2) * L.cny / ny + 2) - Y0 : wy;
+    for (int k = thread; k < rows; k += kResidentThreads)
+        reinterpret_cast<AxisTaps<T>*>(resident_smem + taps)[k] =
+            DOWN ? row_taps<T>(Y0 + k, ny, L.cny, 1) : row_taps<T>(Y0 + k, L.cny, ny, L.cnx);
+    if (!DOWN) __syncthreads();
+    Unit m[kResidentSlots];
+    Point<T> p[2][kResidentSlots];
+    bool in[kResidentSlots];
 #pragma unroll
-    for (int colour = 0; colour < 2; ++colour)
+    for (int s = 0; s < kResidentSlots; ++s) {
+        if (s >= slots) break;
+        int k = thread + s * kResidentThreads;
+        in[s] = k < count;
+        k = min(k, count - 1);  // (a thread without a unit computes the last one's again)
+        const int row = k / h, j = k - row * h, gy = gy0 + row;
+        int gx = gx0 + 2 * j;
+        gx = gx < 0 ? gx + nx : (gx >= nx ? gx - nx : gx);
+        const int at = gy * nx + gx;
+        m[s] = make_unit<T>(u + row * w * kPair, gy, j, w, row == 0, row == wy - 1);
+        const bool odd = m[s].odd;
+        const Pair<T> h0 = load_two(A + at, wide), h1 = load_two(A + P + at, wide), h2 = load_two(A + 2 * P + at, wide);
+        const Pair<T> bx = load_two(B + at, wide), by = load_two(B + P + at, wide);
+        Pair<T> ux = load_two(Uin + at, wide), uy = load_two(Uin + P + at, wide);
+        p[0][s] = {point_system(odd ? h0.y : h0.x, odd ? h1.y : h1.x, odd ? h2.y : h2.x, L.w.w00),
+                   {odd ? bx.y : bx.x, odd ? by.y : by.x}};
+        p[1][s] = {point_system(odd ? h0.x : h0.y, odd ? h1.x : h1.y, odd ? h2.x : h2.y, L.w.w00),
+                   {odd ? bx.x : bx.y, odd ? by.x : by.y}};
+        if (!DOWN) {
+            const AxisTaps<T> t = taps_at<T>(taps, row);
+            const T* f = L.nU + 2 * bi * cP;
+            const int c = gx >> 1, c0 = c > 0 ? c - 1 : L.cnx - 1, c2 = c + 1 < L.cnx ? c + 1 : 0;
+            Pair<T> v[3];
 #pragma unroll
-        for (int j = 0; j < kLegPts; ++j) {
-            const LegPoint& p = own.c[colour][j];
-            if (p.q < 0 || p.depth < kr) continue;
-            const int q = p.q;
-            T reg[2];
-            for (int c = 0; c < 2; ++c) {
-                const T* f = im.u + c * im.n;
-                reg[c] = w00 * f[q] + w01 * (f[p.ym] + f[p.yp]) + w10 * (f[p.xm] + f[p.xp]);
+            for (int r = 0; r < 3; ++r) {
+                const T* g = f + t.o[r];
+                add_row(v, r, t.w[r], Pair<T>{g[c0], g[cP + c0]}, Pair<T>{g[c], g[cP + c]}, Pair<T>{g[c2], g[cP + c2]});
             }
-            const T u0 = im.u[q], u1 = im.u[im.n + q];
-            const T a0 = reg[0] + im.a[q] * u0 + im.a[2 * im.n + q] * u1;
-            const T a1 = reg[1] + im.a[2 * im.n + q] * u0 + im.a[im.n + q] * u1;
-            r[q] = im.b[q] - a0;
-            r[im.n + q] = im.b[im.n + q] - a1;
+            const Pair<T> even = doubled(v, false, false), other = doubled(v, false, true);
+            ux = {ux.x + even.x, ux.y + other.x};
+            uy = {uy.x + even.y, uy.y + other.y};
         }
-    __syncthreads();
-    store_tile(im, g, L.nx, L.ny, bi, L.Uout);
-    // restriction (resize_at) of the residual to the coarse points whose centre tap lies in this tile
-    const int snx = L.nx, sny = L.ny, tnx = L.cnx, tny = L.cny;
-    const int X0 = max(0, (g.x0 - 2) * tnx / snx - 1), X1 = min(tnx, (g.x1 + 2) * tnx / snx + 2);
-    const int Y0 = max(0, (g.y0 - 2) * tny / sny - 1), Y1 = min(tny, (g.y1 + 2) * tny / sny + 2);
-    const int cw = X1 - X0, ch = Y1 - Y0;
-    const size_t cP = static_cast<size_t>(tnx) * tny;
-    for (int q = threadIdx.x; q < cw * ch; q += blockDim.x) {
-        const int X = X0 + q % cw, Y = Y0 + q / cw;
-        const T yl = (static_cast<T>(Y) + T(0.5)) * static_cast<T>(sny) / static_cast<T>(tny) - T(0.5);
-        const int yo = static_cast<int>(floor(yl + T(0.5)));
-        const T xl = (static_cast<T>(X) + T(0.5)) * static_cast<T>(snx) / static_cast<T>(tnx) - T(0.5);
-        const int xo = static_cast<int>(floor(xl + T(0.5)));
-        const int oy = reflect_y(yo, sny), ox = wrap_x(xo, snx);
-        if (oy < g.y0 || oy >= g.y1 || ox < g.x0 || ox >= g.x1) continue;  // another tile's coarse point
-        const T yof = static_cast<T>(yo);
-        const T yw = wt2(yof - yl), ywm = wt2(yof - T(1) - yl), ywp = wt2(yof + T(1) - yl);
-        const T xof = static_cast<T>(xo);
-        const T xw = wt2(xof - xl), xwm = wt2(xof - T(1) - xl), xwp = wt2(xof + T(1) - xl);
-        const int rm = (reflect_y(yo - 1, sny) - g.gy0) * g.wx, rc = (reflect_y(yo, sny) - g.gy0) * g.wx,
-                  rp = (reflect_y(yo + 1, sny) - g.gy0) * g.wx;
-        auto col = [&](int x) { return g.full_x ? wrap_x(x, snx) : wrap_x(x - g.gx0, snx); };
-        const int cm = col(xo - 1), cc = col(xo), cp = col(xo + 1);
-        for (int c = 0; c < 2; ++c) {
-            const T* f = r + c * im.n;
-            const T vm = ywm * f[rm + cm] + yw * f[rc + cm] + ywp * f[rp + cm];
-            const T vc = ywm * f[rm + cc] + yw * f[rc + cc] + ywp * f[rp + cc];
-            const T vp = ywm * f[rm + cp] + yw * f[rc + cp] + ywp * f[rp + cp];
-            const size_t o = (2 * static_cast<size_t>(bi) + c) * cP + static_cast<size_t>(Y) * tnx + X;
-            L.nB[o] = xwm * vm + xw * vc + xwp * vp;
-            L.nU[o] = T(0);
-        }
-    }
-}
-
-// Up leg of level l: u += prolongation of the coarser solution (resize_at,
-// accumulate), then 2 nit half-sweeps.  Halo 2 nit.
-template <typename T>
-__global__ void __launch_bounds__(kLegThreads) k_vcycle_up(FineLeg<T> L) {
-    csg::pdl_begin();
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int bi = blockIdx.y;
-    const TileGeom g = tile_geom(L.nx, L.ny, 2 * L.nit);
-    FineImage<T> im;
-    im.n = g.wx * g.wy;
-    im.a = reinterpret_cast<T*>(smem_raw);
-    im.b = im.a + 3 * im.n;
-    im.u = im.b + 2 * im.n;
-    LegPoints own;
-    own_points(g, L.nx, L.ny, own);
-    load_image(L.A, L.B, L.Uin, g, L.nx, L.ny, bi, im);
-    for (int q = threadIdx.x; q < im.n; q += blockDim.x) {
-        const int ix = q % g.wx, iy = q / g.wx;
-        const int x = wrap_x(g.gx0 + ix, L.nx), y = g.gy0 + iy;
-        // resize_at's taps and weights for this point (the same for both channels)
-        const T yl = (static_cast<T>(y) + T(0.5)) * static_cast<T>(L.cny) / static_cast<T>(L.ny) - T(0.5);
-        const int yo = static_cast<int>(floor(yl + T(0.5)));
-        const T yof = static_cast<T>(yo);
-        const T yw = wt2(yof - yl), ywm = wt2(yof - T(1) - yl), ywp = wt2(yof + T(1) - yl);
-        const int rm = reflect_y(yo - 1, L.cny) * L.cnx, rc = reflect_y(yo, L.cny) * L.cnx,
-                  rp = reflect_y(yo + 1, L.cny) * L.cnx;
-        const T xl = (static_cast<T>(x) + T(0.5)) * static_cast<T>(L.cnx) / static_cast<T>(L.nx) - T(0.5);
-        const int xo = static_cast<int>(floor(xl + T(0.5)));
-        const T xof = static_cast<T>(xo);
-        const T xw = wt2(xof - xl), xwm = wt2(xof - T(1) - xl), xwp = wt2(xof + T(1) - xl);
-        const int cm = wrap_x(xo - 1, L.cnx), cc = wrap_x(xo, L.cnx), cp = wrap_x(xo + 1, L.cnx);
-        for (int c = 0; c < 2; ++c) {
-            const T* src = L.nU + static_cast<size_t>(2 * bi + c) * L.cnx * L.cny;
-            const T vm = ywm * src[rm + cm] + yw * src[rc + cm] + ywp * src[rp + cm];
-            const T vc = ywm * src[rm + cc] + yw * src[rc + cc] + ywp * src[rp + cc];
-            const T vp = ywm * src[rm + cp] + yw * src[rc + cp] + ywp * src[rp + cp];
-            const T v = xwm * vm + xw * vc + xwp * vp;
-            im.u[c * im.n + q] = im.u[c * im.n + q] + v;
+        if (in[s]) {
+            pair_at<T>(m[s].q[0]) = {odd ? ux.y : ux.x, odd ? uy.y : uy.x};
+            pair_at<T>(m[s].q[1]) = {odd ? ux.x : ux.y, odd ? uy.x : uy.y};
         }
     }
     __syncthreads();
-    image_relax(im, own, L.nit, L.w00, L.w01, L.w10);
-    store_tile(im, g, L.nx, L.ny, bi, L.Uout);
-}
-
-// Points of the largest tile region of a level (tile plus halo, clipped to the grid).
-inline size_t leg_points(int nx, int ny, int halo) {
-    const int tw = std::min(kTileX, nx), th = std::min(kTileY, ny);
-    const int wx = tw + 2 * halo >= nx ? nx : tw + 2 * halo;
-    const int wy = std::min(ny, th + 2 * halo);
-    return static_cast<size_t>(wx) * wy;
-}
-
-// Shared memory of one leg launch: A, B, U (+ the residual going down) over the largest tile region.
-template <typename T>
-size_t leg_smem(int nx, int ny, int halo, bool down) {
-    return leg_points(nx, ny, halo) * (down ? 9 : 7) * sizeof(T);
+    auto half_sweep = [&](auto colour_) {
+        constexpr int colour = decltype(colour_)::value;
+#pragma unroll
+        for (int s = 0; s < kResidentSlots; ++s) {
+            if (s >= slots) break;
+            if constexpr (sizeof(T) == 8) asm volatile("" : "+d"(p[colour][s].s.h0), "+d"(p[colour][s].s.h1));  // (see split_visit)
+            const Pair<T> v = relaxed<colour>(m[s], p[colour][s], L.w);
+            if (in[s]) pair_at<T>(m[s].q[colour]) = v;
+        }
+        __syncthreads();
+    };
+#pragma unroll 1
+    for (int it = 0; it < L.nit; ++it) {
+        half_sweep(std::integral_constant<int, 1>{});
+        half_sweep(std::integral_constant<int, 0>{});
+    }
+    T* Uout = L.Uout + 2 * bi * P;
+#pragma unroll
+    for (int s = 0; s < kResidentSlots; ++s) {
+        if (s >= slots) break;
+        if (DOWN) {
+            const Pair<T> r0 = residual<0>(m[s], p[0][s], L.g), r1 = residual<1>(m[s], p[1][s], L.g);
+            if (in[s]) {
+                pair_at<T>(m[s].q[0] + image) = r0;
+                pair_at<T>(m[s].q[1] + image) = r1;
+            }
+        }
+        const int k = thread + s * kResidentThreads, row = k / h, x = gx0 + 2 * (k - row * h), y = gy0 + row;
+        if (k >= count || x < x0 || x >= x1 || y < y0 || y >= y1) continue;
+        const bool odd = m[s].odd;
+        const Pair<T> a = pair_at<T>(m[s].q[0]), b = pair_at<T>(m[s].q[1]);
+        store_two(Uout + y * nx + x, Pair<T>{odd ? b.x : a.x, odd ? a.x : b.x}, wide);
+        store_two(Uout + P + y * nx + x, Pair<T>{odd ? b.y : a.y, odd ? a.y : b.y}, wide);
+    }
+    if (!DOWN) return;
+    __syncthreads();
+    // restriction of the residual to the coarse points whose centre tap (2 X + 1, the row's) lies in this tile
+    const int cw = (x1 - x0) >> 1;
+    T* nB = L.nB + 2 * bi * cP;
+    T* nU = L.nU + 2 * bi * cP;
+    for (int k = thread; k < cw * rows; k += kResidentThreads) {
+        const int Y = k / cw, j = ((x0 - gx0) >> 1) + k - Y * cw, after = j + 1 >= h ? 0 : j + 1;
+        const AxisTaps<T> t = taps_at<T>(taps, Y);
+        if (t.o[1] < y0 || t.o[1] >= y1) continue;  // another tile's coarse row
+        Pair<T> v[3];
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+            const int row = image + (t.o[r] - gy0) * w * kPair, shift = (t.o[r] & 1) * h * kPair;
+            add_row(v, r, t.w[r], pair_at<T>(row + shift + j * kPair), pair_at<T>(row + h * kPair - shift + j * kPair),
+                    pair_at<T>(row + shift + after * kPair));
+        }
+        const Pair<T> z = halved(v, false);
+        const int at = (Y0 + Y) * L.cnx + (x0 >> 1) + k - Y * cw;
+        nB[at] = z.x;
+        nB[cP + at] = z.y;
+        nU[at] = T(0);
+        nU[cP + at] = T(0);
+    }
 }
 
 constexpr size_t kLegSmemMax = 200 * 1024;
 constexpr size_t kResidentSmemMax = 226 * 1024;
-// Fused legs recompute their halos: past this many CTAs per level launch (tiles x
-// batch) the separate launches are faster.  Measured on 256 x 128 sheets: in
-// float64 a batch of 16 solves in 30.0 ms with the level-0 legs separate against
-// 36.7 ms all fused (32.3 ms all separate); in float32 all fused is fastest.
-template <typename T>
-constexpr long long leg_max_ctas() {
-    return sizeof(T) == 8 ? 256 : 1024;
-}
-
 // The restriction chain of a level-l field to every coarser level at or below
 // kChainPoints points per grid, in one launch with one CTA per batch element:
 // the same resize_at per point as separate k_resize launches, level after
@@ -1806,10 +1646,8 @@ void allow_big_smem() {
     if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return;
     const unsigned long long bit = 1ULL << device;
     if (done.load() & bit) return;
-    cudaFuncSetAttribute(reinterpret_cast<const void*>(k_vcycle_down<T>), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         static_cast<int>(kLegSmemMax));
-    cudaFuncSetAttribute(reinterpret_cast<const void*>(k_vcycle_up<T>), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         static_cast<int>(kLegSmemMax));
+    for (const void* leg : {reinterpret_cast<const void*>(k_vcycle_leg<T, true>), reinterpret_cast<const void*>(k_vcycle_leg<T, false>)})
+        cudaFuncSetAttribute(leg, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kLegSmemMax));
     for (const void* kernel : {reinterpret_cast<const void*>(k_resident_cycles<T, 1>),
                                reinterpret_cast<const void*>(k_resident_cycles<T, sizeof(T) == 4 ? 2 : 1>)}) {
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kResidentSmemMax));
@@ -2104,43 +1942,50 @@ struct Fmg {
         (csg::note_launch(), csg::launch_pdl_cluster(kernel, dim3(static_cast<unsigned>(plan.size), static_cast<unsigned>(batch)),
                                                      static_cast<unsigned>(plan.size), kResidentThreads, plan.smem, s, plan.c));
     }
-    // Level l runs as one down and one up leg launch when its tile regions fit the
-    // shared memory and the per-thread point slots, and its tiles over the batch
-    // stay within kLegMaxCtas CTAs (beyond that the halo recomputation costs more
-    // than the separate launches save).
-    bool fused_leg(size_t l) const {
+    // Level l runs as one launch down and one up when its x size is even and, where a region is not
+    // the whole height of the grid, the halos leave some of its rows (nit <= 6).  `aligned`: the level's
+    // fields start at multiples of a pair.
+    bool leg(size_t l, bool down, const T* uin, T* uout, FineLeg<T>& g) const {
         const int nx = buf.specs[l].first, ny = buf.specs[l].second;
-        if (nx % 2 != 0 || leg_smem<T>(nx, ny, 2 * nit + 2, true) > kLegSmemMax ||
-            leg_points(nx, ny, 2 * nit + 2) > static_cast<size_t>(2 * kLegPts * kLegThreads))
-            return false;
-        return static_cast<long long>(leg_grid(l).x) * batch <= leg_max_ctas<T>();
-    }
-    FineLeg<T> leg(size_t l, const T* uin, T* uout) const {
+        if (nx % 2 != 0 || nit < 1 || nit > 64) return false;
+        g = FineLeg<T>{};
+        g.halo = 2 * nit + (down ? 2 : 0);
+        g.width = std::min(nx, kLegWidth);
+        const int rows = std::min(ny, std::min(kLegRows, 2 * kLegUnits / g.width));
+        g.tw = g.width == nx ? nx : g.width - 2 * g.halo;
+        g.th = rows == ny ? ny : rows - 2 * g.halo;
+        if (g.tw < 2 || g.th < 2) return false;
+        g.tiles_x = (nx + g.tw - 1) / g.tw;
         double pr[5];
         params_at(l, pr);
         const MemWeights w = mem_weights(pr);
-        FineLeg<T> g{};
+        const RegWeights r = reg_weights(pr, 1);
+        g.w = {T(w.w00), T(w.w01), T(w.w10)};
+        g.g = {T(r.w[0]), T(r.w[1]), T(r.w[2])};
         g.A = buf.A[l];
         g.B = buf.B[l];
         g.Uin = uin;
         g.Uout = uout;
-        g.nx = buf.specs[l].first;
-        g.ny = buf.specs[l].second;
-        g.w00 = T(w.w00);
-        g.w01 = T(w.w01);
-        g.w10 = T(w.w10);
-        g.rw = reg_weights(pr, 1);
+        g.nx = nx;
+        g.ny = ny;
         g.nB = buf.B[l + 1];
         g.nU = buf.U[l + 1];
         g.cnx = buf.specs[l + 1].first;
         g.cny = buf.specs[l + 1].second;
         g.nit = nit;
-        return g;
+        g.wide = ((reinterpret_cast<size_t>(g.A) | reinterpret_cast<size_t>(g.B) | reinterpret_cast<size_t>(uin) |
+                   reinterpret_cast<size_t>(uout)) %
+                  (2 * sizeof(T))) == 0;
+        return true;
     }
-    dim3 leg_grid(size_t l) const {
-        const int nx = buf.specs[l].first, ny = buf.specs[l].second;
-        return dim3(static_cast<unsigned>(((nx + kTileX - 1) / kTileX) * ((ny + kTileY - 1) / kTileY)),
-                    static_cast<unsigned>(batch));
+    template <bool DOWN>
+    void launch_leg(const FineLeg<T>& g) {
+        allow_big_smem<T>();
+        const int rows = std::min(g.ny, g.th == g.ny ? g.ny : g.th + 2 * g.halo);
+        const size_t smem = static_cast<size_t>(rows) * g.width * sizeof(Pair<T>) * (DOWN ? 2 : 1) +
+                            (rows + 8) * sizeof(AxisTaps<T>);
+        const dim3 grid(static_cast<unsigned>(g.tiles_x * ((g.ny + g.th - 1) / g.th)), static_cast<unsigned>(batch));
+        (csg::note_launch(), csg::launch_pdl(k_vcycle_leg<T, DOWN>, grid, kResidentThreads, smem, s, g));
     }
     // `count` V-cycles from level `start` on: resident from the first level that fits a cluster,
     // the levels above it leg by leg in every cycle.
@@ -2155,16 +2000,14 @@ struct Fmg {
             return;
         }
         if (plan.size == 0) fit = last;
+        FineLeg<T> g;
         for (int c = 0; c < count; ++c) {
             // down: relax, residual, restriction (a fused leg leaves the relaxed solution in R[l]);
             // up: prolongation, relax (a fused leg reads R[l] and writes U[l])
             for (size_t l = start; l < fit; ++l) {
                 const int nx = buf.specs[l].first, ny = buf.specs[l].second;
-                if (fused_leg(l)) {
-                    allow_big_smem<T>();
-                    (csg::note_launch(), csg::launch_pdl(k_vcycle_down<T>, leg_grid(l), kLegThreads,
-                                                         leg_smem<T>(nx, ny, 2 * nit + 2, true), s,
-                                                         leg(l, buf.U[l], buf.R[l])));
+                if (leg(l, false, buf.R[l], buf.U[l], g) && leg(l, true, buf.U[l], buf.R[l], g)) {
+                    launch_leg<true>(g);
                     continue;
                 }
                 relax(l);
@@ -2179,11 +2022,8 @@ struct Fmg {
             if (plan.size > 0) launch_resident(plan);
             else relax(last);
             for (size_t l = fit; l-- > start;) {
-                const int nx = buf.specs[l].first, ny = buf.specs[l].second;
-                if (fused_leg(l)) {
-                    (csg::note_launch(), csg::launch_pdl(k_vcycle_up<T>, leg_grid(l), kLegThreads,
-                                                         leg_smem<T>(nx, ny, 2 * nit, false), s,
-                                                         leg(l, buf.R[l], buf.U[l])));
+                if (leg(l, true, buf.U[l], buf.R[l], g) && leg(l, false, buf.R[l], buf.U[l], g)) {
+                    launch_leg<false>(g);
                     continue;
                 }
                 resize(buf.U[l + 1], l + 1, buf.U[l], l, 2, true);

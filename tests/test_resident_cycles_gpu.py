@@ -1,4 +1,4 @@
-"""Resident V-cycles against the separate relaxation, residual and transfer kernels.
+"""Resident V-cycles and V-cycle legs against the separate relaxation, residual and transfer kernels.
 
 Every point sees the operations of the separate kernels in their order, so a solve
 must equal, bit for bit, the same V-cycles composed of those kernels: at grids on
@@ -98,8 +98,12 @@ def _separate(lib, code, hess, rhs, start, cycles, nit):
         (256, 128, 2, 2, 3, "division"),  # the largest resident grid
         (256, 128, 10, 1, 1, "plain"),
         (512, 64, 1, 1, 2, "plain"),
-        (256, 130, 1, 1, 1, "plain"),  # the first level in separate launches
-        (512, 256, 1, 1, 3, "plain"),
+        (256, 130, 1, 1, 1, "plain"),  # the first level as two legs of tiles
+        (512, 256, 1, 1, 3, "division"),
+        (512, 131, 2, 2, 6, "plain"),  # the widest halo
+        (64, 601, 2, 1, 2, "plain"),  # tiles of whole rows
+        (2, 17000, 1, 1, 1, "plain"),
+        (512, 100, 1, 1, 7, "plain"),  # the first level in separate launches
     ],
 )
 def test_resident_cycles_equal_the_separate_kernels(native_library, dtype, nx, ny, batch, cycles, nit, kind):
