@@ -1295,54 +1295,90 @@ __global__ void __launch_bounds__(kResidentThreads, CTAS) k_resident_cycles(cons
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(barrier + 8) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    // systems of every level (the first split level's are read when it is visited) and the
-    // first level's b and u
-    for (int l = c.first; l <= c.last; ++l) {
+    // The fields and tables of all levels, each as one list over the levels with several loads in
+    // flight per thread: level by level every one waits for its loads in turn (4 us more per launch).
+    constexpr int kAhead = 4;
+    const int thread = threadIdx.x;
+    // the row's points of level l that this CTA holds systems for in shared memory (the first split
+    // level's are read when it is visited) and its first one
+    auto held = [&](int l, int& lo) {
         const ResidentLevel<T>& L = c.lv[l];
-        const int P = L.nx * L.ny;
-        const T* A = L.A + 3 * bi * P;
         const Slab V(L.lg, L.nx, L.ny, rank, c.lgsize);
-        if (L.rows > 0) {
-            const int g0 = V.lo << L.lg;
-            if (l == c.first) {
-                // the image of u with its halo rows (rows outside the grid are never read)
-                const T* U = L.U + 2 * bi * P;
-                for (int j = threadIdx.x; j < (V.n + 2) << L.lg; j += kResidentThreads) {
-                    const int row = j >> L.lg, g = V.lo - 1 + row, x = j & (L.nx - 1), i = (g << L.lg) + x;
-                    if (g >= 0 && g < L.ny)
-                        pair_at<T>(L.u + ((row << L.lg) + image_column(g, x, L.nx)) * kPair) = Pair<T>{U[i], U[P + i]};
-                }
-            } else {
-                for (int j = threadIdx.x; j < V.n << L.lg; j += kResidentThreads) {
-                    const int row = j >> L.lg, i = g0 + j;
-                    store_system(L.a, L.own, (row << L.lg) + image_column(V.lo + row, j & (L.nx - 1), L.nx),
-                                 point_system(A[i], A[P + i], A[2 * P + i], L.w.w00));
-                }
+        lo = L.rows > 0 ? V.lo : 0;
+        return L.rows > 0 ? (l > c.first ? V.n << L.lg : 0) : (rank == 0 ? L.nx * L.ny : 0);
+    };
+    int points = 0, lo;
+    for (int l = c.first; l <= c.last; ++l) points += held(l, lo);
+    for (int k0 = thread; k0 < points; k0 += kAhead * kResidentThreads) {
+        T h[kAhead][3];
+        int level[kAhead], at[kAhead];
+#pragma unroll
+        for (int s = 0; s < kAhead; ++s) {
+            int k = k0 + s * kResidentThreads, l = c.first;
+            level[s] = -1;
+            if (k >= points) continue;
+            for (int n = held(l, lo); k >= n; n = held(++l, lo)) k -= n;
+            const ResidentLevel<T>& L = c.lv[l];
+            const int P = L.nx * L.ny, row = k >> L.lg;
+            const T* A = L.A + 3 * bi * P + (lo << L.lg) + k;
+            level[s] = l;
+            at[s] = (row << L.lg) + image_column(lo + row, k & (L.nx - 1), L.nx);
+            h[s][0] = __ldg(A);
+            h[s][1] = __ldg(A + P);
+            h[s][2] = __ldg(A + 2 * P);
+        }
+#pragma unroll
+        for (int s = 0; s < kAhead; ++s)
+            if (level[s] >= 0) {
+                const ResidentLevel<T>& L = c.lv[level[s]];
+                store_system(L.a, L.own, at[s], point_system(h[s][0], h[s][1], h[s][2], L.w.w00));
             }
-        } else if (rank == 0) {
-            for (int i = threadIdx.x; i < P; i += kResidentThreads) {
-                const int y = i >> L.lg, q = (y << L.lg) + image_column(y, i & (L.nx - 1), L.nx);
-                store_system(L.a, L.own, q, point_system(A[i], A[P + i], A[2 * P + i], L.w.w00));
-                if (l == c.first) {
-                    const T* B = L.B + 2 * bi * P;
-                    const T* U = L.U + 2 * bi * P;
-                    pair_at<T>(L.b + q * kPair) = Pair<T>{B[i], B[P + i]};
-                    pair_at<T>(L.u + q * kPair) = Pair<T>{U[i], U[P + i]};
-                }
+    }
+    {
+        // the first level's u, with its halo rows when it is split (rows outside the grid are never
+        // read), and b when it is not
+        const ResidentLevel<T>& L = c.lv[c.first];
+        const Slab V(L.lg, L.nx, L.ny, rank, c.lgsize);
+        const int P = L.nx * L.ny, halo = split ? 1 : 0, total = (V.n + 2 * halo) << L.lg;
+        const T* U = L.U + 2 * bi * P;
+        const T* B = L.B + 2 * bi * P;
+        for (int j0 = thread; j0 < total; j0 += 2 * kAhead * kResidentThreads) {
+            Pair<T> v[2 * kAhead];
+#pragma unroll
+            for (int s = 0; s < 2 * kAhead; ++s) {
+                const int j = j0 + s * kResidentThreads, g = V.lo - halo + (j >> L.lg), i = (g << L.lg) + (j & (L.nx - 1));
+                if (j < total && g >= 0 && g < L.ny) v[s] = Pair<T>{U[i], U[P + i]};
+            }
+#pragma unroll
+            for (int s = 0; s < 2 * kAhead; ++s) {
+                const int j = j0 + s * kResidentThreads, row = j >> L.lg, g = V.lo - halo + row;
+                const int q = ((row << L.lg) + image_column(g, j & (L.nx - 1), L.nx)) * kPair;
+                if (j < total && g >= 0 && g < L.ny) pair_at<T>(L.u + q) = v[s];
             }
         }
-        // row taps (row numbers and weights) of the rows this CTA restricts to and prolongates to
-        if (l < c.last) {
-            const ResidentLevel<T>& N = c.lv[l + 1];
-            const bool whole = L.rows == 0;
-            const Slab W(N.lg, N.nx, N.ny, rank, c.lgsize);
-            const int nlo = whole ? 0 : W.lo, nn = whole ? N.ny : W.n, lo = whole ? 0 : V.lo, n = whole ? L.ny : V.n;
-            for (int k = threadIdx.x; k < nn + n; k += kResidentThreads) {
-                AxisTaps<T>* taps = reinterpret_cast<AxisTaps<T>*>(resident_smem + (k < nn ? L.down : L.up));
-                if (k < nn) taps[k] = row_taps<T>(nlo + k, L.ny, N.ny, 1);
-                else taps[k - nn] = row_taps<T>(lo + k - nn, N.ny, L.ny, 1);
+        if (!split)
+            for (int i = thread; i < P; i += kResidentThreads) {
+                const int y = i >> L.lg;
+                pair_at<T>(L.b + ((y << L.lg) + image_column(y, i & (L.nx - 1), L.nx)) * kPair) = Pair<T>{B[i], B[P + i]};
             }
+    }
+    // row taps (row numbers and weights) of the rows this CTA restricts to and prolongates to
+    for (int k = thread, l = c.first, base = 0; l < c.last;) {
+        const ResidentLevel<T>& L = c.lv[l];
+        const ResidentLevel<T>& N = c.lv[l + 1];
+        const bool whole = L.rows == 0;
+        const Slab V(L.lg, L.nx, L.ny, rank, c.lgsize), W(N.lg, N.nx, N.ny, rank, c.lgsize);
+        const int nn = whole ? N.ny : W.n, n = whole ? L.ny : V.n, i = k - base;
+        if (i >= nn + n) {
+            base += nn + n;
+            ++l;
+            continue;
         }
+        const bool down = i < nn;
+        const int row = down ? (whole ? 0 : W.lo) + i : (whole ? 0 : V.lo) + i - nn;
+        AxisTaps<T>* taps = reinterpret_cast<AxisTaps<T>*>(resident_smem + (down ? L.down : L.up));
+        taps[down ? i : i - nn] = row_taps<T>(row, down ? L.ny : N.ny, down ? N.ny : L.ny, 1);
+        k += kResidentThreads;
     }
     if (split) cooperative_groups::this_cluster().sync();
     else __syncthreads();
