@@ -10,12 +10,12 @@
 // float32 with one rounding per operation (compiled with --fmad=false):
 // 3-term dot products are (a0 b0 + a1 b1) + a2 b2.
 //
-// Work decomposition: one work item = (surface, candidate, tile of kTile
-// source points).  A persistent grid walks the flattened item list, so any
-// mix of surfaces of uneven size and candidate counts is one launch.  Each
-// item writes one float64 partial (block reduction); a second kernel sums
-// the partials of each (surface, candidate) in a fixed order, so costs are
-// deterministic.
+// Work decomposition: one work item = (surface, candidate, tile of source points), or
+// up to kMaxGroup consecutive tiles in a launch large enough.  A persistent grid walks the
+// flattened item list, so any mix of surfaces of uneven size and candidate counts is one
+// launch.  Each tile has one float64 partial (block reduction of its points in their order,
+// whichever order they were taken in); a second kernel sums the partials of each (surface,
+// candidate) in a fixed order, so costs are deterministic.
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
@@ -45,7 +45,7 @@ struct RotSurface {
     int n_features;              // >= 1; values are feature-major
     int n_tgt_points;            // feature stride of tgt_values
     int tiles;                   // ceil(n_src / tile)
-    long long item_begin;        // first flat work item of this surface
+    long long item_begin;        // first flat work item of this surface (ceil(tiles / group) per candidate)
 };
 
 // Up to kInlineSurfaces surfaces travel to the kernels as a launch parameter (no host-to-device
@@ -185,6 +185,12 @@ __device__ __forceinline__ float candidate_record(const float* q, const float* r
 // terms (the float32 values candidate() forms), then a bounding sphere: centre and a
 // radius that also covers the closest-polygon test's 1e-3 parametric tolerance.
 constexpr int kRecordFloats = 20;
+// Tiles whose points one CTA of a large launch takes in order of place: threads of a warp then
+// read the same triangles.  8 tiles: 22.7 -> 19.6 ms on 2 x 512 candidates of 61,442 and 102,400
+// points (with float32 reaches 24.6 -> 22.2, 23.5 with 4 tiles, 25.5 with 16).  Below kGroupItems groups there are too few for the device: 46 candidates
+// of 40,962 points are 926 groups, a wave and a half, and no faster than their 7,406 tiles.
+constexpr int kMaxGroup = 8;
+constexpr long long kGroupItems = 2400;
 constexpr int kMaxCompact = 64;  // candidates per cell whose reaches the cost scan keeps
 static_assert(kMaxCompact <= 64, "the survivors of a cell are one 64-bit mask");
 
@@ -231,6 +237,11 @@ __device__ __forceinline__ float record_reach(const float* q, const float* rec) 
     return dist > b.w ? dist - b.w : 0.0f;
 }
 
+// A reach as a multiple of kReachUnit, rounded down (at most 255): still a lower bound.  The
+// unit is a power of two, so the products are exact.
+constexpr float kReachUnit = 1.0f / 16384.0f;
+__device__ __forceinline__ unsigned reach_code(float r) { return static_cast<unsigned>(fminf(r * (1.0f / kReachUnit), 255.0f)); }
+
 // Barycentric weights of `point` in triangle t (surface_rotation.py:335-352).
 __device__ __forceinline__ void barycentric(const float* point, const float* t, float w[3]) {
     const int order[3][3] = {{1, 2, 0}, {2, 0, 1}, {0, 1, 2}};
@@ -248,129 +259,248 @@ __device__ __forceinline__ void barycentric(const float* point, const float* t, 
     }
 }
 
+// Squared difference(s) at the rotated source point q (index i): 0 and an error without a candidate.
+__device__ __forceinline__ double cost_at(const RotSurface& S, const float (&q)[3], int i, int* __restrict__ error) {
+    double contrib = 0.0;
+    const int G = S.grid_size;
+    const float half = static_cast<float>(G / 2.0);
+    int cell[3];
+    for (int k = 0; k < 3; ++k) {
+        int c = static_cast<int>(floorf((q[k] + 1.0f) * half));
+        cell[k] = c < 0 ? 0 : (c > G - 1 ? G - 1 : c);
+    }
+    const long long cid = cell[0] + static_cast<long long>(G) * (cell[1] + static_cast<long long>(G) * cell[2]);
+    const int begin = S.grid_offsets[cid], end = S.grid_offsets[cid + 1];
+    if (begin >= end) {
+        atomicExch(error, CSG_ERR_COVERAGE);
+    } else {
+        float best = INFINITY;
+        int best_face = -1;
+        float best_point[3] = {0.0f, 0.0f, 0.0f};
+        // With records: the candidate of least reach gives a distance d0 that the first
+        // minimum cannot exceed, and a candidate whose reach is clearly above sqrt(d0)
+        // cannot be it, so the scan skips it; every other candidate is tested in cell order,
+        // the one of least reach not again: of equal distances the earlier candidate counts,
+        // as without the bound.  Cells of at most kMaxCompact candidates keep a code of each
+        // reach from the first pass and test the survivors of a bit mask, so the threads of a
+        // warp loop over their own short lists.
+        //
+        // What bounds this is the L1: every thread gathers other triangles' records (79% of
+        // the wavefront peak), and a float32 reach per candidate, 256 bytes a thread, left
+        // little of it for them.  Codes of 8 bits, four candidates' records in flight and no
+        // second test of the first candidate: 25.8 -> 22.7 ms (reading the spheres twice
+        // instead of keeping reaches 34 ms; several lanes per query 30-45 ms, as the tests
+        // then run with few lanes; more warps per SM 25-30 ms, fewer 26-32 ms).
+        const int count = end - begin;
+        const bool compact = S.records != nullptr && count <= kMaxCompact;
+        unsigned reach[kMaxCompact / 4];  // four codes to a word
+        float limit = INFINITY;
+        int pick_at = -1, best_at = 0;
+        if (S.records) {
+            float least = INFINITY;
+            int pick = -1;
+            for (int k0 = 0; k0 < count; k0 += 4) {
+                int f[4];
+                float r[4];
+                unsigned codes = 0;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) f[j] = S.grid_faces[begin + min(k0 + j, count - 1)];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) r[j] = record_reach(q, S.records + kRecordFloats * static_cast<long long>(f[j]));
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    if (k0 + j < count && r[j] < least) {
+                        least = r[j];
+                        pick = f[j];
+                        pick_at = k0 + j;
+                    }
+                    codes |= reach_code(r[j]) << 8 * j;
+                }
+                if (compact) reach[k0 / 4] = codes;
+            }
+            if (pick >= 0) {
+                float point[3];
+                const float d0 = candidate_record(q, S.records + kRecordFloats * static_cast<long long>(pick), point);
+                // margins far above float32 rounding of the distances, relative to the
+                // coordinates' scale
+                const float scale = sqrtf(q[0] * q[0] + q[1] * q[1] + q[2] * q[2]);
+                if (d0 >= 0.0f && d0 < INFINITY) limit = sqrtf(d0) * 1.0001f + 1.0e-6f * scale;
+                if (d0 < best) {
+                    best = d0;
+                    best_face = pick;
+                    best_at = pick_at;
+                    best_point[0] = point[0];
+                    best_point[1] = point[1];
+                    best_point[2] = point[2];
+                }
+            }
+        }
+        auto test = [&](int at, int f) {
+            float point[3];
+            const float d = S.records ? candidate_record(q, S.records + kRecordFloats * static_cast<long long>(f), point)
+                                      : candidate(q, S.triangles + 9 * static_cast<long long>(f), point);
+            if (d < best || (d == best && at < best_at)) {
+                best = d;
+                best_at = at;
+                best_face = f;
+                best_point[0] = point[0];
+                best_point[1] = point[1];
+                best_point[2] = point[2];
+            }
+        };
+        if (compact) {
+            unsigned long long live = 0;
+            for (int k0 = 0; k0 < count; k0 += 4) {
+                const unsigned codes = reach[k0 / 4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (k0 + j < count && !(static_cast<float>(codes >> 8 * j & 255u) * kReachUnit > limit))
+                        live |= 1ull << (k0 + j);
+            }
+            if (pick_at >= 0) live &= ~(1ull << pick_at);
+            while (live) {
+                const int k = __ffsll(static_cast<long long>(live)) - 1;
+                live &= live - 1;
+                test(k, S.grid_faces[begin + k]);
+            }
+        } else {
+            for (int k = begin; k < end; ++k) {
+                const int f = S.grid_faces[k];
+                if (S.records && record_reach(q, S.records + kRecordFloats * static_cast<long long>(f)) > limit)
+                    continue;
+                if (k - begin != pick_at) test(k - begin, f);
+            }
+        }
+        if (best_face < 0) {  // every candidate produced NaN
+            best_face = S.grid_faces[begin];
+            candidate(q, S.triangles + 9 * static_cast<long long>(best_face), best_point);
+        }
+        float w[3];
+        if (S.records) {
+            const float4* r4 = reinterpret_cast<const float4*>(S.records + kRecordFloats * static_cast<long long>(best_face));
+            const float4 r0 = __ldg(r4), r1 = __ldg(r4 + 1), r2 = __ldg(r4 + 2);
+            const float c[9] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w, r2.x};
+            barycentric(best_point, c, w);
+        } else {
+            barycentric(best_point, S.triangles + 9 * static_cast<long long>(best_face), w);
+        }
+        const int* fv = S.faces + 3 * static_cast<long long>(best_face);
+        for (int f = 0; f < S.n_features; ++f) {
+            const double* tv = S.tgt_values + static_cast<long long>(f) * S.n_tgt_points;
+            const double sampled = (tv[fv[0]] * static_cast<double>(w[0]) +
+                                    tv[fv[1]] * static_cast<double>(w[1])) +
+                                   tv[fv[2]] * static_cast<double>(w[2]);
+            const double diff = S.src_values[static_cast<long long>(f) * S.n_src + i] - sampled;
+            contrib = contrib + diff * diff;
+        }
+    }
+    return contrib;
+}
+
+// Morton order of the 16^3 boxes of [-1, 1]^3: points of one box are close on the sphere.
+constexpr int kBoxes = 4096;
+__device__ __forceinline__ int box_of(const float* q) {
+    int key = 0;
+    for (int k = 0; k < 3; ++k) {
+        const int c = min(max(static_cast<int>((q[k] + 1.0f) * 8.0f), 0), 15);
+        key |= ((c & 1) | (c & 2) << 2 | (c & 4) << 4 | (c & 8) << 6) << k;
+    }
+    return key;
+}
+
+// Bytes of a group's contributions, which hold the boxes' counts before.
+__host__ __device__ constexpr size_t sort_bytes(int points) {
+    return sizeof(double) * points > sizeof(int) * kBoxes ? sizeof(double) * points : sizeof(int) * kBoxes;
+}
+
+__device__ __forceinline__ void rotated_point(const RotSurface& S, const float* m, int i, float (&q)[3]) {
+    const float px = S.src_points[3 * i], py = S.src_points[3 * i + 1], pz = S.src_points[3 * i + 2];
+    for (int j = 0; j < 3; ++j) q[j] = (px * m[3 * j] + py * m[3 * j + 1]) + pz * m[3 * j + 2];
+}
+
+
 template <int TILE>
-__global__ void __launch_bounds__(TILE) k_rotation_cost(const __grid_constant__ SurfaceTable table,
+__global__ void __launch_bounds__(TILE, 1024 / TILE) k_rotation_cost(const __grid_constant__ SurfaceTable table,
                                                         const RotSurface* __restrict__ many, int n_surfaces,
-                                                        long long n_items, int* __restrict__ error) {
+                                                        long long n_items, int group, int* __restrict__ error) {
     __shared__ double red[TILE / 32];
+    __shared__ int warp_sums[TILE / 32];
+    extern __shared__ double contrib[];  // [group * TILE]; the boxes' counts before; then order
     const RotSurface* surfaces = n_surfaces <= kInlineSurfaces ? table.s : many;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (long long item = blockIdx.x; item < n_items; item += gridDim.x) {
         // locate the surface of this item (few surfaces: linear scan)
         int s = 0;
         while (s + 1 < n_surfaces && surfaces[s + 1].item_begin <= item) ++s;
         const RotSurface& S = surfaces[s];
         const long long local = item - S.item_begin;
-        const int cand = static_cast<int>(local / S.tiles);
-        const int tile = static_cast<int>(local - static_cast<long long>(cand) * S.tiles);
-        const int i = tile * TILE + threadIdx.x;
-        double contrib = 0.0;
-        if (i < S.n_src) {
-            const float* m = S.matrices + 9 * cand;
-            const float px = S.src_points[3 * i], py = S.src_points[3 * i + 1], pz = S.src_points[3 * i + 2];
-            float q[3];
-            for (int j = 0; j < 3; ++j) q[j] = (px * m[3 * j] + py * m[3 * j + 1]) + pz * m[3 * j + 2];
-            const int G = S.grid_size;
-            const float half = static_cast<float>(G / 2.0);
-            int cell[3];
-            for (int k = 0; k < 3; ++k) {
-                int c = static_cast<int>(floorf((q[k] + 1.0f) * half));
-                cell[k] = c < 0 ? 0 : (c > G - 1 ? G - 1 : c);
+        const int groups = (S.tiles + group - 1) / group;
+        const int cand = static_cast<int>(local / groups);
+        const int tile = static_cast<int>(local - static_cast<long long>(cand) * groups) * group;
+        const int base = tile * TILE, tiles = min(group, S.tiles - tile), n = min(tiles * TILE, S.n_src - base);
+        const float* m = S.matrices + 9 * cand;
+        unsigned short* order = reinterpret_cast<unsigned short*>(reinterpret_cast<char*>(contrib) + sort_bytes(group * TILE));
+        float q[3];
+        if (group > 1) {
+            // counting sort of the group's points by box; the order inside a box does not matter
+            int* counts = reinterpret_cast<int*>(contrib);
+            for (int k = threadIdx.x; k < kBoxes; k += TILE) counts[k] = 0;
+            __syncthreads();
+            for (int k = threadIdx.x; k < n; k += TILE) {
+                rotated_point(S, m, base + k, q);
+                atomicAdd(&counts[box_of(q)], 1);
             }
-            const long long cid = cell[0] + static_cast<long long>(G) * (cell[1] + static_cast<long long>(G) * cell[2]);
-            const int begin = S.grid_offsets[cid], end = S.grid_offsets[cid + 1];
-            if (begin >= end) {
-                atomicExch(error, CSG_ERR_COVERAGE);
+            __syncthreads();
+            // exclusive scan of the counts: kBoxes / TILE consecutive ones per thread
+            constexpr int kOwn = kBoxes / TILE;
+            int sum = 0;
+            for (int k = 0; k < kOwn; ++k) sum += counts[threadIdx.x * kOwn + k];
+            int before = sum;
+            for (int off = 1; off < 32; off <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, before, off);
+                if (lane >= off) before += v;
+            }
+            if (lane == 31) warp_sums[warp] = before;
+            __syncthreads();
+            before -= sum;
+            for (int k = 0; k < warp; ++k) before += warp_sums[k];
+            for (int k = 0; k < kOwn; ++k) {
+                const int v = counts[threadIdx.x * kOwn + k];
+                counts[threadIdx.x * kOwn + k] = before;
+                before += v;
+            }
+            __syncthreads();
+            for (int k = threadIdx.x; k < n; k += TILE) {
+                rotated_point(S, m, base + k, q);
+                order[atomicAdd(&counts[box_of(q)], 1)] = static_cast<unsigned short>(k);
+            }
+            __syncthreads();
+        }
+#pragma unroll 1
+        for (int r = 0; r < tiles; ++r) {
+            const int k = r * TILE + threadIdx.x;
+            if (k < n) {
+                const int i = group > 1 ? order[k] : k;
+                rotated_point(S, m, base + i, q);
+                contrib[i] = cost_at(S, q, base + i, error);
             } else {
-                float best = INFINITY;
-                int best_face = -1;
-                float best_point[3] = {0.0f, 0.0f, 0.0f};
-                // With records: the candidate of least reach gives a distance d0 that the first
-                // minimum cannot exceed, and a candidate whose reach is clearly above sqrt(d0)
-                // cannot be it, so the scan skips it; every other candidate is tested in cell
-                // order exactly as without the bound. Cells of at most kMaxCompact candidates
-                // keep the reaches of the first pass and test the survivors of a bit mask, so
-                // the threads of a warp loop over their own short lists.
-                const int count = end - begin;
-                const bool compact = S.records != nullptr && count <= kMaxCompact;
-                float reach[kMaxCompact];
-                float limit = INFINITY;
-                if (S.records) {
-                    float least = INFINITY;
-                    int pick = -1;
-                    for (int k = 0; k < count; ++k) {
-                        const int f = S.grid_faces[begin + k];
-                        const float r = record_reach(q, S.records + kRecordFloats * static_cast<long long>(f));
-                        if (compact) reach[k] = r;
-                        if (r < least) {
-                            least = r;
-                            pick = f;
-                        }
-                    }
-                    if (pick >= 0) {
-                        float point[3];
-                        const float d0 = candidate_record(q, S.records + kRecordFloats * static_cast<long long>(pick), point);
-                        // margins far above float32 rounding of the distances, relative to the
-                        // coordinates' scale
-                        const float scale = sqrtf(q[0] * q[0] + q[1] * q[1] + q[2] * q[2]);
-                        if (d0 >= 0.0f && d0 < INFINITY) limit = sqrtf(d0) * 1.0001f + 1.0e-6f * scale;
-                    }
-                }
-                auto test = [&](int f) {
-                    float point[3];
-                    const float d = S.records ? candidate_record(q, S.records + kRecordFloats * static_cast<long long>(f), point)
-                                              : candidate(q, S.triangles + 9 * static_cast<long long>(f), point);
-                    if (d < best) {
-                        best = d;
-                        best_face = f;
-                        best_point[0] = point[0];
-                        best_point[1] = point[1];
-                        best_point[2] = point[2];
-                    }
-                };
-                if (compact) {
-                    unsigned long long live = 0;
-                    for (int k = 0; k < count; ++k)
-                        if (!(reach[k] > limit)) live |= 1ull << k;
-                    while (live) {
-                        const int k = __ffsll(static_cast<long long>(live)) - 1;
-                        live &= live - 1;
-                        test(S.grid_faces[begin + k]);
-                    }
-                } else {
-                    for (int k = begin; k < end; ++k) {
-                        const int f = S.grid_faces[k];
-                        if (S.records && record_reach(q, S.records + kRecordFloats * static_cast<long long>(f)) > limit)
-                            continue;
-                        test(f);
-                    }
-                }
-                if (best_face < 0) {  // every candidate produced NaN
-                    best_face = S.grid_faces[begin];
-                    candidate(q, S.triangles + 9 * static_cast<long long>(best_face), best_point);
-                }
-                float w[3];
-                barycentric(best_point, S.triangles + 9 * static_cast<long long>(best_face), w);
-                const int* fv = S.faces + 3 * static_cast<long long>(best_face);
-                for (int f = 0; f < S.n_features; ++f) {
-                    const double* tv = S.tgt_values + static_cast<long long>(f) * S.n_tgt_points;
-                    const double sampled = (tv[fv[0]] * static_cast<double>(w[0]) +
-                                            tv[fv[1]] * static_cast<double>(w[1])) +
-                                           tv[fv[2]] * static_cast<double>(w[2]);
-                    const double diff = S.src_values[static_cast<long long>(f) * S.n_src + i] - sampled;
-                    contrib = contrib + diff * diff;
-                }
+                contrib[k] = 0.0;
             }
         }
-        // fixed-order block reduction: warp tree, then warp 0 over warp sums
-        for (int off = 16; off > 0; off >>= 1) contrib += __shfl_down_sync(0xffffffffu, contrib, off);
-        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = contrib;
         __syncthreads();
-        if (threadIdx.x < 32) {
-            double v = threadIdx.x < TILE / 32 ? red[threadIdx.x] : 0.0;
+        for (int r = 0; r < tiles; ++r) {
+            // fixed-order block reduction: warp tree, then warp 0 over warp sums
+            double v = contrib[r * TILE + threadIdx.x];
             for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
-            if (threadIdx.x == 0) S.partials[static_cast<long long>(cand) * S.tiles + tile] = v;
+            if (lane == 0) red[warp] = v;
+            __syncthreads();
+            if (threadIdx.x < 32) {
+                v = threadIdx.x < TILE / 32 ? red[threadIdx.x] : 0.0;
+                for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+                if (threadIdx.x == 0) S.partials[static_cast<long long>(cand) * S.tiles + tile + r] = v;
+            }
+            __syncthreads();
         }
-        __syncthreads();
     }
 }
 
@@ -594,7 +724,10 @@ int csg_rotation_cost_batch(int n_surfaces, const csg_rotation_surface* surfaces
     used += 256;
     std::vector<RotSurface> host(n_surfaces);
     std::vector<long long> cost_off(n_surfaces);
-    long long items = 0, coff = 0;
+    long long items = 0, coff = 0, tile_items = 0;
+    for (int s = 0; s < n_surfaces; ++s)
+        tile_items += static_cast<long long>((surfaces[s].n_src + tile - 1) / tile) * surfaces[s].n_candidates;
+    const int group = tile_items >= kMaxGroup * kGroupItems ? kMaxGroup : 1;
     int max_c = 0;
     for (int s = 0; s < n_surfaces; ++s) {
         const csg_rotation_surface& in = surfaces[s];
@@ -617,7 +750,7 @@ int csg_rotation_cost_batch(int n_surfaces, const csg_rotation_surface* surfaces
         r.partials = reinterpret_cast<double*>(base + used);
         used += align256(sizeof(double) * static_cast<size_t>(r.tiles) * r.n_candidates);
         r.item_begin = items;
-        items += static_cast<long long>(r.tiles) * r.n_candidates;
+        items += static_cast<long long>((r.tiles + group - 1) / group) * r.n_candidates;
         cost_off[s] = coff;
         coff += r.n_candidates;
         max_c = std::max(max_c, r.n_candidates);
@@ -637,12 +770,14 @@ int csg_rotation_cost_batch(int n_surfaces, const csg_rotation_surface* surfaces
     int device = 0, sms = 0;
     CSG_CUDA_CHECK(cudaGetDevice(&device));
     CSG_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    const long long want = n_ctas > 0 ? n_ctas : static_cast<long long>(sms) * (2048 / tile);
+    const long long want = n_ctas > 0 ? n_ctas : static_cast<long long>(sms) * (1024 / tile);  // what is resident
     const unsigned blocks = static_cast<unsigned>(std::min<long long>(std::max<long long>(1, want), items));
+    // the points' contributions, and their order by place
+    const size_t smem = group > 1 ? sort_bytes(group * tile) + sizeof(unsigned short) * group * tile : sizeof(double) * tile;
     switch (tile) {
-        case 128: (csg::note_launch(), k_rotation_cost<128><<<blocks, 128, 0, st>>>(table, d_surf, n_surfaces, items, d_err)); break;
-        case 512: (csg::note_launch(), k_rotation_cost<512><<<blocks, 512, 0, st>>>(table, d_surf, n_surfaces, items, d_err)); break;
-        default: (csg::note_launch(), k_rotation_cost<256><<<blocks, 256, 0, st>>>(table, d_surf, n_surfaces, items, d_err)); break;
+        case 128: (csg::note_launch(), k_rotation_cost<128><<<blocks, 128, smem, st>>>(table, d_surf, n_surfaces, items, group, d_err)); break;
+        case 512: (csg::note_launch(), k_rotation_cost<512><<<blocks, 512, smem, st>>>(table, d_surf, n_surfaces, items, group, d_err)); break;
+        default: (csg::note_launch(), k_rotation_cost<256><<<blocks, 256, smem, st>>>(table, d_surf, n_surfaces, items, group, d_err)); break;
     }
     (csg::note_launch(), k_rotation_finalize<<<dim3((max_c + 127) / 128, n_surfaces), 128, 0, st>>>(table, d_surf, n_surfaces, costs, d_off));
     CSG_CUDA_CHECK(cudaGetLastError());

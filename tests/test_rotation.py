@@ -284,3 +284,33 @@ def test_host_driven_evaluations_equal_the_batched_costs(device_index):
         assert host.shape == (count,)
         np.testing.assert_array_equal(host, device)
         np.testing.assert_allclose(host, _oracle_cost(angles), rtol=1e-12)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tile", [128, 256, 512])
+@pytest.mark.parametrize("grid_size", [4, 24])  # cells of more candidates than a mask holds, and fewer
+@pytest.mark.parametrize("points", [1, 1290, 5000])
+def test_groups_of_tiles_equal_single_candidates(native_library, tile, grid_size, points):
+    """A launch large enough to take several tiles' points in order of place gives the costs of
+    launches that take them tile by tile, bit for bit: points that fill no group, part of one, and
+    more than one."""
+
+    import torch
+
+    from cat_surface_gpu_b200 import synthetic
+    from cat_surface_gpu_b200.surface_rotation import RotationGridIndex, batched_costs, rotation_matrices_flat
+
+    rng = np.random.default_rng(points + tile)
+    tp, tf = synthetic.unit_icosphere(3)
+    index = RotationGridIndex.from_geometry(tp, tf, grid_size=grid_size, margin=1,
+                                            include_dense_candidate_table=False).to("cuda")
+    src = rng.normal(size=(points, 3))
+    src = (src / np.linalg.norm(src, axis=1, keepdims=True)).astype(np.float32)
+    inputs = index.prepare_cost_inputs(src, np.sin(4 * src[:, 0]).astype(np.float64), np.sin(4 * tp[:, 0]))
+    few = rotation_matrices_flat(rng.uniform(-1, 1, size=(7, 3)))
+    tiles = -(-points // tile)
+    repeats = -(-8 * 2400 // (tiles * few.shape[0]))
+    many = np.tile(few, (repeats, 1))
+    alone = batched_costs([index], [inputs], matrix_sets=[few], tile=tile)[0]
+    together = batched_costs([index], [inputs], matrix_sets=[many], tile=tile)[0]
+    assert torch.equal(together, alone.repeat(repeats))
