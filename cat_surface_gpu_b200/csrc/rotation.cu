@@ -24,6 +24,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/catsurf_b200.h"
+#include "common.cuh"
 #include "errors.h"
 
 namespace {
@@ -504,31 +505,20 @@ __global__ void __launch_bounds__(TILE, 1024 / TILE) k_rotation_cost(const __gri
     }
 }
 
-__global__ void k_rotation_finalize(const __grid_constant__ SurfaceTable table, const RotSurface* __restrict__ many,
-                                    int n_surfaces, double* __restrict__ costs, const long long* __restrict__ many_offsets) {
-    const int s = blockIdx.y;
-    if (s >= n_surfaces) return;
+// The partials of one candidate, added in tile order (160 tiles: 10.3 -> 3.9 us against a thread per
+// candidate that reads them from global memory; 2 x 512 candidates of 240 and 400: 36.8 -> 6.5).
+__global__ void __launch_bounds__(csg::kOrderedThreads)
+    k_rotation_finalize(const __grid_constant__ SurfaceTable table, const RotSurface* __restrict__ many, int n_surfaces,
+                        double* __restrict__ costs, const long long* __restrict__ many_offsets) {
+    __shared__ double buf[csg::kOrderedChunk];
+    const int s = blockIdx.y, c = blockIdx.x;
     const bool inline_table = n_surfaces <= kInlineSurfaces;
     const RotSurface* surfaces = inline_table ? table.s : many;
     const long long* cost_offsets = inline_table ? table.cost_off : many_offsets;
     const RotSurface& S = surfaces[s];
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= S.n_candidates) return;
-    // the partials in tile order, loaded kAhead at a time before they are added (the
-    // additions stay in that order; the loads no longer wait on one another)
-    constexpr int kAhead = 32;
-    double total = 0.0;
-    const double* p = S.partials + static_cast<long long>(c) * S.tiles;
-    int t = 0;
-    for (; t + kAhead <= S.tiles; t += kAhead) {
-        double part[kAhead];
-#pragma unroll
-        for (int j = 0; j < kAhead; ++j) part[j] = p[t + j];
-#pragma unroll
-        for (int j = 0; j < kAhead; ++j) total += part[j];
-    }
-    for (; t < S.tiles; ++t) total += p[t];
-    costs[cost_offsets[s] + c] = total;
+    const double total = csg::ordered_sum(S.partials + static_cast<long long>(c) * S.tiles, S.tiles, buf);
+    if (threadIdx.x == 0) costs[cost_offsets[s] + c] = total;
 }
 
 size_t align256(size_t x) { return (x + 255) & ~static_cast<size_t>(255); }
@@ -779,7 +769,7 @@ int csg_rotation_cost_batch(int n_surfaces, const csg_rotation_surface* surfaces
         case 512: (csg::note_launch(), k_rotation_cost<512><<<blocks, 512, smem, st>>>(table, d_surf, n_surfaces, items, group, d_err)); break;
         default: (csg::note_launch(), k_rotation_cost<256><<<blocks, 256, smem, st>>>(table, d_surf, n_surfaces, items, group, d_err)); break;
     }
-    (csg::note_launch(), k_rotation_finalize<<<dim3((max_c + 127) / 128, n_surfaces), 128, 0, st>>>(table, d_surf, n_surfaces, costs, d_off));
+    (csg::note_launch(), k_rotation_finalize<<<dim3(max_c, n_surfaces), csg::kOrderedThreads, 0, st>>>(table, d_surf, n_surfaces, costs, d_off));
     CSG_CUDA_CHECK(cudaGetLastError());
     return CSG_OK;
 }
