@@ -36,12 +36,15 @@ namespace {
 
 constexpr int kThreads = 256;
 
+// (the remainders only for an index outside the grid: each costs ~25 instructions)
 __device__ __forceinline__ int wrap_x(int ix, int nx) {
+    if (static_cast<unsigned>(ix) < static_cast<unsigned>(nx)) return ix;
     int r = ix % nx;
     return r < 0 ? r + nx : r;
 }
 
 __device__ __forceinline__ int reflect_y(int iy, int ny) {
+    if (static_cast<unsigned>(iy) < static_cast<unsigned>(ny)) return iy;
     if (ny == 1) return 0;
     const int period = 2 * ny;
     int r = iy % period;
@@ -73,9 +76,13 @@ struct Stencil {
     }
 };
 
+// c moved by whole periods to within half a period of c22.  Less than a quarter of a period apart the
+// quotient's floor is 0 and c itself the result; only samples across the periodic seam divide.
 template <typename T>
 __device__ __forceinline__ T unwrap(T c, T c22, T period) {
-    return c - floor((c - c22) / period + T(0.5)) * period;
+    const T d = c - c22;
+    if (fabs(d) < T(0.25) * period) return c;
+    return c - floor(d / period + T(0.5)) * period;
 }
 
 struct Pt {
