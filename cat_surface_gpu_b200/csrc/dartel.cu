@@ -85,6 +85,22 @@ __device__ __forceinline__ T unwrap(T c, T c22, T period) {
     return c - floor(d / period + T(0.5)) * period;
 }
 
+// The stencil's samples (22, 12, 21, 11) of both channels, all read before the seam tests' branches,
+// behind which the second channel's reads would wait for the first's (solve 256 x 128: 4.68 -> 4.59 ms).
+template <typename T>
+struct Samples {
+    T v[2][4];
+    __device__ __forceinline__ Samples(const Stencil<T>& st, const T* __restrict__ f, int P) {
+#pragma unroll
+        for (int ch = 0; ch < 2; ++ch) {
+            v[ch][0] = f[ch * P + st.i22];
+            v[ch][1] = f[ch * P + st.i12];
+            v[ch][2] = f[ch * P + st.i21];
+            v[ch][3] = f[ch * P + st.i11];
+        }
+    }
+};
+
 struct Pt {
     int b, x, y, i;  // batch, column, row, flat index in a channel
 };
@@ -141,16 +157,15 @@ __device__ __forceinline__ void compose_at(const Stencil<T>& st, const T* __rest
                                            T* __restrict__ jc, int nx, int ny, const Pt& p) {
     const int P = nx * ny;
     const size_t o2 = static_cast<size_t>(p.b) * 2 * P, o4 = static_cast<size_t>(p.b) * 4 * P;
-    const T* Bm = b + o2;
     T* C = c + o2;
+    const Samples<T> f(st, b + o2, P);
 #pragma unroll
     for (int ch = 0; ch < 2; ++ch) {
-        const T* f = Bm + ch * P;
         const T period = static_cast<T>(ch == 0 ? nx : ny);
-        const T c22 = f[st.i22] - T(1);
-        const T c12 = unwrap(f[st.i12] - T(1), c22, period);
-        const T c21 = unwrap(f[st.i21] - T(1), c22, period);
-        const T c11 = unwrap(f[st.i11] - T(1), c22, period);
+        const T c22 = f.v[ch][0] - T(1);
+        const T c12 = unwrap(f.v[ch][1] - T(1), c22, period);
+        const T c21 = unwrap(f.v[ch][2] - T(1), c22, period);
+        const T c11 = unwrap(f.v[ch][3] - T(1), c22, period);
         C[ch * P + p.i] = (c22 * st.dx2 + c12 * st.dx1) * st.dy2 + (c21 * st.dx2 + c11 * st.dx1) * st.dy1 + T(1);
     }
     if (jc) {
@@ -2362,15 +2377,16 @@ __global__ void k_data_compose_adjoint(const T* __restrict__ f, const T* __restr
     const Stencil<T> st(F[p.i] - T(1), F[P + p.i] - T(1), nx, ny);
     T* out = pbar + o2;
     T pos_x = T(0), pos_y = T(0);
+    const Samples<T> f4(st, F, P);
+    const T adjoint[2] = {abar[o2 + p.i], abar[o2 + P + p.i]};
 #pragma unroll
     for (int ch = 0; ch < 2; ++ch) {
-        const T* fc = F + ch * P;
         const T period = static_cast<T>(ch == 0 ? nx : ny);
-        const T c22 = fc[st.i22] - T(1);
-        const T c12 = unwrap(fc[st.i12] - T(1), c22, period);
-        const T c21 = unwrap(fc[st.i21] - T(1), c22, period);
-        const T c11 = unwrap(fc[st.i11] - T(1), c22, period);
-        const T a = abar[o2 + ch * P + p.i];
+        const T c22 = f4.v[ch][0] - T(1);
+        const T c12 = unwrap(f4.v[ch][1] - T(1), c22, period);
+        const T c21 = unwrap(f4.v[ch][2] - T(1), c22, period);
+        const T c11 = unwrap(f4.v[ch][3] - T(1), c22, period);
+        const T a = adjoint[ch];
         pos_x = pos_x + a * ((c12 - c22) * st.dy2 + (c11 - c21) * st.dy1);
         pos_y = pos_y + a * ((c21 * st.dx2 + c11 * st.dx1) - (c22 * st.dx2 + c12 * st.dx1));
         T* oc = out + ch * P;
