@@ -2365,38 +2365,83 @@ __global__ void k_data_sample(const T* __restrict__ source, const T* __restrict_
 }
 
 // pbar += adjoint of C = phi_i o phi_i at every x (pbar zeroed by the caller).
+//
+// What bounds this is the float64 additions to global memory, ten per point.  Where the next
+// lane's stencil continues this one's -- everywhere but at seams and strong stretches -- the
+// right-hand samples' terms are handed to it and added to its left-hand ones, and the term of
+// the point itself joins the sample that is the point: four additions per point (32 float64 grids of
+// 256 x 128: 29.6 -> 22.2 us).
 template <typename T>
 __global__ void k_data_compose_adjoint(const T* __restrict__ f, const T* __restrict__ abar, T* __restrict__ pbar,
                                        int nx, int ny) {
     csg::pdl_begin();
     Pt p;
-    if (!point(nx, ny, p)) return;
+    const bool in = point(nx, ny, p);
     const int P = nx * ny;
-    const size_t o2 = static_cast<size_t>(p.b) * 2 * P;
+    const size_t o2 = static_cast<size_t>(blockIdx.y) * 2 * P;
     const T* F = f + o2;
-    const Stencil<T> st(F[p.i] - T(1), F[P + p.i] - T(1), nx, ny);
     T* out = pbar + o2;
-    T pos_x = T(0), pos_y = T(0);
-    const Samples<T> f4(st, F, P);
-    const T adjoint[2] = {abar[o2 + p.i], abar[o2 + P + p.i]};
+    int at[4] = {-1, -1, -1, -1};  // 22, 12, 21, 11
+    T term[2][4] = {};
+    if (in) {
+        const Stencil<T> st(F[p.i] - T(1), F[P + p.i] - T(1), nx, ny);
+        at[0] = st.i22;
+        at[1] = st.i12;
+        at[2] = st.i21;
+        at[3] = st.i11;
+        T pos[2] = {T(0), T(0)};
+        const Samples<T> f4(st, F, P);
+        const T adjoint[2] = {abar[o2 + p.i], abar[o2 + P + p.i]};
+#pragma unroll
+        for (int ch = 0; ch < 2; ++ch) {
+            const T period = static_cast<T>(ch == 0 ? nx : ny);
+            const T c22 = f4.v[ch][0] - T(1);
+            const T c12 = unwrap(f4.v[ch][1] - T(1), c22, period);
+            const T c21 = unwrap(f4.v[ch][2] - T(1), c22, period);
+            const T c11 = unwrap(f4.v[ch][3] - T(1), c22, period);
+            const T a = adjoint[ch];
+            pos[0] = pos[0] + a * ((c12 - c22) * st.dy2 + (c11 - c21) * st.dy1);
+            pos[1] = pos[1] + a * ((c21 * st.dx2 + c11 * st.dx1) - (c22 * st.dx2 + c12 * st.dx1));
+            term[ch][0] = a * (st.dx2 * st.dy2);
+            term[ch][1] = a * (st.dx1 * st.dy2);
+            term[ch][2] = a * (st.dx2 * st.dy1);
+            term[ch][3] = a * (st.dx1 * st.dy1);
+        }
+        bool apart = true;
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (apart && at[k] == p.i) {
+                term[0][k] = term[0][k] + pos[0];
+                term[1][k] = term[1][k] + pos[1];
+                apart = false;
+            }
+        if (apart) {
+            atomicAdd(out + p.i, pos[0]);
+            atomicAdd(out + P + p.i, pos[1]);
+        }
+    }
+    const int lane = threadIdx.x & 31;
+    const int next_upper = __shfl_down_sync(0xffffffffu, at[0], 1), next_lower = __shfl_down_sync(0xffffffffu, at[2], 1);
+    const bool give = in && lane < 31 && next_upper == at[1] && next_lower == at[3];
+    const int given = __shfl_up_sync(0xffffffffu, static_cast<int>(give), 1);
+    const bool take = given != 0 && lane > 0;
 #pragma unroll
     for (int ch = 0; ch < 2; ++ch) {
-        const T period = static_cast<T>(ch == 0 ? nx : ny);
-        const T c22 = f4.v[ch][0] - T(1);
-        const T c12 = unwrap(f4.v[ch][1] - T(1), c22, period);
-        const T c21 = unwrap(f4.v[ch][2] - T(1), c22, period);
-        const T c11 = unwrap(f4.v[ch][3] - T(1), c22, period);
-        const T a = adjoint[ch];
-        pos_x = pos_x + a * ((c12 - c22) * st.dy2 + (c11 - c21) * st.dy1);
-        pos_y = pos_y + a * ((c21 * st.dx2 + c11 * st.dx1) - (c22 * st.dx2 + c12 * st.dx1));
-        T* oc = out + ch * P;
-        atomicAdd(oc + st.i22, a * (st.dx2 * st.dy2));
-        atomicAdd(oc + st.i12, a * (st.dx1 * st.dy2));
-        atomicAdd(oc + st.i21, a * (st.dx2 * st.dy1));
-        atomicAdd(oc + st.i11, a * (st.dx1 * st.dy1));
+        const T upper = __shfl_up_sync(0xffffffffu, term[ch][1], 1), lower = __shfl_up_sync(0xffffffffu, term[ch][3], 1);
+        if (take) {
+            term[ch][0] = term[ch][0] + upper;
+            term[ch][2] = term[ch][2] + lower;
+        }
+        if (in) {
+            T* o = out + ch * P;
+            atomicAdd(o + at[0], term[ch][0]);
+            atomicAdd(o + at[2], term[ch][2]);
+            if (!give) {
+                atomicAdd(o + at[1], term[ch][1]);
+                atomicAdd(o + at[3], term[ch][3]);
+            }
+        }
     }
-    atomicAdd(out + p.i, pos_x);
-    atomicAdd(out + P + p.i, pos_y);
 }
 
 // grad = scale_b * s * abar (phi_0 = id + s v).

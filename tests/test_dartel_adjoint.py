@@ -143,3 +143,17 @@ def test_float32_gradient_tracks_float64(native_library):
     want = od.data_term_gradient(V, S, T, 7)
     rel = np.linalg.norm(v32.grad.cpu().numpy() - want) / np.linalg.norm(want)
     assert rel <= 1e-3  # float32 rounding (6e-8) grows through 7 squarings of the map (measured 1.4e-4)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("ny, nx", [(1, 2), (3, 2), (5, 7), (4, 32), (9, 33), (16, 128)])
+@pytest.mark.parametrize("scale", [0.05, 3.0])  # stencils that continue from lane to lane, and torn ones
+def test_gpu_gradient_on_ragged_and_torn_maps(native_library, ny, nx, scale):
+    from cat_surface_gpu_b200.dartel_adjoint import dartel_data_term
+
+    rng = np.random.default_rng(nx)
+    vel, src, tgt = scale * rng.normal(size=(2, ny, nx)), rng.normal(size=(ny, nx)), rng.normal(size=(ny, nx))
+    v = _cuda(vel).requires_grad_(True)
+    dartel_data_term(v, _cuda(src), _cuda(tgt), 3).backward()
+    want = od.data_term_gradient(vel, src, tgt, 3)
+    assert np.abs(v.grad.cpu().numpy() - want).max() <= 1e-12 * np.abs(want).max()
