@@ -114,7 +114,9 @@ __global__ void k_sum_partials(const double* __restrict__ partial, int n, double
 // registers, so an iteration is one round of gathers, the three components together, and a
 // barrier: read per iteration and component, the list put a dependent load before each of
 // 18 gathers (40,962 points: 269 -> 195 us with the barriers of an FWHM of 50 mm).
-constexpr int kHeld = 8;
+// CTAs of 128 threads spread 40,962 points evenly over 148 SMs (321 CTAs; of 256 threads 161, two on
+// 13 of the SMs): curvature sheets 361 -> 341 us in spite of twice the arrivals at each barrier.
+constexpr int kHeld = 8, kSmoothThreads = 128;
 __global__ void k_smooth_geometry_all(const float* __restrict__ in, float* __restrict__ out, float* __restrict__ tmp,
                                       const int* __restrict__ off, const int* __restrict__ nbr, int n, int iterations,
                                       csg::Control* ctl, unsigned long long timeout_ns) {
@@ -267,15 +269,15 @@ __global__ void k_smooth_values_all(const double* __restrict__ in, double* __res
     }
 }
 
-// Grid of a cooperative launch of `kernel`: as many kThreads-blocks as `work`
+// Grid of a cooperative launch of `kernel`: as many kSmoothThreads-blocks as `work`
 // needs, at most as many as the device holds at once.
 int cooperative_grid(const void* kernel, long long work, unsigned* grid) {
     int device = 0, sms = 0, per_sm = 0;
     CSG_CUDA_CHECK(cudaGetDevice(&device));
     CSG_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    CSG_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kThreads, 0));
+    CSG_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kSmoothThreads, 0));
     const long long resident = static_cast<long long>(sms) * (per_sm > 0 ? per_sm : 1);
-    *grid = static_cast<unsigned>(std::max(1LL, std::min(resident, (work + kThreads - 1) / kThreads)));
+    *grid = static_cast<unsigned>(std::max(1LL, std::min(resident, (work + kSmoothThreads - 1) / kSmoothThreads)));
     return CSG_OK;
 }
 
@@ -546,7 +548,7 @@ int csg_feature_smooth_geometry(int n_points, const int32_t* nbr_off, const int3
     void* args[] = {&in, &out, &tmp, const_cast<int32_t**>(&nbr_off), const_cast<int32_t**>(&nbr), &n_points,
                     &iterations, &ctl, &timeout_ns};
     CSG_CUDA_CHECK(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_smooth_geometry_all), dim3(grid),
-                                               dim3(kThreads), args, 0, s));
+                                               dim3(kSmoothThreads), args, 0, s));
     csg::note_launch();
     CSG_CUDA_CHECK(cudaGetLastError());
     return CSG_OK;
@@ -598,7 +600,7 @@ int csg_feature_smooth_values(int n_points, const int32_t* nbr_off, const int32_
         void* args[] = {&in, &out, &tmp, &weights, &wsum, const_cast<int32_t**>(&nbr_off), const_cast<int32_t**>(&nbr),
                         &n_points, &series, &sp, &max_it, &ctl, &timeout_ns};
         CSG_CUDA_CHECK(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_smooth_values_all), dim3(cgrid),
-                                                   dim3(kThreads), args, 0, s));
+                                                   dim3(kSmoothThreads), args, 0, s));
         csg::note_launch();
     }
     if (max_it == 0)
