@@ -11,7 +11,7 @@
 // 3-term dot products are (a0 b0 + a1 b1) + a2 b2.
 //
 // Work decomposition: one work item = (surface, candidate, tile of source points), or
-// up to kMaxGroup consecutive tiles in a launch large enough.  A persistent grid walks the
+// up to kMaxGroup consecutive tiles of a surface that gains by it.  A persistent grid takes the
 // flattened item list, so any mix of surfaces of uneven size and candidate counts is one
 // launch.  Each tile has one float64 partial (block reduction of its points in their order,
 // whichever order they were taken in); a second kernel sums the partials of each (surface,
@@ -46,6 +46,7 @@ struct RotSurface {
     int n_features;              // >= 1; values are feature-major
     int n_tgt_points;            // feature stride of tgt_values
     int tiles;                   // ceil(n_src / tile)
+    int group;                   // tiles of an item
     long long item_begin;        // first flat work item of this surface (ceil(tiles / group) per candidate)
 };
 
@@ -186,12 +187,24 @@ __device__ __forceinline__ float candidate_record(const float* q, const float* r
 // terms (the float32 values candidate() forms), then a bounding sphere: centre and a
 // radius that also covers the closest-polygon test's 1e-3 parametric tolerance.
 constexpr int kRecordFloats = 20;
-// Tiles whose points one CTA of a large launch takes in order of place: threads of a warp then
-// read the same triangles.  8 tiles: 22.7 -> 19.6 ms on 2 x 512 candidates of 61,442 and 102,400
-// points (with float32 reaches 24.6 -> 22.2, 23.5 with 4 tiles, 25.5 with 16).  Below kGroupItems groups there are too few for the device: 46 candidates
-// of 40,962 points are 926 groups, a wave and a half, and no faster than their 7,406 tiles.
+// A launch of kLargeItems tiles or more deals its items from a counter, and of its surfaces of
+// kGroupPoints points or more a CTA takes kMaxGroup tiles at a time, their points in order of
+// place: threads of a warp then read the same triangles.
+//   Dealing: items differ in cost (a candidate's last group has one to eight tiles), and with a
+// fixed stride the CTAs whose stride shares a factor with the groups per candidate always got
+// the long ones (2,048 candidates of 2,562 points in groups 2.78 ms, dealt 1.90).  Below the limit
+// the counter's round trip shows (four candidates of 40,962 points 139 us by stride, 158 dealt).
+//   Grouping: what a warp gains depends on the points per box (a group of n points' surface has
+// about n / 800 in each) and on the order the points come in.  Along a spiral, where neighbours
+// in the list are far apart, groups against single tiles, both dealt, in ms (tile 256, two features):
+// 1,365 candidates of 61,442 points 19.7 and 21.9, 819 of 102,400 18.1 and 21.7, 2,047 of 40,962 21.1
+// and 22.0, 2,048 of 30,000 16.3 and 16.3, of 12,000 7.3 and 6.8, of 2,562 1.90 and 1.64.  In the order
+// of a subdivided icosahedron, whose neighbours are close already, they lose (2,047 of 40,962:
+// 22.1 and 19.8), as in shuffled order (61,442: 25.7 and 24.0).  So the limit lies above the
+// 40,962 points of the resampling sphere.  8 tiles: with 4 102,400 points take 19.2, with 2 21.3.
 constexpr int kMaxGroup = 8;
-constexpr long long kGroupItems = 2400;
+constexpr int kGroupPoints = 42000;
+constexpr long long kLargeItems = 19200;
 constexpr int kMaxCompact = 64;  // candidates per cell whose reaches the cost scan keeps
 static_assert(kMaxCompact <= 64, "the survivors of a cell are one 64-bit mask");
 
@@ -419,22 +432,30 @@ __device__ __forceinline__ void rotated_point(const RotSurface& S, const float* 
     for (int j = 0; j < 3; ++j) q[j] = (px * m[3 * j] + py * m[3 * j + 1]) + pz * m[3 * j + 2];
 }
 
-
 template <int TILE>
 __global__ void __launch_bounds__(TILE, 1024 / TILE) k_rotation_cost(const __grid_constant__ SurfaceTable table,
                                                         const RotSurface* __restrict__ many, int n_surfaces,
-                                                        long long n_items, int group, int* __restrict__ error) {
+                                                        long long n_items, int deal, int* __restrict__ error) {
     __shared__ double red[TILE / 32];
     __shared__ int warp_sums[TILE / 32];
+    __shared__ int dealt;
     extern __shared__ double contrib[];  // [group * TILE]; the boxes' counts before; then order
     const RotSurface* surfaces = n_surfaces <= kInlineSurfaces ? table.s : many;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (long long item = blockIdx.x; item < n_items; item += gridDim.x) {
+    for (long long item = blockIdx.x;; item += gridDim.x) {
+        if (deal) {  // the counter behind the status word
+            if (threadIdx.x == 0) dealt = atomicAdd(error + 1, 1);
+            __syncthreads();
+            item = dealt;
+            __syncthreads();
+        }
+        if (item >= n_items) break;
         // locate the surface of this item (few surfaces: linear scan)
         int s = 0;
         while (s + 1 < n_surfaces && surfaces[s + 1].item_begin <= item) ++s;
         const RotSurface& S = surfaces[s];
         const long long local = item - S.item_begin;
+        const int group = S.group;
         const int groups = (S.tiles + group - 1) / group;
         const int cand = static_cast<int>(local / groups);
         const int tile = static_cast<int>(local - static_cast<long long>(cand) * groups) * group;
@@ -710,15 +731,16 @@ int csg_rotation_cost_batch(int n_surfaces, const csg_rotation_surface* surfaces
     size_t used = align256(sizeof(RotSurface) * n_surfaces);
     long long* d_off = reinterpret_cast<long long*>(base + used);
     used += align256(sizeof(long long) * n_surfaces);
-    int* d_err = reinterpret_cast<int*>(base + used);
+    int* d_err = reinterpret_cast<int*>(base + used);  // status word, item counter
     used += 256;
     std::vector<RotSurface> host(n_surfaces);
     std::vector<long long> cost_off(n_surfaces);
     long long items = 0, coff = 0, tile_items = 0;
     for (int s = 0; s < n_surfaces; ++s)
         tile_items += static_cast<long long>((surfaces[s].n_src + tile - 1) / tile) * surfaces[s].n_candidates;
-    const int group = tile_items >= kMaxGroup * kGroupItems ? kMaxGroup : 1;
-    int max_c = 0;
+    const bool large = tile_items >= kLargeItems;
+    int max_c = 0, group = 1;  // group: the largest of the surfaces'
+
     for (int s = 0; s < n_surfaces; ++s) {
         const csg_rotation_surface& in = surfaces[s];
         RotSurface& r = host[s];
@@ -739,8 +761,10 @@ int csg_rotation_cost_batch(int n_surfaces, const csg_rotation_surface* surfaces
         r.tiles = (in.n_src + tile - 1) / tile;
         r.partials = reinterpret_cast<double*>(base + used);
         used += align256(sizeof(double) * static_cast<size_t>(r.tiles) * r.n_candidates);
+        r.group = large && in.n_src >= kGroupPoints ? kMaxGroup : 1;
+        group = std::max(group, r.group);
         r.item_begin = items;
-        items += static_cast<long long>((r.tiles + group - 1) / group) * r.n_candidates;
+        items += static_cast<long long>((r.tiles + r.group - 1) / r.group) * r.n_candidates;
         cost_off[s] = coff;
         coff += r.n_candidates;
         max_c = std::max(max_c, r.n_candidates);
@@ -756,18 +780,19 @@ int csg_rotation_cost_batch(int n_surfaces, const csg_rotation_surface* surfaces
         CSG_CUDA_CHECK(cudaMemcpyAsync(d_surf, host.data(), sizeof(RotSurface) * n_surfaces, cudaMemcpyHostToDevice, st));
         CSG_CUDA_CHECK(cudaMemcpyAsync(d_off, cost_off.data(), sizeof(long long) * n_surfaces, cudaMemcpyHostToDevice, st));
     }
-    CSG_CUDA_CHECK(cudaMemsetAsync(d_err, 0, sizeof(int), st));
+    CSG_CUDA_CHECK(cudaMemsetAsync(d_err, 0, 2 * sizeof(int), st));
     int device = 0, sms = 0;
     CSG_CUDA_CHECK(cudaGetDevice(&device));
     CSG_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     const long long want = n_ctas > 0 ? n_ctas : static_cast<long long>(sms) * (1024 / tile);  // what is resident
     const unsigned blocks = static_cast<unsigned>(std::min<long long>(std::max<long long>(1, want), items));
+    const int deal = large && items + blocks < (1LL << 31);  // the counter is an int
     // the points' contributions, and their order by place
     const size_t smem = group > 1 ? sort_bytes(group * tile) + sizeof(unsigned short) * group * tile : sizeof(double) * tile;
     switch (tile) {
-        case 128: (csg::note_launch(), k_rotation_cost<128><<<blocks, 128, smem, st>>>(table, d_surf, n_surfaces, items, group, d_err)); break;
-        case 512: (csg::note_launch(), k_rotation_cost<512><<<blocks, 512, smem, st>>>(table, d_surf, n_surfaces, items, group, d_err)); break;
-        default: (csg::note_launch(), k_rotation_cost<256><<<blocks, 256, smem, st>>>(table, d_surf, n_surfaces, items, group, d_err)); break;
+        case 128: (csg::note_launch(), k_rotation_cost<128><<<blocks, 128, smem, st>>>(table, d_surf, n_surfaces, items, deal, d_err)); break;
+        case 512: (csg::note_launch(), k_rotation_cost<512><<<blocks, 512, smem, st>>>(table, d_surf, n_surfaces, items, deal, d_err)); break;
+        default: (csg::note_launch(), k_rotation_cost<256><<<blocks, 256, smem, st>>>(table, d_surf, n_surfaces, items, deal, d_err)); break;
     }
     (csg::note_launch(), k_rotation_finalize<<<dim3(max_c, n_surfaces), csg::kOrderedThreads, 0, st>>>(table, d_surf, n_surfaces, costs, d_off));
     CSG_CUDA_CHECK(cudaGetLastError());

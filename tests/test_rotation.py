@@ -314,3 +314,35 @@ def test_groups_of_tiles_equal_single_candidates(native_library, tile, grid_size
     alone = batched_costs([index], [inputs], matrix_sets=[few], tile=tile)[0]
     together = batched_costs([index], [inputs], matrix_sets=[many], tile=tile)[0]
     assert torch.equal(together, alone.repeat(repeats))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tile", [128, 256, 512])
+@pytest.mark.parametrize("sizes", [(42000,), (41999, 42000), (42001, 300, 46097), (1, 42000, 513, 41999, 44032, 2562)])
+def test_large_launches_equal_single_candidates(native_library, tile, sizes):
+    """Launches whose items are dealt from the counter, with surfaces on either side of the size from which
+    a CTA takes several tiles' points in order of place, alone and mixed (in the launch parameter and, from
+    five surfaces on, in the uploaded table): the costs of launches tile by tile, bit for bit."""
+
+    import torch
+
+    from cat_surface_gpu_b200 import synthetic
+    from cat_surface_gpu_b200.surface_rotation import RotationGridIndex, batched_costs, rotation_matrices_flat
+
+    rng = np.random.default_rng(tile + len(sizes))
+    tp, tf = synthetic.unit_icosphere(4)
+    index = RotationGridIndex.from_geometry(tp, tf, grid_size=32, margin=1,
+                                            include_dense_candidate_table=False).to("cuda")
+    inputs = []
+    for points in sizes:
+        src = rng.normal(size=(points, 3))
+        src = (src / np.linalg.norm(src, axis=1, keepdims=True)).astype(np.float32)
+        inputs.append(index.prepare_cost_inputs(src, np.sin(4 * src[:, 0]).astype(np.float64), np.sin(4 * tp[:, 0])))
+    few = rotation_matrices_flat(rng.uniform(-1, 1, size=(5, 3)))
+    tiles = sum(-(-points // tile) for points in sizes)
+    repeats = -(-19200 // (tiles * few.shape[0]))
+    many = [np.tile(few, (repeats, 1))] * len(sizes)
+    together = batched_costs([index] * len(sizes), inputs, matrix_sets=many, tile=tile)
+    for i, costs in enumerate(together):
+        alone = batched_costs([index], [inputs[i]], matrix_sets=[few], tile=tile)[0]
+        assert torch.equal(costs, alone.repeat(repeats)), sizes[i]
