@@ -1463,9 +1463,12 @@ __global__ void __launch_bounds__(kResidentThreads, CTAS) k_resident_cycles(cons
 //
 // Separate launches are bound by reading 56 bytes per point for each half-sweep from L2: on two
 // 512 x 256 float64 grids 6.7 us each, 104 us a V-cycle for the level, where both legs take 52
-// although they update each point 2.5 times.  A V-cycle of the whole hierarchy: 178 -> 127 us
-// (eight grids 419 -> 335, two in float32 146 -> 109, one of 1024 x 512 290 -> 195); no batch
-// was found at which the separate launches are faster.
+// although they update each point 2.5 times.  A V-cycle of the whole hierarchy with three
+// iterations: 171 -> 123 us (eight grids 353 -> 326, two in float32 154 -> 106, one of
+// 1024 x 512 271 -> 190).  The halo grows with the iterations and a tile shrinks: a point is updated
+// 2.8 times at four of them, 4 at five, 7 at six, 28 at eight (one 512 x 256 grid at eight: 403 us
+// against 275, eight of them at five: 566 against 493), so the cheaper form is estimated
+// for each launch (see LegCosts).
 
 constexpr int kLegUnits = kResidentSlots * kResidentThreads;  // of a region, one row of tap weights each at most 128
 constexpr int kLegWidth = 48;                                 // columns of a region (nx when fewer); 40-64 within 2%, 80 10% slower
@@ -1627,6 +1630,21 @@ __global__ void __launch_bounds__(kResidentThreads, sizeof(T) == 4 ? 2 : 1)
 }
 
 constexpr size_t kLegSmemMax = 200 * 1024;
+
+// What one V-cycle spends on a level above the resident ones, in microseconds: as two legs, a
+// wave of CTAs (148 at once, 296 in float32) takes leg + leg_nit x iterations; as separate
+// launches, each of the 4 x iterations + 4 takes launch + point per 100,000 points.  Fitted to
+// V-cycles of 16 x 4096 to 2048 x 1024 points, batches of 1 to 128 and 1 to 8 iterations in both forms
+// (an estimated V-cycle is 8% off on average, 35% at most); where it picks the slower form, the two
+// differ by less than 5%.
+template <typename T>
+struct LegCosts {
+    static constexpr bool f64 = sizeof(T) == 8;
+    static constexpr double leg = f64 ? 7.6 : 6.8, leg_nit = f64 ? 0.95 : 1.18;
+    static constexpr double launch = f64 ? 3.3 : 3.4, point = f64 ? 1.0 : 0.74;
+    static constexpr double resident = f64 ? 148 : 296;
+};
+
 constexpr size_t kResidentSmemMax = 226 * 1024;
 // The restriction chain of a level-l field to every coarser level at or below
 // kChainPoints points per grid, in one launch with one CTA per batch element:
@@ -2000,9 +2018,8 @@ struct Fmg {
         (csg::note_launch(), csg::launch_pdl_cluster(kernel, dim3(static_cast<unsigned>(plan.size), static_cast<unsigned>(batch)),
                                                      static_cast<unsigned>(plan.size), kResidentThreads, plan.smem, s, plan.c));
     }
-    // Level l runs as one launch down and one up when its x size is even and, where a region is not
-    // the whole height of the grid, the halos leave some of its rows (nit <= 6).  `aligned`: the level's
-    // fields start at multiples of a pair.
+    // The leg of level l, where it can run as one: an even x size, and halos that leave some of a
+    // region's columns and rows (of 48 x 42 up to nit = 9).
     bool leg(size_t l, bool down, const T* uin, T* uout, FineLeg<T>& g) const {
         const int nx = buf.specs[l].first, ny = buf.specs[l].second;
         if (nx % 2 != 0 || nit < 1 || nit > 64) return false;
@@ -2036,17 +2053,28 @@ struct Fmg {
                   (2 * sizeof(T))) == 0;
         return true;
     }
+    static int leg_tiles(const FineLeg<T>& g) { return g.tiles_x * ((g.ny + g.th - 1) / g.th); }
+    // Whether level l runs as legs, by the estimate of LegCosts.
+    bool as_legs(size_t l) const {
+        using C = LegCosts<T>;
+        FineLeg<T> down, up;
+        if (!leg(l, true, buf.U[l], buf.R[l], down) || !leg(l, false, buf.R[l], buf.U[l], up)) return false;
+        const double points = static_cast<double>(buf.specs[l].first) * buf.specs[l].second * batch;
+        const double waves = std::max(1.0, leg_tiles(down) * static_cast<double>(batch) / C::resident) +
+                             std::max(1.0, leg_tiles(up) * static_cast<double>(batch) / C::resident);
+        return waves * (C::leg + C::leg_nit * nit) <= (4.0 * nit + 4.0) * (C::launch + C::point * 1e-5 * points);
+    }
     template <bool DOWN>
     void launch_leg(const FineLeg<T>& g) {
         allow_big_smem<T>();
         const int rows = std::min(g.ny, g.th == g.ny ? g.ny : g.th + 2 * g.halo);
         const size_t smem = static_cast<size_t>(rows) * g.width * sizeof(Pair<T>) * (DOWN ? 2 : 1) +
                             (rows + 8) * sizeof(AxisTaps<T>);
-        const dim3 grid(static_cast<unsigned>(g.tiles_x * ((g.ny + g.th - 1) / g.th)), static_cast<unsigned>(batch));
+        const dim3 grid(static_cast<unsigned>(leg_tiles(g)), static_cast<unsigned>(batch));
         (csg::note_launch(), csg::launch_pdl(k_vcycle_leg<T, DOWN>, grid, kResidentThreads, smem, s, g));
     }
     // `count` V-cycles from level `start` on: resident from the first level that fits a cluster,
-    // the levels above it leg by leg in every cycle.
+    // the levels above it as legs or separate launches in every cycle.
     void run_cycles(size_t start, int count) {
         if (count < 1) return;
         const size_t last = buf.specs.size() - 1;
@@ -2059,12 +2087,14 @@ struct Fmg {
         }
         if (plan.size == 0) fit = last;
         FineLeg<T> g;
+        std::vector<char> legs(fit);
+        for (size_t l = start; l < fit; ++l) legs[l] = as_legs(l);
         for (int c = 0; c < count; ++c) {
             // down: relax, residual, restriction (a fused leg leaves the relaxed solution in R[l]);
             // up: prolongation, relax (a fused leg reads R[l] and writes U[l])
             for (size_t l = start; l < fit; ++l) {
                 const int nx = buf.specs[l].first, ny = buf.specs[l].second;
-                if (leg(l, false, buf.R[l], buf.U[l], g) && leg(l, true, buf.U[l], buf.R[l], g)) {
+                if (legs[l] && leg(l, true, buf.U[l], buf.R[l], g)) {
                     launch_leg<true>(g);
                     continue;
                 }
@@ -2080,7 +2110,7 @@ struct Fmg {
             if (plan.size > 0) launch_resident(plan);
             else relax(last);
             for (size_t l = fit; l-- > start;) {
-                if (leg(l, true, buf.U[l], buf.R[l], g) && leg(l, false, buf.R[l], buf.U[l], g)) {
+                if (legs[l] && leg(l, false, buf.R[l], buf.U[l], g)) {
                     launch_leg<false>(g);
                     continue;
                 }

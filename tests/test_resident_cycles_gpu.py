@@ -117,3 +117,38 @@ def test_resident_cycles_equal_the_separate_kernels(native_library, dtype, nx, n
     torch.cuda.synchronize()
     assert torch.isfinite(u).all()
     assert torch.equal(u, _separate(lib, code, hess, rhs, start, cycles, nit))
+
+
+@pytest.mark.parametrize(
+    "dtype, nx, ny, batch, nit, legs",
+    [
+        (torch.float64, 512, 256, 1, 3, True),
+        (torch.float64, 512, 256, 8, 3, True),
+        (torch.float64, 512, 256, 8, 5, False),  # many tiles, a point updated four times
+        (torch.float32, 512, 256, 8, 5, True),
+        (torch.float64, 512, 256, 1, 6, True),
+        (torch.float64, 512, 256, 1, 8, False),  # tiles of 12 x 6
+        (torch.float32, 512, 256, 1, 9, False),
+        (torch.float64, 512, 100, 1, 9, False),
+        (torch.float64, 512, 100, 1, 10, False),  # halos that leave nothing
+        (torch.float64, 16, 4096, 1, 9, True),  # whole rows
+    ],
+)
+def test_fine_levels_take_the_cheaper_form(native_library, dtype, nx, ny, batch, nit, legs):
+    """The first level, above the resident ones, as two launches or as separate ones, with equal results."""
+
+    lib = native_library
+    code = 1 if dtype == torch.float64 else 0
+    hess, rhs, start = _problem(nx, ny, batch, dtype, "plain")
+    scratch = torch.empty(lib.csg_dartel_scratch_bytes(code, batch, nx, ny), dtype=torch.uint8, device="cuda")
+    launches = []
+    for cycles in (0, 1):
+        u = start.clone()
+        before = lib.csg_kernel_launches()
+        assert lib.csg_dartel_fmg(code, batch, nx, ny, hess.data_ptr(), rhs.data_ptr(), _params((nx, ny), (nx, ny)), cycles, nit,
+                                  u.data_ptr(), 1, 1, scratch.data_ptr(), scratch.numel(), 0) == 0
+        launches.append(lib.csg_kernel_launches() - before)
+    torch.cuda.synchronize()
+    # two legs, or the half-sweeps of both ways, residual, restriction and prolongation; and the resident cycle
+    assert launches[1] - launches[0] == (2 if legs else 4 * nit + 3) + 1
+    assert torch.equal(u, _separate(lib, code, hess, rhs, start, 1, nit))
