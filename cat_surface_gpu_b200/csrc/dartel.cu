@@ -1631,6 +1631,28 @@ __global__ void __launch_bounds__(kResidentThreads, sizeof(T) == 4 ? 2 : 1)
 
 constexpr size_t kLegSmemMax = 200 * 1024;
 
+// What a wave of clusters spends on a resident V-cycle, in microseconds, summed over its levels: on a split
+// level split + split_nit x iterations, (unit + unit_nit x iterations) for each unit of a thread, far where its
+// transfers read other CTAs' rows; on a level of CTA 0 local + local_nit x iterations.  Fitted to V-cycles
+// of 32 x 17 to 256 x 128 points, batches of 2 to 4,096 and 1 to 5 iterations (5% off at most in float64, 8% with
+// two CTAs to an SM, 23% with one in float32).  Clusters of 16 CTAs run 7 at a time, so a batch of 32 grids of
+// 256 x 128 in float32 took three waves of 82 us, where legs on the first level and clusters of
+// 4 CTAs below take 156 (64 in float64 551 and 483 us, 128 of 256 x 113 with one iteration 757 and
+// 490, and 587 before there were resident cycles).  In one wave, and with one CTA per grid, the resident form is
+// the faster one throughout.
+struct ResidentCosts {
+    double split, split_nit, unit, unit_nit, far, local, local_nit;
+};
+template <typename T>
+constexpr ResidentCosts resident_costs(bool paired) {
+    if (sizeof(T) == 8) return {2.1, 0.69, 2.0, 0.85, 1.0, 1.0, 0.58};
+    if (paired) return {3.9, -1.86, 1.1, 2.9, 1.3, 0.84, 1.14};
+    return {1.8, 0.79, 0.71, 1.2, 0.43, 0.70, 0.83};
+}
+// A resident launch in every cycle, below legs, against one for all cycles: each loads its fields again.
+// The estimates are up to 20% off where neither form is far ahead, so only a clear gain counts.
+constexpr double kRelaunch = 9.5, kClearly = 0.85;
+
 // What one V-cycle spends on a level above the resident ones, in microseconds: as two legs, a
 // wave of CTAs (148 at once, 296 in float32) takes leg + leg_nit x iterations; as separate
 // launches, each of the 4 x iterations + 4 takes launch + point per 100,000 points.  Fitted to
@@ -1646,6 +1668,7 @@ struct LegCosts {
 };
 
 constexpr size_t kResidentSmemMax = 226 * 1024;
+constexpr size_t kPairedSmemMax = 113 * 1024;  // of each of two CTAs to an SM
 // The restriction chain of a level-l field to every coarser level at or below
 // kChainPoints points per grid, in one launch with one CTA per batch element:
 // the same resize_at per point as separate k_resize launches, level after
@@ -1734,36 +1757,43 @@ void allow_big_smem() {
     done.fetch_or(bit);
 }
 
-// Largest cluster (16, 8, 4, 2 or 1 CTAs) of the resident kernel this device can hold with
-// kResidentSmemMax of shared memory per CTA, found once per device.
+// Clusters of 1, 2, 4, 8 and 16 CTAs of a resident kernel that this device runs at once: with kResidentSmemMax of
+// shared memory per CTA (one CTA to an SM), and of the kernel of two CTAs to an SM with half of that.  0: a size
+// that the device refuses.  Found once per device.
+struct ClusterCounts {
+    int one[5], two[5];
+};
 template <typename T>
-int largest_cluster() {
-    static std::atomic<int> known[64];
+ClusterCounts cluster_counts() {
+    static std::atomic<int> known[64][10];
+    ClusterCounts counts{};
     int device = 0;
-    if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return 1;
-    int size = known[device].load();
-    if (size > 0) return size;
+    if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return counts;
     allow_big_smem<T>();
-    for (size = kMaxCluster; size > 1; size >>= 1) {
-        cudaLaunchAttribute attr{};
-        attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = static_cast<unsigned>(size);
-        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-        cudaLaunchConfig_t config{};
-        config.gridDim = dim3(static_cast<unsigned>(size), 1, 1);
-        config.blockDim = dim3(kResidentThreads, 1, 1);
-        config.dynamicSmemBytes = kResidentSmemMax;
-        config.attrs = &attr;
-        config.numAttrs = 1;
-        int clusters = 0;
-        if (cudaOccupancyMaxActiveClusters(&clusters, reinterpret_cast<const void*>(k_resident_cycles<T, 1>), &config) ==
-                cudaSuccess &&
-            clusters > 0)
-            break;
-        cudaGetLastError();  // a size the device refuses is not the caller's error
+    for (int k = 9; k >= 0; --k) {
+        int found = known[device][k].load() - 1;
+        if (found < 0) {
+            cudaLaunchAttribute attr{};
+            attr.id = cudaLaunchAttributeClusterDimension;
+            attr.val.clusterDim.x = 1u << k % 5;
+            attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+            cudaLaunchConfig_t config{};
+            config.gridDim = dim3(1u << k % 5, 1, 1);
+            config.blockDim = dim3(kResidentThreads, 1, 1);
+            config.dynamicSmemBytes = k < 5 ? kResidentSmemMax : kPairedSmemMax;
+            config.attrs = &attr;
+            config.numAttrs = 1;
+            const void* kernel = k < 5 ? reinterpret_cast<const void*>(k_resident_cycles<T, 1>)
+                                       : reinterpret_cast<const void*>(k_resident_cycles<T, sizeof(T) == 4 ? 2 : 1>);
+            if (cudaOccupancyMaxActiveClusters(&found, kernel, &config) != cudaSuccess) {
+                cudaGetLastError();  // a size the device refuses is not the caller's error
+                found = 0;
+            }
+            known[device][k].store(found + 1);
+        }
+        (k < 5 ? counts.one[k] : counts.two[k - 5]) = found;
     }
-    known[device].store(size);
-    return size;
+    return counts;
 }
 
 template <typename T>
@@ -1935,17 +1965,23 @@ struct Fmg {
         ResidentCycle<T> c{};
         int size = 0;
         size_t smem = 0;
+        bool paired = false;  // two CTAs to an SM
+        int waves = 1;
+        double us = 0;        // estimated time of a V-cycle
     };
     Resident resident(size_t first, int count) const {
         Resident none, plan;
         const size_t L = buf.specs.size();
         if (L > static_cast<size_t>(kMaxLevels) || nit < 1) return none;
+        const ClusterCounts counts = cluster_counts<T>();
         auto points = [&](size_t l) { return static_cast<long long>(buf.specs[l].first) * buf.specs[l].second; };
         size_t local = first;
         while (points(local) > kCoarsePoints) ++local;  // the last level is one point
         int size = 1;
         if (local > first) {
-            const int most = largest_cluster<T>();
+            int most = 1;
+            for (int k = 1; k < 5; ++k)
+                if (counts.one[k] > 0) most = 1 << k;
             while (size < most && points(first) > static_cast<long long>(size) * kCoarsePoints) size *= 2;
             for (size_t l = first; l < local; ++l) {
                 if (buf.specs[l].first < 2) return none;
@@ -2009,12 +2045,21 @@ struct Fmg {
         if (at > kResidentSmemMax) return none;
         plan.smem = static_cast<size_t>(at);
         plan.size = size;
+        plan.paired = sizeof(T) == 4 && static_cast<long long>(size) * batch > kPairedCtas;
+        const int at_once = std::max(1, (plan.paired && plan.smem <= kPairedSmemMax ? counts.two : counts.one)[c.lgsize]);
+        plan.waves = (batch + at_once - 1) / at_once;
+        const ResidentCosts k = resident_costs<T>(plan.paired);
+        for (int l = c.first; l < c.local; ++l) {
+            const int units = (c.lv[l].own / 2 + kResidentThreads - 1) / kResidentThreads;  // of a thread
+            plan.us += k.split + k.split_nit * nit + (k.unit + k.unit_nit * nit) * units + (c.lv[l].near ? 0.0 : k.far);
+        }
+        plan.us = plan.waves * (plan.us + (c.last - c.local + 1) * (k.local + k.local_nit * nit));
         return plan;
     }
     void launch_resident(const Resident& plan) {
         allow_big_smem<T>();
         auto kernel = k_resident_cycles<T, 1>;
-        if (sizeof(T) == 4 && plan.size * batch > kPairedCtas) kernel = k_resident_cycles<T, sizeof(T) == 4 ? 2 : 1>;
+        if (plan.paired) kernel = k_resident_cycles<T, sizeof(T) == 4 ? 2 : 1>;
         (csg::note_launch(), csg::launch_pdl_cluster(kernel, dim3(static_cast<unsigned>(plan.size), static_cast<unsigned>(batch)),
                                                      static_cast<unsigned>(plan.size), kResidentThreads, plan.smem, s, plan.c));
     }
@@ -2054,15 +2099,19 @@ struct Fmg {
         return true;
     }
     static int leg_tiles(const FineLeg<T>& g) { return g.tiles_x * ((g.ny + g.th - 1) / g.th); }
-    // Whether level l runs as legs, by the estimate of LegCosts.
-    bool as_legs(size_t l) const {
+    // Whether level l runs as legs, by the estimate of LegCosts, and its time.
+    bool as_legs(size_t l, double& us) const {
         using C = LegCosts<T>;
+        const double points = static_cast<double>(buf.specs[l].first) * buf.specs[l].second * batch;
+        us = (4.0 * nit + 4.0) * (C::launch + C::point * 1e-5 * points);
         FineLeg<T> down, up;
         if (!leg(l, true, buf.U[l], buf.R[l], down) || !leg(l, false, buf.R[l], buf.U[l], up)) return false;
-        const double points = static_cast<double>(buf.specs[l].first) * buf.specs[l].second * batch;
         const double waves = std::max(1.0, leg_tiles(down) * static_cast<double>(batch) / C::resident) +
                              std::max(1.0, leg_tiles(up) * static_cast<double>(batch) / C::resident);
-        return waves * (C::leg + C::leg_nit * nit) <= (4.0 * nit + 4.0) * (C::launch + C::point * 1e-5 * points);
+        const double legs = waves * (C::leg + C::leg_nit * nit);
+        if (legs > us) return false;
+        us = legs;
+        return true;
     }
     template <bool DOWN>
     void launch_leg(const FineLeg<T>& g) {
@@ -2073,28 +2122,42 @@ struct Fmg {
         const dim3 grid(static_cast<unsigned>(leg_tiles(g)), static_cast<unsigned>(batch));
         (csg::note_launch(), csg::launch_pdl(k_vcycle_leg<T, DOWN>, grid, kResidentThreads, smem, s, g));
     }
-    // `count` V-cycles from level `start` on: resident from the first level that fits a cluster,
-    // the levels above it as legs or separate launches in every cycle.
+    // `count` V-cycles from level `start` on: the levels above the resident ones as legs or separate
+    // launches in every cycle.  Resident from the first level that fits a cluster, unless the batch takes
+    // several waves of clusters and a later level is estimated to be faster (see ResidentCosts).
     void run_cycles(size_t start, int count) {
         if (count < 1) return;
         const size_t last = buf.specs.size() - 1;
-        size_t fit = start;
-        Resident plan = resident(start, count);
-        while (plan.size == 0 && fit < last) plan = resident(++fit, 1);
+        size_t fit = last;
+        Resident plan;
+        std::vector<char> legs;  // whether level start + i runs as legs
+        double above = 0;        // estimated time of the levels before l
+        for (size_t l = start; plan.size == 0 || above < plan.us; ++l) {
+            Resident r = resident(l, l == start ? count : 1);
+            if (r.size > 0) {
+                if (l > start) r.us += above + kRelaunch;
+                if (plan.size == 0 || r.us < kClearly * plan.us) {
+                    plan = r;
+                    fit = l;
+                }
+                if (r.waves == 1 || r.size == 1) break;
+            }
+            if (l == last) break;
+            double us = 0;
+            legs.push_back(as_legs(l, us));
+            above += us;
+        }
         if (plan.size > 0 && fit == start) {
             launch_resident(plan);
             return;
         }
-        if (plan.size == 0) fit = last;
         FineLeg<T> g;
-        std::vector<char> legs(fit);
-        for (size_t l = start; l < fit; ++l) legs[l] = as_legs(l);
         for (int c = 0; c < count; ++c) {
             // down: relax, residual, restriction (a fused leg leaves the relaxed solution in R[l]);
             // up: prolongation, relax (a fused leg reads R[l] and writes U[l])
             for (size_t l = start; l < fit; ++l) {
                 const int nx = buf.specs[l].first, ny = buf.specs[l].second;
-                if (legs[l] && leg(l, true, buf.U[l], buf.R[l], g)) {
+                if (legs[l - start] && leg(l, true, buf.U[l], buf.R[l], g)) {
                     launch_leg<true>(g);
                     continue;
                 }
@@ -2110,7 +2173,7 @@ struct Fmg {
             if (plan.size > 0) launch_resident(plan);
             else relax(last);
             for (size_t l = fit; l-- > start;) {
-                if (legs[l] && leg(l, false, buf.R[l], buf.U[l], g)) {
+                if (legs[l - start] && leg(l, false, buf.R[l], buf.U[l], g)) {
                     launch_leg<false>(g);
                     continue;
                 }

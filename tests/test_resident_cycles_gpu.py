@@ -123,7 +123,7 @@ def test_resident_cycles_equal_the_separate_kernels(native_library, dtype, nx, n
     "dtype, nx, ny, batch, nit, legs",
     [
         (torch.float64, 512, 256, 1, 3, True),
-        (torch.float64, 512, 256, 8, 3, True),
+        (torch.float64, 512, 256, 4, 3, True),
         (torch.float64, 512, 256, 8, 5, False),  # many tiles, a point updated four times
         (torch.float32, 512, 256, 8, 5, True),
         (torch.float64, 512, 256, 1, 6, True),
@@ -152,3 +152,41 @@ def test_fine_levels_take_the_cheaper_form(native_library, dtype, nx, ny, batch,
     # two legs, or the half-sweeps of both ways, residual, restriction and prolongation; and the resident cycle
     assert launches[1] - launches[0] == (2 if legs else 4 * nit + 3) + 1
     assert torch.equal(u, _separate(lib, code, hess, rhs, start, 1, nit))
+
+
+@pytest.mark.parametrize(
+    "dtype, nx, ny, batch, nit, resident",
+    [
+        (torch.float64, 256, 128, 7, 3, True),  # one wave of clusters of 16
+        (torch.float64, 256, 128, 8, 3, True),
+        (torch.float64, 256, 128, 64, 3, False),
+        (torch.float64, 256, 113, 32, 1, False),
+        (torch.float32, 256, 128, 14, 3, True),
+        (torch.float32, 256, 128, 32, 3, False),
+        (torch.float32, 64, 33, 32, 2, True),
+        (torch.float32, 64, 33, 600, 2, False),
+        (torch.float64, 32, 17, 74, 1, True),
+        (torch.float64, 32, 17, 600, 1, False),
+        (torch.float64, 32, 16, 600, 3, True),  # one CTA per grid
+        (torch.float64, 8, 4, 4096, 1, True),
+        (torch.float64, 512, 256, 16, 2, False),
+    ],
+)
+def test_batches_of_several_waves(native_library, dtype, nx, ny, batch, nit, resident):
+    """V-cycles of batches on either side of where resident clusters take too many waves: one launch, or
+    finer levels above the resident ones, with the separate kernels' results."""
+
+    lib = native_library
+    code = 1 if dtype == torch.float64 else 0
+    hess, rhs, start = _problem(nx, ny, batch, dtype, "plain")
+    scratch = torch.empty(lib.csg_dartel_scratch_bytes(code, batch, nx, ny), dtype=torch.uint8, device="cuda")
+    launches = []
+    for cycles in (0, 2):
+        u = start.clone()
+        before = lib.csg_kernel_launches()
+        assert lib.csg_dartel_fmg(code, batch, nx, ny, hess.data_ptr(), rhs.data_ptr(), _params((nx, ny), (nx, ny)), cycles, nit,
+                                  u.data_ptr(), 1, 1, scratch.data_ptr(), scratch.numel(), 0) == 0
+        launches.append(lib.csg_kernel_launches() - before)
+    torch.cuda.synchronize()
+    assert (launches[1] - launches[0] == 1) == resident
+    assert torch.equal(u, _separate(lib, code, hess, rhs, start, 2, nit))
