@@ -76,6 +76,7 @@ SIGNATURES: dict[str, tuple[object, list[object]]] = {
     "csg_dartel_relax": (_I, [_I, _I, _I, _I, _P, _P, _P, _I, _P, _P]),
     "csg_dartel_resize": (_I, [_I, _I, _I, _I, _P, _I, _I, _P, _I, _P]),
     "csg_dartel_fmg": (_I, [_I, _I, _I, _I, _P, _P, _P, _I, _I, _P, _I, _I, _P, c_size_t, _P]),
+    "csg_selftest_exchange_timeout": (_I, [_I, _I, _I, _I, _P, _P, _P, _I, _I, _P, _P, c_size_t, c_double, _I, _P]),
     "csg_dartel_expdef": (_I, [_I, _I, _I, _I, _P, _I, _P, _P, _P, c_size_t, _P]),
     "csg_dartel_sample": (_I, [_I, _I, _I, _P, _I, _P, _P, _P, _P]),
     "csg_dartel_data_scratch_bytes": (c_size_t, [_I, _I, _I, _I, _I, _I]),

@@ -19,6 +19,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <cstddef>
 #include <cstdint>
 #include <cstring>
 #include <type_traits>
@@ -777,6 +778,9 @@ struct ResidentCycle {
     int first, local, last;  // levels first .. local - 1 are split over the cluster, local .. last run on CTA 0
     int nit, cycles;
     int lgsize;              // log2 of the cluster's CTAs
+    int silent;              // a CTA that sends no edge rows (-1: none; the self-test of the waits)
+    unsigned long long timeout_ns;  // of an exchange's wait
+    csg::Control* ctl;       // status word
 };
 
 // The start of a CTA's shared memory; the levels' fields and the row taps follow.  What
@@ -1057,27 +1061,41 @@ __device__ __forceinline__ void get(unsigned from, Pair<float>& v) {
 // The edge-row exchange of the half-sweeps.  Half-sweep e sends each updated edge point to
 // the neighbour's halo, counted on the neighbour's barrier e & 1, which completes when
 // both neighbours' bytes have come and this CTA has announced them.  Half-sweep e waits for
-// half-sweep e - 1; a neighbour can run at most one half-sweep ahead (its e + 1 needs this
-// CTA's e), so two barriers do, and what it then writes is of the colour that no edge point
-// reads in half-sweep e.  An exchange of 16 CTAs in a chain takes 434 cycles from wait to wait.
-// (A cluster barrier with its release and acquire takes 570, 770-980 with remote stores before
+// half-sweep e - 1.  Two barriers do, and a halo point is never overwritten before it is read: an
+// edge unit reads its halo before it sends, and a neighbour starts its half-sweep e + 1, whose
+// points of the halo this CTA's half-sweep e reads, only when all of this CTA's edge points
+// of half-sweep e have been counted there.  An exchange of 16 CTAs in a chain takes 434 cycles from wait
+// to wait.  (A cluster barrier with its release and acquire takes 570, 770-980 with remote stores before
 // it; remote stores with one remote arrival per warp 1,120; bulk copies of the rows 470-480.)
-// Every wait is bounded; one that runs out sets `lost`: the CTA waits no more and its results
-// are replaced by NaN.
-__device__ __forceinline__ void await_exchange(unsigned at, unsigned parity, int* lost) {
-    for (int tries = 0;; ++tries) {
-        unsigned done;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(done)
-            : "r"(at), "r"(parity)
-            : "memory");
-        if (done) return;
-        if (tries > (1 << 16) || *reinterpret_cast<volatile int*>(lost)) {
-            *reinterpret_cast<volatile int*>(lost) = 1;
-            return;
-        }
+//
+// Every wait is bounded.  A thread whose wait runs out (or that sees another's run out) counts as
+// lost from then on: it announces and sends nothing more, so no barrier's phase is announced twice and no
+// neighbour's completes with rows that were not updated, but it goes on through every barrier of its CTA
+// and cluster.  The first to give up tells all CTAs of the cluster; the whole grid's result becomes NaN and
+// the status word CSG_ERR_TIMEOUT.
+__device__ __forceinline__ bool exchanged(unsigned at, unsigned parity) {
+    unsigned done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, 1000;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(at), "r"(parity)
+        : "memory");
+    return done != 0;
+}
+__device__ __noinline__ bool await_exchange_slowly(unsigned at, unsigned parity, int* lost, int lgsize,
+                                                   unsigned long long timeout_ns) {
+    const unsigned long long start = csg::global_timer_ns();
+    while (true) {
+        if (*reinterpret_cast<volatile int*>(lost)) return false;
+        if (exchanged(at, parity)) return true;
+        if (csg::global_timer_ns() - start <= timeout_ns) continue;
+        const unsigned mine = static_cast<unsigned>(__cvta_generic_to_shared(lost));
+        for (int r = 0; r < 1 << lgsize; ++r)
+            asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %0, %1;\n\tst.shared::cluster.u32 [a], 1;\n\t}" ::"r"(mine),
+                         "r"(r)
+                         : "memory");
+        return false;
     }
 }
 
@@ -1138,9 +1156,9 @@ __device__ __forceinline__ int unit_row(int k, int n) { return k == 0 ? 0 : (k =
 // relaxation; down: relaxation, the residual and its restriction to level l + 1, whose
 // solution is zeroed.  Both: the end of one cycle and the start of the next on the first
 // level, whose systems stay in registers in between.  A thread holds up to kResidentSlots
-// units; e: iterations exchanged before.
+// units; e: iterations exchanged before; kept: none of the thread's waits has run out.
 template <typename T>
-__device__ __forceinline__ void split_visit(const ResidentCycle<T>& c, int l, int e, bool up, bool down) {
+__device__ __forceinline__ void split_visit(const ResidentCycle<T>& c, int l, int e, bool up, bool down, bool& kept) {
     constexpr int kPair = sizeof(Pair<T>);
     ResidentHead& S = resident_head();
     const ResidentLevel<T>& L = c.lv[l];
@@ -1164,8 +1182,8 @@ __device__ __forceinline__ void split_visit(const ResidentCycle<T>& c, int l, in
         k = min(k, count - 1);  // (a thread without a unit computes the last one's again)
         const int row = unit_row(k >> (lg - 1), V.n), j = k & (h - 1);
         m[s] = make_unit<T>(u + ((row + 1) << lg) * kPair, V.lo + row, j, nx, V.lo + row == 0, V.lo + row == V.ny - 1);
-        top[s] = in[s] && row == 0 && V.above();
-        bottom[s] = in[s] && row == V.n - 1 && V.below();
+        top[s] = in[s] && row == 0 && V.above() && rank != c.silent;
+        bottom[s] = in[s] && row == V.n - 1 && V.below() && rank != c.silent;
         if (l == c.first) {
             const int P = nx * V.ny, at = ((V.lo + row) << lg) + 2 * j;
             const T* A = L.A + 3 * static_cast<size_t>(blockIdx.y) * P;
@@ -1229,14 +1247,17 @@ __device__ __forceinline__ void split_visit(const ResidentCycle<T>& c, int l, in
         if (V.below()) below_barrier = cluster_address(0, rank + 1);
         const Weights<T> w = L.w;
         const int end = e + c.nit * ((up ? 1 : 0) + (down ? 1 : 0));
+        auto await_exchange = [&](unsigned at, int parity) {
+            if (!exchanged(at, parity)) kept &= await_exchange_slowly(at, parity, &S.lost, c.lgsize, c.timeout_ns);
+        };
         auto half_sweep = [&](auto colour_) {
             constexpr int colour = decltype(colour_)::value, mine = colour ? 0 : 8, theirs = 8 - mine;
             asm volatile(
                 "{\n\t.reg .pred p;\n\tsetp.eq.u32 p, %0, 0;\n\t"
-                "@p mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 _, [%1], %2;\n\t}" ::"r"(thread),
+                "@p mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 _, [%1], %2;\n\t}" ::"r"(kept ? thread : 1),
                 "r"(barrier + mine), "r"(bytes)
                 : "memory");
-            await_exchange(barrier + theirs, (colour ? e - 1 : e) & 1, &S.lost);
+            await_exchange(barrier + theirs, (colour ? e - 1 : e) & 1);
 #pragma unroll
             for (int s = 0; s < kResidentSlots; ++s) {
                 if (s >= slots) break;
@@ -1246,8 +1267,8 @@ __device__ __forceinline__ void split_visit(const ResidentCycle<T>& c, int l, in
                 const Pair<T> v = relaxed<colour>(m[s], p[colour][s], w);
                 if (in[s]) pair_at<T>(q) = v;
                 if (s * kResidentThreads < nx) {  // the units of the first and the last row
-                    send(top[s], above + q, above_barrier + mine, v);
-                    send(bottom[s], below + q, below_barrier + mine, v);
+                    send(top[s] && kept, above + q, above_barrier + mine, v);
+                    send(bottom[s] && kept, below + q, below_barrier + mine, v);
                 }
             }
             asm volatile("bar.sync 3, %0;" ::"r"(active) : "memory");
@@ -1257,7 +1278,7 @@ __device__ __forceinline__ void split_visit(const ResidentCycle<T>& c, int l, in
             half_sweep(std::integral_constant<int, 1>{});
             half_sweep(std::integral_constant<int, 0>{});
         }
-        await_exchange(barrier + 8, (e - 1) & 1, &S.lost);
+        await_exchange(barrier + 8, (e - 1) & 1);
         if (down) {
             const Weights<T> g = L.g;
             const int r = L.r - u;
@@ -1408,7 +1429,7 @@ __global__ void __launch_bounds__(kResidentThreads, CTAS) k_resident_cycles(cons
     // and the start of the next are one visit.  (One call of each visit, as they are inlined:
     // behind a call every half-sweep takes 160 cycles more.)
     int e = 0, l = c.first, cycle = 0;  // e: iterations exchanged
-    bool up = false;
+    bool up = false, kept = true;
 #pragma unroll 1
     while (true) {
         if (l == c.local) {
@@ -1423,7 +1444,7 @@ __global__ void __launch_bounds__(kResidentThreads, CTAS) k_resident_cycles(cons
         }
         if (l == c.first && up) ++cycle;
         const bool down = !up || (l == c.first && cycle < c.cycles);
-        split_visit<T>(c, l, e, up, down);
+        split_visit<T>(c, l, e, up, down, kept);
         e += c.nit * ((up ? 1 : 0) + (down ? 1 : 0));
         if (l == c.first && cycle == c.cycles) break;
         if (down) {
@@ -1436,7 +1457,8 @@ __global__ void __launch_bounds__(kResidentThreads, CTAS) k_resident_cycles(cons
     const ResidentLevel<T>& F = c.lv[c.first];
     const int P = F.nx * F.ny, halo = split ? 1 : 0;
     T* U = F.U + 2 * bi * P;
-    // every exchange has been waited for and the cluster has met: no CTA touches another's memory past here
+    // The cluster has met after its last exchange: no CTA stores to another's memory past here, and all agree on
+    // whether a wait ran out.  If none did, every exchange has been waited for.
     const bool lost = *reinterpret_cast<volatile int*>(&S.lost) != 0;
     const Slab V(F.lg, F.nx, F.ny, rank, c.lgsize);
     for (int i = threadIdx.x; i < V.n << F.lg; i += kResidentThreads) {
@@ -1445,6 +1467,14 @@ __global__ void __launch_bounds__(kResidentThreads, CTAS) k_resident_cycles(cons
             pair_at<T>(F.u + (((row + halo) << F.lg) + image_column(V.lo + row, i & (F.nx - 1), F.nx)) * kPair);
         U[(V.lo << F.lg) + i] = lost ? T(NAN) : v.x;
         U[P + (V.lo << F.lg) + i] = lost ? T(NAN) : v.y;
+    }
+    if (lost) {
+        if (rank == 0 && threadIdx.x == 0 && atomicCAS(&c.ctl->status, CSG_OK, CSG_ERR_TIMEOUT) == CSG_OK)
+            c.ctl->where = static_cast<int>(bi);
+        // edge points sent before the last barrier may still be on their way to this CTA: a millisecond outlasts them
+        const unsigned long long start = csg::global_timer_ns();
+        while (csg::global_timer_ns() - start < 1000000ull) {
+        }
     }
 }
 
@@ -1903,7 +1933,12 @@ template <typename T>
 struct FmgBuffers {
     std::vector<std::pair<int, int>> specs;
     std::vector<T*> A, B, B0, U, R;
+    csg::Control* ctl = nullptr;  // the scratch's first 256 bytes: status word, and the flag of k_any_nonzero
     int* flag = nullptr;
+    void take_control(Arena& ar) {
+        ctl = ar.take<csg::Control>(1);
+        flag = ctl ? ctl->pad : nullptr;
+    }
     bool carve(Arena& ar, int batch, int nx, int ny) {
         specs = grid_levels(nx, ny);
         const size_t L = specs.size();
@@ -1922,7 +1957,6 @@ struct FmgBuffers {
             }
             R[l] = ar.take<T>(2 * P * batch);
         }
-        flag = ar.take<int>(1);
         return ar.ok;
     }
 };
@@ -1935,6 +1969,8 @@ struct Fmg {
     int cycles, nit;
     cudaStream_t s;
     int nx0, ny0;
+    double timeout_s = 2.0;
+    int silent = -1;
 
     void params_at(size_t l, double out[5]) const {
         out[0] = base[0] * buf.specs[l].first / nx0;
@@ -1998,6 +2034,9 @@ struct Fmg {
         c.last = static_cast<int>(L - 1);
         c.nit = nit;
         c.cycles = count;
+        c.silent = silent;
+        c.timeout_ns = static_cast<unsigned long long>(timeout_s * 1e9);
+        c.ctl = buf.ctl;
         while ((1 << c.lgsize) < size) ++c.lgsize;
         long long at = kHead;
         auto take = [&](long long elements) {  // a byte offset of that many elements, aligned for pairs
@@ -2253,6 +2292,7 @@ struct StepBuffers {
     int nblocks;
     bool carve(Arena& ar, int batch, int nx, int ny) {
         const size_t P = static_cast<size_t>(nx) * ny * batch;
+        fmg.take_control(ar);
         for (int i = 0; i < 2; ++i) {
             map[i] = ar.take<T>(2 * P);
             jac[i] = ar.take<T>(4 * P);
@@ -2315,7 +2355,8 @@ Squaring<T> run_squaring(T* rb[2], T* ha[2], T* maps[2], T* jacs[2], int k, bool
 template <typename T>
 int dartel_step_impl(StepBuffers<T>& W, const T* source, const T* target, T* velocity, T* metrics, int metric_stride,
                      int batch, int nx, int ny, int k, const double* params, double lmreg, int cycles, int nit,
-                     int code, int assume_initial_nonzero, cudaStream_t s) {
+                     int code, int assume_initial_nonzero, bool first, cudaStream_t s) {
+    if (first) CSG_CUDA_CHECK(cudaMemsetAsync(W.fmg.ctl, 0, sizeof(csg::Control), s));
     const dim3 g = grid_for(nx * ny, batch);
     const double scale = 1.0 / static_cast<double>(1LL << k);
     const size_t P = static_cast<size_t>(nx) * ny * batch;
@@ -2359,13 +2400,15 @@ int dartel_step_impl(StepBuffers<T>& W, const T* source, const T* target, T* vel
     W.fmg.U[0] = initial;
     bool coarse_init = false;
     if (!assume_initial_nonzero) {
-        int flag = 0;
-        CSG_CUDA_CHECK(cudaMemsetAsync(W.fmg.flag, 0, sizeof(int), s));
+        csg::Control ctl{};
+        if (!first) CSG_CUDA_CHECK(cudaMemsetAsync(W.fmg.flag, 0, sizeof(int), s));
         (csg::note_launch(), csg::launch_pdl(k_any_nonzero<T>, static_cast<unsigned>((2 * P + kThreads - 1) / kThreads), kThreads, 0, s, initial, 2 * P,
                                                                                                      W.fmg.flag));
-        CSG_CUDA_CHECK(cudaMemcpyAsync(&flag, W.fmg.flag, sizeof(int), cudaMemcpyDeviceToHost, s));
+        CSG_CUDA_CHECK(cudaMemcpyAsync(&ctl, W.fmg.ctl, offsetof(csg::Control, pad) + sizeof(int), cudaMemcpyDeviceToHost, s));
         CSG_CUDA_CHECK(cudaStreamSynchronize(s));
-        coarse_init = flag == 0;
+        if (ctl.status != CSG_OK)  // of an earlier step's solve
+            return csg::fail(ctl.status, "dartel: a wait of the multigrid ran out (map %d)", ctl.where);
+        coarse_init = ctl.pad[0] == 0;
         if (coarse_init) CSG_CUDA_CHECK(cudaMemsetAsync(initial, 0, 2 * P * sizeof(T), s));
     }
     fmg.run(coarse_init);
@@ -2404,7 +2447,7 @@ int solve_typed(const void* source, const void* target, void* velocity, void* me
             int rc = dartel_step_impl<T>(W, static_cast<const T*>(source), static_cast<const T*>(target),
                                          static_cast<T*>(velocity), static_cast<T*>(metrics) + 3 * (index * its + it),
                                          3 * per, batch, nx, ny, index, params + 5 * index, lmreg, cycles, nit, code,
-                                         assume, s);
+                                         assume, index == 0 && it == 0, s);
             if (rc) return rc;
         }
     return CSG_OK;
@@ -2706,14 +2749,14 @@ int csg_dartel_step(int dtype, int batch, int nx, int ny, const void* source, co
         if (!W.carve(ar, batch, nx, ny)) return csg::fail(CSG_ERR_ARG, "dartel step: scratch too small");
         return dartel_step_impl<double>(W, static_cast<const double*>(source), static_cast<const double*>(target),
                                         static_cast<double*>(velocity), static_cast<double*>(metrics), 3, batch, nx, ny,
-                                        k, params, lmreg, cycles, nit, code, assume_initial_nonzero, s);
+                                        k, params, lmreg, cycles, nit, code, assume_initial_nonzero, true, s);
     }
     Arena ar{static_cast<char*>(scratch), scratch_bytes};
     StepBuffers<float> W;
     if (!W.carve(ar, batch, nx, ny)) return csg::fail(CSG_ERR_ARG, "dartel step: scratch too small");
     return dartel_step_impl<float>(W, static_cast<const float*>(source), static_cast<const float*>(target),
                                    static_cast<float*>(velocity), static_cast<float*>(metrics), 3, batch, nx, ny, k,
-                                   params, lmreg, cycles, nit, code, assume_initial_nonzero, s);
+                                   params, lmreg, cycles, nit, code, assume_initial_nonzero, true, s);
 }
 
 }  // extern "C"
@@ -2786,18 +2829,20 @@ int expdef_typed(int batch, int nx, int ny, const void* v, int k, void* map_out,
 
 template <typename T>
 int fmg_typed(int batch, int nx, int ny, const void* hess, const void* rhs, const double* params, int cycles, int nit,
-              void* u, int has_initial, int assume_nonzero, void* work, size_t bytes, cudaStream_t s) {
+              void* u, int has_initial, int assume_nonzero, void* work, size_t bytes, cudaStream_t s,
+              double timeout_s = 2.0, int silent = -1) {
     const size_t P = static_cast<size_t>(nx) * ny * batch;
     Arena ar{static_cast<char*>(work), bytes};
     FmgBuffers<T> buf;
+    buf.take_control(ar);
     if (!buf.carve(ar, batch, nx, ny)) return csg::fail(CSG_ERR_ARG, "fmg: scratch too small");
+    CSG_CUDA_CHECK(cudaMemsetAsync(buf.ctl, 0, sizeof(csg::Control), s));
     buf.A[0] = const_cast<T*>(static_cast<const T*>(hess));
     buf.B[0] = const_cast<T*>(static_cast<const T*>(rhs));
     buf.U[0] = static_cast<T*>(u);
     bool coarse_init = !has_initial;
     if (has_initial && !assume_nonzero) {
         int flag = 0;
-        CSG_CUDA_CHECK(cudaMemsetAsync(buf.flag, 0, sizeof(int), s));
         (csg::note_launch(), csg::launch_pdl(k_any_nonzero<T>, static_cast<unsigned>((2 * P + kThreads - 1) / kThreads), kThreads, 0, s, buf.U[0], 2 * P,
                                                                                                      buf.flag));
         CSG_CUDA_CHECK(cudaMemcpyAsync(&flag, buf.flag, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -2805,7 +2850,7 @@ int fmg_typed(int batch, int nx, int ny, const void* hess, const void* rhs, cons
         coarse_init = flag == 0;
     }
     if (coarse_init) CSG_CUDA_CHECK(cudaMemsetAsync(u, 0, 2 * P * sizeof(T), s));
-    Fmg<T> fmg{buf, batch, {params[0], params[1], params[2], params[3], params[4]}, cycles, nit, s, nx, ny};
+    Fmg<T> fmg{buf, batch, {params[0], params[1], params[2], params[3], params[4]}, cycles, nit, s, nx, ny, timeout_s, silent};
     fmg.run(coarse_init);
     CSG_CUDA_CHECK(cudaGetLastError());
     return CSG_OK;
@@ -3001,6 +3046,21 @@ int csg_dartel_fmg(int dtype, int batch, int nx, int ny, const void* hess, const
                                  scratch, scratch_bytes, s);
     return fmg_typed<float>(batch, nx, ny, hess, rhs, params, cycles, nit, u, has_initial, assume_initial_nonzero,
                             scratch, scratch_bytes, s);
+}
+
+int csg_selftest_exchange_timeout(int dtype, int batch, int nx, int ny, const void* hess, const void* rhs,
+                                  const double* params, int cycles, int nit, void* u, void* scratch,
+                                  size_t scratch_bytes, double timeout_s, int silent, csg_stream_t stream) {
+    int rc = check_grid(dtype, batch, nx, ny);
+    if (rc) return rc;
+    if (!hess || !rhs || !params || !u || !scratch || cycles < 0 || nit < 0 || !(timeout_s > 0.0) || timeout_s > 10.0)
+        return csg::fail(CSG_ERR_ARG, "exchange self-test: null pointer, negative cycles / nit or no 0 < timeout_s <= 10");
+    rc = check_levels(nx, ny);
+    if (rc) return rc;
+    cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+    return dtype == CSG_DTYPE_F64
+               ? fmg_typed<double>(batch, nx, ny, hess, rhs, params, cycles, nit, u, 1, 1, scratch, scratch_bytes, s, timeout_s, silent)
+               : fmg_typed<float>(batch, nx, ny, hess, rhs, params, cycles, nit, u, 1, 1, scratch, scratch_bytes, s, timeout_s, silent);
 }
 
 int csg_dartel_expdef(int dtype, int batch, int nx, int ny, const void* velocity, int k, void* map_out, void* jac_out,

@@ -38,8 +38,8 @@ from .device import resolve_device
 from .gifti import GiftiMesh, read_gifti_mesh, write_gifti_mesh
 from .rotation_pipeline import RotationPipeline, read_rotation_values
 from .surface_stencil import SurfaceStencil, build_surface_stencil
-from .surface_warp import (apply_flow_to_stenciled_sphere, average_xz_surfaces, solve_dartel_from_surfaces,
-                           solve_dartel_from_surfaces_many)
+from .surface_warp import (_solve_from_surfaces_many, apply_flow_to_stenciled_sphere, average_xz_surfaces, check_solve,
+                           solve_dartel_from_surfaces)
 
 
 @dataclass(frozen=True)
@@ -434,19 +434,20 @@ def register_meshes(
                 avg_source_stencil = rotated_builder.build(GiftiMesh(avg_source_sphere, source_sphere.faces),
                                                            normalize=False)
                 avg_source_dev = avg_source_stencil.to(target_device)
-                last_flow, avg_flow = solve_dartel_from_surfaces_many(
+                (last_flow, avg_flow), status = _solve_from_surfaces_many(
                     [(source_surface_dev, target_surface_dev, current_dev, target_dev, run_fwhm),
                      (on_device(avg_source_surface), on_device(avg_target_surface), avg_source_dev,
                       avg_target_stencil.to(target_device), avg_fwhm)],
                     curvtypes=tuple(curvtypes), loop=loop, n_steps=steps, cycles=cycles, nit=nit, its=its, code=code,
                     device=target_device, dtype=solve_dtype, parallel_sides=parallel_sides, cuda_graph=graph_requested)
             else:
-                last_flow = solve_one(source_surface_dev, target_surface_dev, current_dev, target_dev, run_fwhm,
-                                      loop).flow
+                solved = solve_one(source_surface_dev, target_surface_dev, current_dev, target_dev, run_fwhm, loop)
+                last_flow, status = solved.flow, solved.status
                 current_sphere = apply_flow_to_stenciled_sphere(
                     on_device(current_sphere), last_flow, current_dev, inverse=True, device=target_device,
                     dtype=solve_dtype).cpu().numpy().astype(np.float32)
             torch.cuda.synchronize(target_device)
+            check_solve(status)
             timings[f"dartel_run_{run_index}_seconds"] = time.perf_counter() - run_start
             if run_index + 1 < runs:
                 current_stencil = rotated_builder.build(GiftiMesh(current_sphere, source_sphere.faces),

@@ -22,12 +22,25 @@ from .dartel_grid import _addr, _dtype_code, _scratch, _tensor, expdef, resolve_
 
 @dataclass(frozen=True)
 class DartelSolveResult:
-    """Store a solved flow, warped feature maps, and DARTEL diagnostics."""
+    """Store a solved flow, warped feature maps, and DARTEL diagnostics.
+
+    ``status`` (int32, on the device) is 0, or the error of a wait between a multigrid solve's
+    CTAs that ran out (the flow is then NaN); :func:`check_solve` raises for it.
+    """
 
     flow: torch.Tensor
     source_maps: torch.Tensor
     target_maps: torch.Tensor
     metrics: torch.Tensor
+    status: torch.Tensor | None = None
+
+
+def check_solve(status: torch.Tensor) -> None:
+    """Raise ``RuntimeError`` for a solve whose status word reports an error (waits for the solve)."""
+
+    code = int(status)
+    if code != _native.CSG_OK:
+        raise RuntimeError(f"DARTEL solve: a wait between the CTAs of a multigrid solve ran out (status {code})")
 
 
 def default_dartel_parameters(loop: int = 6, *, mu: float = 0.125, lambda_: float = 0.0, lmreg: float = 1e-3,
@@ -63,6 +76,8 @@ class _Solver:
         self.velocity = torch.zeros((batch, 2, ny, nx), dtype=dtype, device=device)
         self.metrics = torch.zeros((batch, loop * its, 3), dtype=dtype, device=device)
         self.scratch = _scratch(dtype, device, batch, nx, ny)
+        self.status = self.scratch[4:8].view(torch.int32)[0]
+        self.after_status = self.scratch[256:]  # what follows a solve leaves its status word alone
         self.expdef_scratch = _scratch(dtype, device, 1, nx, ny)
         self.flow = torch.empty((2, ny, nx), dtype=dtype, device=device)
         self.flows = torch.empty((batch, 2, ny, nx), dtype=dtype, device=device)
@@ -106,7 +121,7 @@ class _Solver:
             _native.check(
                 lib.csg_dartel_expdef(
                     _dtype_code(self.dtype), count, self.nx, self.ny, self.last_velocity.data_ptr(), 10,
-                    self.flows.data_ptr(), None, self.scratch.data_ptr(), self.scratch.numel(), stream_handle,
+                    self.flows.data_ptr(), None, self.after_status.data_ptr(), self.after_status.numel(), stream_handle,
                 ),
                 "csg_dartel_expdef",
             )
@@ -114,7 +129,7 @@ class _Solver:
             _native.check(
                 lib.csg_dartel_expdef(
                     _dtype_code(self.dtype), self.batch, self.nx, self.ny, self.velocity.data_ptr(), 10,
-                    self.flows.data_ptr(), None, self.scratch.data_ptr(), self.scratch.numel(), stream_handle,
+                    self.flows.data_ptr(), None, self.after_status.data_ptr(), self.after_status.numel(), stream_handle,
                 ),
                 "csg_dartel_expdef",
             )
@@ -229,13 +244,14 @@ def solve_dartel_maps(source_maps, target_maps, *, loop: int = 6, lmreg: float =
         entry.solver.target.copy_(target)
         entry.replay()
         s = entry.solver
-        return DartelSolveResult(s.flow.clone(), s.source.clone(), s.target.clone(), s.metrics.clone())
+        return DartelSolveResult(s.flow.clone(), s.source.clone(), s.target.clone(), s.metrics.clone(),
+                                 s.status.clone())
     steps, ny, nx = (int(v) for v in source.shape)
     solver = _Solver(steps, ny, nx, dtype, dev, loop, lmreg, cycles, nit, its, code, assume_initial_nonzero)
     solver.source.copy_(source)
     solver.target.copy_(target)
     solver.launch(_native.stream_handle(like=solver.source))
-    return DartelSolveResult(solver.flow, source, target, solver.metrics)
+    return DartelSolveResult(solver.flow, source, target, solver.metrics, solver.status.clone())
 
 
 def solve_dartel_batch(source_maps, target_maps, *, loop: int = 6, lmreg: float = 1e-3, cycles: int = 3,
@@ -278,6 +294,15 @@ def solve_dartel_registrations(source_maps, target_maps, *, loop: int = 6, lmreg
     then assumes a nonzero initial update in every multigrid solve.
     """
 
+    return _solve_registrations(source_maps, target_maps, loop=loop, lmreg=lmreg, cycles=cycles, nit=nit, its=its,
+                                code=code, device=device, dtype=dtype, assume_initial_nonzero=assume_initial_nonzero,
+                                cuda_graph=cuda_graph)[:2]
+
+
+def _solve_registrations(source_maps, target_maps, *, loop, lmreg, cycles, nit, its, code, device, dtype,
+                         assume_initial_nonzero, cuda_graph):
+    """:func:`solve_dartel_registrations`'s flows and metrics, and the solve's status word."""
+
     dev = resolve_device(device)
     source = _tensor(source_maps, dev, dtype)
     target = _tensor(target_maps, dev, dtype)
@@ -299,13 +324,14 @@ def solve_dartel_registrations(source_maps, target_maps, *, loop: int = 6, lmreg
         entry.solver.target.copy_(target.reshape(regs * steps, ny, nx))
         entry.replay()
         solver = entry.solver
-        return solver.flows[:regs].clone(), solver.metrics.view(regs, steps, -1, 3).clone()
+        return (solver.flows[:regs].clone(), solver.metrics.view(regs, steps, -1, 3).clone(),
+                solver.status.clone())
     solver = _Solver(regs * steps, ny, nx, dtype, dev, loop, lmreg, cycles, nit, its, code,
                      bool(assume_initial_nonzero))
     solver.source.copy_(source.reshape(regs * steps, ny, nx))
     solver.target.copy_(target.reshape(regs * steps, ny, nx))
     solver.launch(_native.stream_handle(like=solver.source), "registrations", steps)
-    return solver.flows[:regs], solver.metrics.view(regs, steps, -1, 3)
+    return solver.flows[:regs], solver.metrics.view(regs, steps, -1, 3), solver.status.clone()
 
 
 def _surface_sheets(source_vertices, target_vertices, source_stencil, target_stencil, fwhm, curvtypes, n_steps, dev,
@@ -373,16 +399,26 @@ def solve_dartel_from_surfaces_many(problems, *, curvtypes: Sequence[int] = (5, 
     same ``assume_initial_nonzero`` / ``cuda_graph``.
     """
 
+    return _solve_from_surfaces_many(problems, curvtypes=curvtypes, loop=loop, n_steps=n_steps, lmreg=lmreg,
+                                     cycles=cycles, nit=nit, its=its, code=code, device=device, dtype=dtype,
+                                     parallel_sides=parallel_sides, assume_initial_nonzero=assume_initial_nonzero,
+                                     cuda_graph=cuda_graph)[0]
+
+
+def _solve_from_surfaces_many(problems, *, curvtypes, loop, n_steps, cycles, nit, its, code, device, dtype,
+                              parallel_sides, cuda_graph, lmreg=1e-3, assume_initial_nonzero=False):
+    """:func:`solve_dartel_from_surfaces_many`'s flows, and the solve's status word."""
+
     dev = resolve_device(device)
     sheets = [_surface_sheets(sv, tv, ss, ts, f, curvtypes, n_steps, dev, dtype, parallel_sides)
               for sv, tv, ss, ts, f in problems]
     if len({tuple(src.shape) for src, _ in sheets}) != 1:
         raise ValueError("batched registrations need sheets of one size")
-    flows, _ = solve_dartel_registrations(torch.stack([src for src, _ in sheets]), torch.stack([tgt for _, tgt in sheets]),
-                                          loop=loop, lmreg=lmreg, cycles=cycles, nit=nit, its=its, code=code,
-                                          device=dev, dtype=dtype, assume_initial_nonzero=assume_initial_nonzero,
-                                          cuda_graph=cuda_graph)
-    return [flows[r] for r in range(len(problems))]
+    flows, _, status = _solve_registrations(torch.stack([src for src, _ in sheets]),
+                                            torch.stack([tgt for _, tgt in sheets]), loop=loop, lmreg=lmreg,
+                                            cycles=cycles, nit=nit, its=its, code=code, device=dev, dtype=dtype,
+                                            assume_initial_nonzero=assume_initial_nonzero, cuda_graph=cuda_graph)
+    return [flows[r] for r in range(len(problems))], status
 
 
 def apply_flow_to_sphere(sphere_vertices, flow, *, unit_sphere_vertices=None, inverse: bool = True, device="auto",

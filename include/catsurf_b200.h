@@ -280,7 +280,11 @@ CSG_API int csg_dartel_data_backward(int dtype, int batch, int nx, int ny, const
                                      int k, int checkpoint_every, const void *checkpoints, const void *grad_scale,
                                      void *grad_velocity, void *scratch, size_t scratch_bytes, csg_stream_t stream);
 
-/* Scratch for csg_dartel_solve / _step / _fmg / _expdef / _squaring / _objfun. */
+/* Scratch for csg_dartel_solve / _step / _fmg / _expdef / _squaring / _objfun.  After a
+ * _solve, _step or _fmg its status word (csg_read_status) is CSG_OK, or CSG_ERR_TIMEOUT when a
+ * wait between the CTAs of a multigrid solve ran out after 2 s; `where` is then the map,
+ * whose update is NaN throughout.  A _solve without assume_initial_nonzero returns the
+ * error of all steps but its last. */
 CSG_API size_t csg_dartel_scratch_bytes(int dtype, int batch, int nx, int ny);
 
 /* Whole solve of `batch` independent (source, target) sheet pairs:
@@ -357,6 +361,15 @@ CSG_API int csg_dartel_resize(int dtype, int fields, int src_nx, int src_ny, con
 CSG_API int csg_dartel_fmg(int dtype, int batch, int nx, int ny, const void *hess, const void *rhs,
                            const double *params, int cycles, int nit, void *u, int has_initial,
                            int assume_initial_nonzero, void *scratch, size_t scratch_bytes, csg_stream_t stream);
+
+/* Self-test of the bounded waits between the CTAs of a multigrid solve (no reference
+ * counterpart): csg_dartel_fmg from the initial guess in u, in which CTA `silent` of every
+ * cluster sends no edge rows (-1: all do).  Its neighbours' waits give up after
+ * timeout_s (<= 10 s); the kernels return, the maps become NaN and scratch's status word
+ * CSG_ERR_TIMEOUT. */
+CSG_API int csg_selftest_exchange_timeout(int dtype, int batch, int nx, int ny, const void *hess, const void *rhs,
+                                          const double *params, int cycles, int nit, void *u, void *scratch,
+                                          size_t scratch_bytes, double timeout_s, int silent, csg_stream_t stream);
 
 /* expdef: scaling and squaring of id + v / 2^k (dartel_grid.py:1619-1666);
  * jac_out may be NULL. */

@@ -190,3 +190,54 @@ def test_batches_of_several_waves(native_library, dtype, nx, ny, batch, nit, res
     torch.cuda.synchronize()
     assert (launches[1] - launches[0] == 1) == resident
     assert torch.equal(u, _separate(lib, code, hess, rhs, start, 2, nit))
+
+
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+@pytest.mark.parametrize(
+    "nx, ny, batch, silent",
+    [(64, 32, 1, 0), (64, 32, 3, 3), (64, 33, 40, 1), (128, 65, 2, 8), (256, 128, 1, 15), (256, 128, 2, 0), (512, 256, 1, 7)],
+)
+def test_waits_that_run_out_report_it(native_library, dtype, nx, ny, batch, silent):
+    """A CTA that sends no edge rows: its neighbours' waits run out, every kernel returns, all rows of all maps are
+    NaN and the status word tells; the next solve on the same scratch is whole again."""
+
+    lib = native_library
+    code = 1 if dtype == torch.float64 else 0
+    hess, rhs, start = _problem(nx, ny, batch, dtype, "plain")
+    params = _params((nx, ny), (nx, ny))
+    scratch = torch.empty(lib.csg_dartel_scratch_bytes(code, batch, nx, ny), dtype=torch.uint8, device="cuda")
+
+    def status():
+        word = ctypes.c_int(1)
+        assert lib.csg_read_status(scratch.data_ptr(), 0, ctypes.addressof(word), 0) == 0
+        return word.value
+
+    def solve(timeout, rank):
+        u = start.clone()
+        assert lib.csg_selftest_exchange_timeout(code, batch, nx, ny, hess.data_ptr(), rhs.data_ptr(), params, 2, 2,
+                                                 u.data_ptr(), scratch.data_ptr(), scratch.numel(), timeout, rank, 0) == 0
+        return u
+
+    lost = solve(0.005, silent)
+    assert status() == -3  # CSG_ERR_TIMEOUT
+    assert torch.isnan(lost).all()
+    whole = solve(2.0, -1)
+    assert status() == 0
+    u = start.clone()
+    assert lib.csg_dartel_fmg(code, batch, nx, ny, hess.data_ptr(), rhs.data_ptr(), params, 2, 2, u.data_ptr(), 1, 1,
+                              scratch.data_ptr(), scratch.numel(), 0) == 0
+    assert status() == 0
+    assert torch.isfinite(u).all() and torch.equal(u, whole)
+
+
+def test_a_lost_solve_raises():
+    """The Python layer turns a solve's status word into an error, and a solve's own is zero."""
+
+    from cat_surface_gpu_b200.surface_warp import check_solve, solve_dartel_maps
+
+    sheets = torch.rand(2, 1, 16, 32, dtype=torch.float64, device="cuda", generator=torch.Generator("cuda").manual_seed(0))
+    for graph in (False, True):
+        result = solve_dartel_maps(sheets[0], sheets[1], loop=2, its=1, cuda_graph=graph)
+        check_solve(result.status)
+        with pytest.raises(RuntimeError, match="ran out"):
+            check_solve(result.status - 3)
