@@ -898,8 +898,9 @@ Layout layout(int n, int nf, int batch, long long nnz) {
     L.r = take(8 * nb);
     L.z = take(8 * nb);
     L.pv = take(8 * nb);
-    L.ap = take(8 * nb);
-    L.pub = L.r;  // the SOR's published words (kWordPitch quads per value) lie over the CG's four vectors
+    L.ap = take(8 * nb + 8);
+    L.pub = L.r;  // the SOR's published words (kWordPitch quads per value) lie over the CG's four vectors, 8 bytes on
+                  // where the scratch is aligned for doubles alone
     L.level_of = take(4 * static_cast<size_t>(n));
     L.total = at;
     return L;
@@ -1062,7 +1063,7 @@ int csg_depth_potential(const float* geometry, int batch, int n, const int32_t* 
             p.max_row = 3 * max_incidences + 1;
             p.relaxation = relaxation;
             p.timeout_ns = timeout_ns;
-            p.pub = reinterpret_cast<csg::Quad*>(base + L.pub);
+            p.pub = reinterpret_cast<csg::Quad*>((reinterpret_cast<uintptr_t>(base + L.pub) + 15) & ~uintptr_t(15));
             p.level_of = reinterpret_cast<int*>(base + L.level_of);
             (csg::note_launch(), k_level_of<<<dim3(blocks(n, kThreads) > 64 ? 64 : blocks(n, kThreads), n_levels),
                                               kThreads, 0, s>>>(order, level_begin, level_end, p.level_of));

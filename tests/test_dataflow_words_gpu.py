@@ -92,3 +92,26 @@ def test_depth_sor_equals_the_oracle(native_library, n, seed, lanes, batch):
             want, _, want_residual = oracle_depth.System(surfaces[b], faces).sor(groups, sweeps)
             np.testing.assert_array_equal(got[b].cpu().numpy(), want)
             assert residual[b] == want_residual
+
+
+@pytest.mark.parametrize("n", [60, 96])  # 96 vertices: the vectors that the words lie over leave no gap
+@pytest.mark.parametrize("batch", [1, 2])
+def test_depth_scratch_needs_the_alignment_of_a_double(native_library, monkeypatch, n, batch):
+    """Scratch of just the size asked for, 8 bytes off a multiple of 16: the same values."""
+
+    from cat_surface_gpu_b200 import rotation_feature
+
+    vertices, faces = synthetic.folded_hull(n, 2)
+    surfaces = torch.as_tensor(np.stack([vertices * np.float32(1.0 + 0.25 * b) for b in range(batch)]), device="cuda:0")
+    topology = rotation_feature.DepthTopology.build(faces, n, torch.device("cuda:0"))
+    empty = torch.empty
+
+    def off_by_eight(*size, dtype=None, **options):
+        if dtype is torch.uint8:
+            return empty(size[0] + 8, dtype=dtype, **options)[8:]
+        return empty(*size, dtype=dtype, **options)
+
+    want = rotation_feature.depth_potential(surfaces, topology, max_iter=25)
+    monkeypatch.setattr(rotation_feature.torch, "empty", off_by_eight)
+    got = rotation_feature.depth_potential(surfaces, topology, max_iter=25)
+    assert torch.equal(got[0], want[0]) and got[1:] == want[1:]
