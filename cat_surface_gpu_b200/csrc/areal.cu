@@ -35,6 +35,7 @@
 #include <cuda_runtime.h>
 
 #include "common.cuh"
+#include "cooperative.h"
 #include "errors.h"
 
 namespace {
@@ -549,6 +550,12 @@ __device__ __forceinline__ bool poll_ring(const ArealParams& p, const Quad* word
 
 constexpr int kStagePitch = 34;  // doubles per staged row: the four rows of a warp start on different banks
 
+// A warp's staged face terms (the float32 mode sums by shuffles).
+template <int MODE>
+__host__ __device__ constexpr int dataflow_stage_bytes() {
+    return sizeof(typename Traits<MODE>::Acc) == 8 ? 4 * kStagePitch * static_cast<int>(sizeof(double)) : 0;
+}
+
 // The area total (lanes 0..2) and one coordinate's weighted sum (lane k: coordinate k) of up
 // to G staged faces, added in slot order.  Slots past the last face hold +0, which leaves a
 // sum that started from +0 unchanged, so the G additions need no test.
@@ -710,7 +717,7 @@ __global__ void __launch_bounds__(512) areal_dataflow_kernel(ArealParams p) {
     // level / D), ring and face codes; per level the owned range; per residue the
     // top level
     double (*stage)[kStagePitch] = reinterpret_cast<double (*)[kStagePitch]>(smem) + 4 * (threadIdx.x >> 5);
-    float4* pos0 = reinterpret_cast<float4*>(smem + (blockDim.x / 32) * 4 * kStagePitch * sizeof(double));
+    float4* pos0 = reinterpret_cast<float4*>(smem + (blockDim.x / 32) * dataflow_stage_bytes<MODE>());
     float4* pos = pos0 + (threadIdx.x / G) * cap;
     int4* lmeta = reinterpret_cast<int4*>(pos0 + (blockDim.x / G) * cap);
     int* lring = reinterpret_cast<int*>(lmeta + p.nloc_max);
@@ -819,42 +826,6 @@ __global__ void __launch_bounds__(512) areal_dataflow_kernel(ArealParams p) {
 constexpr size_t kMaxTopologySmem = 200 * 1024;
 constexpr size_t kMaxDataflowSmem = 216 * 1024;  // the staged face terms are part of it
 
-template <int MODE, int G, bool SMEM>
-int launch_variant(ArealParams params, int n_ctas, int threads, size_t smem, cudaStream_t stream) {
-    auto kernel = areal_sweeps_kernel<MODE, G, SMEM>;
-    int device = 0, sms = 0, per_sm = 0;
-    CSG_CUDA_CHECK(cudaGetDevice(&device));
-    CSG_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    if (SMEM) CSG_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    CSG_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
-    if (per_sm < 1 || n_ctas > per_sm * sms)
-        return csg::fail(CSG_ERR_LAUNCH, "areal sweeps: %d CTAs x %d threads (%zu B smem) cannot be co-resident (%d per SM, %d SMs)",
-                         n_ctas, threads, smem, per_sm, sms);
-    void* args[] = {&params};
-    CSG_CUDA_CHECK(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), dim3(n_ctas), dim3(threads), args,
-                                               smem, stream));
-    csg::note_launch();
-    return CSG_OK;
-}
-
-template <int MODE, int G>
-int launch_dataflow(ArealParams params, int n_ctas, int threads, size_t smem, cudaStream_t stream) {
-    auto kernel = areal_dataflow_kernel<MODE, G>;
-    int device = 0, sms = 0, per_sm = 0;
-    CSG_CUDA_CHECK(cudaGetDevice(&device));
-    CSG_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    CSG_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    CSG_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
-    if (per_sm < 1 || n_ctas > per_sm * sms)
-        return csg::fail(CSG_ERR_LAUNCH, "areal sweeps: %d CTAs x %d threads (%zu B smem) cannot be co-resident (%d per SM, %d SMs)",
-                         n_ctas, threads, smem, per_sm, sms);
-    void* args[] = {&params};
-    CSG_CUDA_CHECK(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), dim3(n_ctas), dim3(threads), args,
-                                               smem, stream));
-    csg::note_launch();
-    return CSG_OK;
-}
-
 template <int MODE, int G>
 int launch(ArealParams params, int n_ctas, int threads, cudaStream_t stream) {
     int device = 0, sms = 0;
@@ -862,6 +833,10 @@ int launch(ArealParams params, int n_ctas, int threads, cudaStream_t stream) {
     CSG_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     if (n_ctas <= 0) n_ctas = sms;
     params.nloc_max = (params.n + n_ctas - 1) / n_ctas;
+    void* args[] = {&params};
+    bool launched = false;
+    // The dataflow form, the barrier form with its topology in shared memory, and from global memory: the first
+    // whose CTAs fit the device together.
     if constexpr (MODE != CSG_ARITH_FP64) {
         // a ring has at most 2 max_degree + 1 vertices
         if (params.allow_dataflow && params.max_degree > 0 && 2 * params.max_degree + 1 <= kRingMax) {
@@ -870,17 +845,27 @@ int launch(ArealParams params, int n_ctas, int threads, cudaStream_t stream) {
                                      ? static_cast<unsigned int>(((1LL << 32) + pe - 1) / pe)
                                      : 0u;
             const size_t cap = dataflow_ring_capacity(params.max_degree, G);
-            const size_t smem = (threads / 32) * 4 * kStagePitch * sizeof(double) + sizeof(float4) * (threads / G) * cap +
+            const size_t smem = (threads / 32) * dataflow_stage_bytes<MODE>() + sizeof(float4) * (threads / G) * cap +
                                 static_cast<size_t>(params.nloc_max) * sizeof(int) * (cap + params.max_degree + 4) +
                                 sizeof(int) * (2 * static_cast<size_t>(params.n_levels) + params.stride);
-            if (smem <= kMaxDataflowSmem) return launch_dataflow<MODE, G>(params, n_ctas, threads, smem, stream);
+            if (smem <= kMaxDataflowSmem) {
+                const int rc = csg::launch_if_resident(reinterpret_cast<const void*>(areal_dataflow_kernel<MODE, G>), n_ctas,
+                                                       threads, smem, args, stream, launched);
+                if (rc || launched) return rc;
+            }
         }
     }
     const size_t smem = static_cast<size_t>(params.nloc_max) * (params.max_degree * sizeof(int4) + 2 * sizeof(int)) +
                         sizeof(int) * (2 * static_cast<size_t>(params.n_levels) + params.stride);
-    if (params.max_degree > 0 && smem <= kMaxTopologySmem)
-        return launch_variant<MODE, G, true>(params, n_ctas, threads, smem, stream);
-    return launch_variant<MODE, G, false>(params, n_ctas, threads, 0, stream);
+    if (params.max_degree > 0 && smem <= kMaxTopologySmem) {
+        const int rc = csg::launch_if_resident(reinterpret_cast<const void*>(areal_sweeps_kernel<MODE, G, true>), n_ctas,
+                                               threads, smem, args, stream, launched);
+        if (rc || launched) return rc;
+    }
+    const int rc = csg::launch_if_resident(reinterpret_cast<const void*>(areal_sweeps_kernel<MODE, G, false>), n_ctas,
+                                           threads, 0, args, stream, launched);
+    if (rc || launched) return rc;
+    return csg::fail(CSG_ERR_LAUNCH, "areal sweeps: %d CTAs x %d threads cannot be co-resident on %d SMs", n_ctas, threads, sms);
 }
 
 template <int MODE>

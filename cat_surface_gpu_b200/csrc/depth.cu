@@ -32,6 +32,7 @@
 #include <cuda_runtime.h>
 
 #include "common.cuh"
+#include "cooperative.h"
 #include "errors.h"
 
 namespace {
@@ -911,60 +912,36 @@ inline unsigned blocks(long long n, int threads) { return static_cast<unsigned>(
 constexpr size_t kMaxRowSmem = 200 * 1024;
 constexpr size_t kMaxDataflowSmem = 206 * 1024;  // its staged rows are longer than the 16-entry rings they lie over
 
-template <int G, bool SMEM>
-int launch_sor(const SorParams& params, int n_ctas, int threads, size_t smem, cudaStream_t s) {
-    auto kernel = k_depth_sor<G, SMEM>;
-    int device = 0, sms = 0, per_sm = 0;
-    CSG_CUDA_CHECK(cudaGetDevice(&device));
-    CSG_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    CSG_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    CSG_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
-    if (per_sm < 1 || n_ctas > per_sm * sms)
-        return csg::fail(CSG_ERR_LAUNCH, "depth SOR: %d CTAs x %d threads (%zu B smem) cannot be co-resident", n_ctas,
-                         threads, smem);
-    SorParams p = params;
-    void* args[] = {&p};
-    CSG_CUDA_CHECK(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), dim3(n_ctas), dim3(threads), args,
-                                               smem, s));
-    csg::note_launch();
-    return CSG_OK;
-}
-
-template <int G>
-int launch_sor_df(const SorParams& params, int n_ctas, int threads, size_t smem, cudaStream_t s) {
-    auto kernel = k_depth_sor_df<G>;
-    int device = 0, sms = 0, per_sm = 0;
-    CSG_CUDA_CHECK(cudaGetDevice(&device));
-    CSG_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    CSG_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    CSG_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
-    if (per_sm < 1 || n_ctas > per_sm * sms)
-        return csg::fail(CSG_ERR_LAUNCH, "depth SOR: %d CTAs x %d threads (%zu B smem) cannot be co-resident", n_ctas,
-                         threads, smem);
-    SorParams p = params;
-    void* args[] = {&p};
-    CSG_CUDA_CHECK(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), dim3(n_ctas), dim3(threads), args,
-                                               smem, s));
-    csg::note_launch();
-    return CSG_OK;
-}
-
 template <int G>
 int dispatch_sor(SorParams p, int n_ctas, int threads, cudaStream_t s) {
     p.nloc_max = (p.n + n_ctas - 1) / n_ctas;
+    void* args[] = {&p};
+    bool launched = false;
+    // the forms in the order of their speed; the first whose CTAs fit the device together (see the Surf2Sphere sweeps)
     // dataflow form: a row's distinct columns (at most 2 max_incidences + 1) fit the ring
     if (p.pub && p.max_row > 0 && p.max_row <= kSRowMax && 2 * ((p.max_row - 1) / 3) + 1 <= kSRing) {
         const long long nb = static_cast<long long>(p.batch) * p.nloc_max;
         const size_t smem = sizeof(double) * (static_cast<size_t>(threads / G) * kSRowMax + nb * (p.max_row + 2)) +
                             sizeof(int) * (static_cast<size_t>(p.nloc_max) * (kSRing + 4) + 2 * static_cast<size_t>(p.n_levels)) +
                             static_cast<size_t>(p.nloc_max) * p.max_row;
-        if (smem <= kMaxDataflowSmem) return launch_sor_df<G>(p, n_ctas, threads, smem, s);
+        if (smem <= kMaxDataflowSmem) {
+            const int rc = csg::launch_if_resident(reinterpret_cast<const void*>(k_depth_sor_df<G>), n_ctas, threads, smem, args,
+                                                   s, launched);
+            if (rc || launched) return rc;
+        }
     }
     const size_t ints = static_cast<size_t>(p.nloc_max) * (p.max_row + 2) + 2 * static_cast<size_t>(p.n_levels);
     const size_t smem = sizeof(double) * static_cast<size_t>(p.batch) * p.nloc_max * (p.max_row + 3) + sizeof(int) * ints;
-    if (p.max_row > 0 && smem <= kMaxRowSmem) return launch_sor<G, true>(p, n_ctas, threads, smem, s);
+    if (p.max_row > 0 && smem <= kMaxRowSmem) {
+        const int rc = csg::launch_if_resident(reinterpret_cast<const void*>(k_depth_sor<G, true>), n_ctas, threads, smem, args,
+                                               s, launched);
+        if (rc || launched) return rc;
+    }
     p.max_row = 0;
-    return launch_sor<G, false>(p, n_ctas, threads, 0, s);
+    const int rc = csg::launch_if_resident(reinterpret_cast<const void*>(k_depth_sor<G, false>), n_ctas, threads, 0, args, s,
+                                           launched);
+    if (rc || launched) return rc;
+    return csg::fail(CSG_ERR_LAUNCH, "depth SOR: %d CTAs x %d threads cannot be co-resident", n_ctas, threads);
 }
 
 }  // namespace

@@ -26,6 +26,7 @@
 #include <cuda_runtime.h>
 
 #include "common.cuh"
+#include "cooperative.h"
 #include "errors.h"
 
 namespace {
@@ -807,44 +808,6 @@ Layout layout(int n, int nf) {
 constexpr size_t kMaxTopologySmem = 160 * 1024;
 constexpr size_t kMaxDataflowSmem = 176 * 1024;  // the staged terms are part of it
 
-template <int G, bool SMEM>
-int launch_variant(const PassParams& params, int n_ctas, int threads, size_t smem, cudaStream_t s) {
-    auto kernel = smooth_passes_kernel<G, SMEM>;
-    int device = 0, sms = 0, per_sm = 0;
-    CSG_CUDA_CHECK(cudaGetDevice(&device));
-    CSG_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    if (SMEM) CSG_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    CSG_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
-    if (per_sm < 1 || n_ctas > per_sm * sms)
-        return csg::fail(CSG_ERR_LAUNCH, "preprocess passes: %d CTAs x %d threads (%zu B smem) cannot be co-resident",
-                         n_ctas, threads, smem);
-    PassParams p = params;
-    void* args[] = {&p};
-    CSG_CUDA_CHECK(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), dim3(n_ctas), dim3(threads), args,
-                                               smem, s));
-    csg::note_launch();
-    return CSG_OK;
-}
-
-template <int G>
-int launch_dataflow(const PassParams& params, int n_ctas, int threads, size_t smem, cudaStream_t s) {
-    auto kernel = smooth_passes_df<G>;
-    int device = 0, sms = 0, per_sm = 0;
-    CSG_CUDA_CHECK(cudaGetDevice(&device));
-    CSG_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    CSG_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    CSG_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
-    if (per_sm < 1 || n_ctas > per_sm * sms)
-        return csg::fail(CSG_ERR_LAUNCH, "preprocess passes: %d CTAs x %d threads (%zu B smem) cannot be co-resident",
-                         n_ctas, threads, smem);
-    PassParams p = params;
-    void* args[] = {&p};
-    CSG_CUDA_CHECK(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), dim3(n_ctas), dim3(threads), args,
-                                               smem, s));
-    csg::note_launch();
-    return CSG_OK;
-}
-
 template <int G>
 int launch_passes(PassParams params, int n_ctas, int threads, cudaStream_t s) {
     int device = 0, sms = 0;
@@ -852,17 +815,31 @@ int launch_passes(PassParams params, int n_ctas, int threads, cudaStream_t s) {
     CSG_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     if (n_ctas <= 0) n_ctas = sms;
     params.nloc_max = (params.n + n_ctas - 1) / n_ctas;
+    void* args[] = {&params};
+    bool launched = false;
+    // the forms in the order of their speed; the first whose CTAs fit the device together (see the sweeps)
     if (params.max_degree > 0 && params.max_degree + 1 <= kPRing) {
         const size_t cap = static_cast<size_t>(params.max_degree) + 1;
         const size_t smem = (threads / 32) * 4 * kStagePitch * sizeof(double) + sizeof(float4) * (threads / G) * cap +
                             sizeof(int) * (static_cast<size_t>(params.nloc_max) * (cap + 4) +
                                            2 * static_cast<size_t>(params.n_levels));
-        if (smem <= kMaxDataflowSmem) return launch_dataflow<G>(params, n_ctas, threads, smem, s);
+        if (smem <= kMaxDataflowSmem) {
+            const int rc = csg::launch_if_resident(reinterpret_cast<const void*>(smooth_passes_df<G>), n_ctas, threads, smem,
+                                                   args, s, launched);
+            if (rc || launched) return rc;
+        }
     }
     const size_t smem = sizeof(int) * (static_cast<size_t>(params.nloc_max) * (params.max_degree + 2) +
                                        2 * static_cast<size_t>(params.n_levels));
-    if (params.max_degree > 0 && smem <= kMaxTopologySmem) return launch_variant<G, true>(params, n_ctas, threads, smem, s);
-    return launch_variant<G, false>(params, n_ctas, threads, 0, s);
+    if (params.max_degree > 0 && smem <= kMaxTopologySmem) {
+        const int rc = csg::launch_if_resident(reinterpret_cast<const void*>(smooth_passes_kernel<G, true>), n_ctas, threads,
+                                               smem, args, s, launched);
+        if (rc || launched) return rc;
+    }
+    const int rc = csg::launch_if_resident(reinterpret_cast<const void*>(smooth_passes_kernel<G, false>), n_ctas, threads, 0,
+                                           args, s, launched);
+    if (rc || launched) return rc;
+    return csg::fail(CSG_ERR_LAUNCH, "preprocess passes: %d CTAs x %d threads cannot be co-resident", n_ctas, threads);
 }
 
 // The passes queued since the last launch, launched as one wavefront.

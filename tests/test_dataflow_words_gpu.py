@@ -115,3 +115,66 @@ def test_depth_scratch_needs_the_alignment_of_a_double(native_library, monkeypat
     monkeypatch.setattr(rotation_feature.torch, "empty", off_by_eight)
     got = rotation_feature.depth_potential(surfaces, topology, max_iter=25)
     assert torch.equal(got[0], want[0]) and got[1:] == want[1:]
+
+
+def _tube(sides, rows):
+    """(vertices, faces) of a long closed tube, numbered along it: thousands of dependency levels, two vertices of
+    ``sides`` faces."""
+
+    angle = 2 * np.pi * np.arange(sides) / sides
+    z = 0.05 * (np.arange(rows) - (rows - 1) / 2)
+    radius = 30 + 0.1 * (np.arange(rows) % 7)
+    rings = np.stack((radius[:, None] * np.cos(angle), radius[:, None] * np.sin(angle), np.repeat(z[:, None], sides, 1)), -1)
+    vertices = np.concatenate((rings.reshape(-1, 3), [[0, 0, z[0] - 5], [0, 0, z[-1] + 5]]))
+    here, there = np.arange(sides), (np.arange(sides) + 1) % sides
+    low, high = np.stack((here, there, here + sides), 1), np.stack((there, there + sides, here + sides), 1)
+    walls = (np.concatenate((low, high))[None] + sides * np.arange(rows - 1)[:, None, None]).reshape(-1, 3)
+    n, top = sides * rows, sides * (rows - 1)
+    ends = np.concatenate((np.stack((np.full(sides, n), there, here), 1),
+                           np.stack((np.full(sides, n + 1), top + here, top + there), 1)))
+    return vertices.astype(np.float32), np.concatenate((walls, ends)).astype(np.int32)
+
+
+# Launches whose shared memory the 8-byte words' layout just held for two CTAs to an SM.
+@pytest.mark.parametrize("arithmetic", ["cat", "fp32"])
+def test_sweeps_of_two_large_ctas_to_an_sm(native_library, arithmetic):
+    from cat_surface_gpu_b200.autotune import sm_count
+    from cat_surface_gpu_b200.gifti import GiftiMesh
+    from cat_surface_gpu_b200.surf2sphere import Surf2SphereTopology, run_areal_smoothing_cuda
+
+    vertices, faces = _tube(9, 4080)
+    topology = Surf2SphereTopology.plan_only(GiftiMesh(vertices, faces))
+    launch = {"n_ctas": 2 * sm_count(), "threads_per_cta": 512, "lanes_per_vertex": 8}
+    got, _ = run_areal_smoothing_cuda(vertices, faces, topology, iterations=4, project_every=2, radius=60.0,
+                                      arithmetic=arithmetic, launch=launch)
+    np.testing.assert_array_equal(got, oracle.areal_sweeps(vertices, faces, iterations=4, project_every=2, radius=60.0,
+                                                           arithmetic=arithmetic))
+
+
+def test_stage_passes_of_two_large_ctas_to_an_sm(native_library):
+    from cat_surface_gpu_b200.autotune import sm_count
+    from cat_surface_gpu_b200.gifti import GiftiMesh
+    from cat_surface_gpu_b200.surf2sphere import Surf2SphereTopology, run_surf2sphere_preprocess_cuda
+    from oracle import preprocess as oracle_pre
+
+    vertices, faces = _tube(16, 4480)
+    topology = Surf2SphereTopology.plan_only(GiftiMesh(vertices, faces))
+    launch = {"n_ctas": 2 * sm_count(), "threads_per_cta": 512, "lanes_per_vertex": 16}
+    got, _ = run_surf2sphere_preprocess_cuda(vertices, faces, topology, stop_at=1, desired_surface_area=1.0, launch=launch)
+    np.testing.assert_array_equal(got, oracle_pre.preprocess(vertices, faces, stop_at=1))
+
+
+def test_depth_sor_of_two_large_ctas_to_an_sm(native_library):
+    from cat_surface_gpu_b200.autotune import sm_count
+    from cat_surface_gpu_b200.rotation_feature import DepthTopology, depth_potential
+    from cat_surface_gpu_b200.surface_stencil import resampling_sphere
+
+    points, faces = resampling_sphere(4)
+    n = points.shape[0]
+    topology = DepthTopology.build(faces, n, torch.device("cuda:0"))
+    surfaces = torch.as_tensor(np.stack([points * (40.0 + b) for b in range(64)]).astype(np.float32), device="cuda:0")
+    launch = {"n_ctas": 2 * sm_count(), "threads_per_cta": 512, "lanes_per_row": 4}
+    got, _, _ = depth_potential(surfaces, topology, max_iter=20, launch=launch)
+    for b in (0, 63):
+        want, _, _ = depth_potential(surfaces[b], topology, max_iter=20)
+        assert torch.equal(got[b], want[0])
