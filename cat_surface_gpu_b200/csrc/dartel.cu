@@ -1551,8 +1551,9 @@ __global__ void __launch_bounds__(kResidentThreads, sizeof(T) == 4 ? 2 : 1)
     const T* B = L.B + 2 * bi * P;
     const T* Uin = L.Uin + 2 * bi * P;
     // taps of the coarse rows whose centre tap may lie in the tile / of the region's rows
-    const int Y0 = DOWN ? max(0, (y0 - 2) * L.cny / ny - 1) : gy0;
-    const int rows = DOWN ? min(L.cny, (y1 + 2) * L.cny / ny + 2) - Y0 : wy;
+    // (64-bit products: they pass 2^31 from 65,536 rows on)
+    const int Y0 = DOWN ? max(0, static_cast<int>((y0 - 2LL) * L.cny / ny) - 1) : gy0;
+    const int rows = DOWN ? min(L.cny, static_cast<int>((y1 + 2LL) * L.cny / ny) + 2) - Y0 : wy;
     for (int k = thread; k < rows; k += kResidentThreads)
         reinterpret_cast<AxisTaps<T>*>(resident_smem + taps)[k] =
             DOWN ? row_taps<T>(Y0 + k, ny, L.cny, 1) : row_taps<T>(Y0 + k, L.cny, ny, L.cnx);

@@ -241,3 +241,19 @@ def test_a_lost_solve_raises():
         check_solve(result.status)
         with pytest.raises(RuntimeError, match="ran out"):
             check_solve(result.status - 3)
+
+
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+@pytest.mark.parametrize("nx, ny", [(4, 65536), (16, 70000), (8, 100001)])
+def test_legs_of_very_tall_grids(native_library, dtype, nx, ny):
+    """Grids of so many rows that the products of row numbers pass 32 bits."""
+
+    lib = native_library
+    code = 1 if dtype == torch.float64 else 0
+    hess, rhs, start = _problem(nx, ny, 1, dtype, "plain")
+    scratch = torch.empty(lib.csg_dartel_scratch_bytes(code, 1, nx, ny), dtype=torch.uint8, device="cuda")
+    u = start.clone()
+    assert lib.csg_dartel_fmg(code, 1, nx, ny, hess.data_ptr(), rhs.data_ptr(), _params((nx, ny), (nx, ny)), 1, 3, u.data_ptr(),
+                              1, 1, scratch.data_ptr(), scratch.numel(), 0) == 0
+    torch.cuda.synchronize()
+    assert torch.equal(u, _separate(lib, code, hess, rhs, start, 1, 3))
