@@ -10,6 +10,7 @@ from __future__ import annotations
 
 import ctypes
 
+import numpy as np
 import pytest
 import torch
 
@@ -257,3 +258,57 @@ def test_legs_of_very_tall_grids(native_library, dtype, nx, ny):
                               1, 1, scratch.data_ptr(), scratch.numel(), 0) == 0
     torch.cuda.synchronize()
     assert torch.equal(u, _separate(lib, code, hess, rhs, start, 1, 3))
+
+
+def _operands(kind, count, rng):
+    """(numerators [2, count], first diagonal entries [count]): exponents and mantissas of the point systems."""
+
+    def mantissa(shape):
+        special = np.array([1.0, 2.0 - 2.0**-52, 1.0 + 2.0**-52, 1.5, 2.0 - 2.0**-51])  # power of two, all ones, ...
+        m = 1.0 + rng.random(shape)
+        return np.where(rng.random(shape) < 0.3, rng.choice(special, shape), m) * rng.choice([-1.0, 1.0], shape)
+
+    if kind == "inside":
+        ea, ed = rng.integers(-500, 500, (2, count)), rng.integers(-400, 401, count)
+    elif kind == "edges":  # of the windows in which the reciprocal is used, on both sides
+        ea = rng.choice([-502, -501, -500, -499, 498, 499, 500, 501], (2, count))
+        ed = rng.choice([-402, -401, -400, -399, 398, 399, 400, 401], count)
+    else:
+        ea, ed = rng.integers(-1073, 1024, (2, count)), rng.integers(-1073, 1024, count)
+    det = np.ldexp(mantissa(count), ed)
+    first = det / 1.0000000001  # the determinant's rounding takes it back to det, or next to it
+    for near in (np.nextafter(first, 0.0), np.nextafter(first, 2.0 * first)):
+        first = np.where((first * 1.0000000001 != det) & (near * 1.0000000001 == det), near, first)
+    numerators = np.ldexp(mantissa((2, count)), ea)
+    if kind == "outside":
+        numerators[:, ::97] = 0.0
+        first[::89] = 0.0
+    return numerators, first
+
+
+@pytest.mark.parametrize("kind", ["inside", "edges", "outside"])
+def test_quotients_equal_the_division(native_library, kind):
+    """Point systems of one point without weights: the resident cycle's quotients by the kept reciprocal against
+    csg_dartel_relax's divisions, bit for bit."""
+
+    lib = native_library
+    batch, rng = 65535, np.random.default_rng(len(kind))
+    params = (ctypes.c_double * 5)(1.0, 1.0, 0.0, 0.0, 0.0)
+    scratch = torch.empty(lib.csg_dartel_scratch_bytes(1, batch, 1, 1), dtype=torch.uint8, device="cuda")
+    hits = 0
+    with np.errstate(over="ignore", under="ignore"):
+        for _ in range(16):
+            numerators, first = _operands(kind, batch, rng)
+            # det = first * 1 * 1.0000000001; quotients numerators[0] / det and (first * numerators[1]) / det
+            hess = torch.as_tensor(np.stack((first, np.ones(batch), np.zeros(batch)), 1), device="cuda").contiguous()
+            rhs = torch.as_tensor(np.ascontiguousarray(numerators.T), device="cuda")
+            plain, kept = torch.zeros_like(rhs), torch.zeros_like(rhs)
+            assert lib.csg_dartel_relax(1, batch, 1, 1, hess.data_ptr(), rhs.data_ptr(), params, 1, plain.data_ptr(), 0) == 0
+            assert lib.csg_dartel_fmg(1, batch, 1, 1, hess.data_ptr(), rhs.data_ptr(), params, 1, 1, kept.data_ptr(), 1, 1,
+                                      scratch.data_ptr(), scratch.numel(), 0) == 0
+            torch.cuda.synchronize()
+            same = (plain.view(torch.int64) == kept.view(torch.int64)) | (plain.isnan() & kept.isnan())
+            assert bool(same.all()), (rhs[~same.all(1)][:3], hess[~same.all(1)][:3])
+            det = first * 1.0000000001
+            hits += int(np.count_nonzero(np.frexp(np.abs(det))[0] == 1.0 - 2.0**-53))
+    assert hits > 1000  # divisors of all ones were among them
