@@ -64,8 +64,8 @@ WORKLOAD = ("Surf2Sphere (stages 1-5 + 4,999 ordered sweeps, 61,442 v / 122,880 
             "to a second 61,442-v hull, 256x128 float64 DARTEL sheet")
 SWEEPS = 4999
 # dram__bytes_read.sum + dram__bytes_write.sum of areal_dataflow_kernel<CAT, 8> over 200 sweeps of the
-# 61,442-vertex hull (9.1 MB + 0.85 MB; ncu summary in profiles/areal_dataflow_61k_hull_200sweeps.md)
-SWEEP_DRAM_BYTES = 9.95e6
+# 61,442-vertex hull (11.1 MB + 1.5 MB; ncu summary in profiles/areal_dataflow_61k_hull_200sweeps.md)
+SWEEP_DRAM_BYTES = 12.6e6
 SHEET = (256, 128)
 CHAIN = dict(steps=2, runs=2, avg=True, loop=6, sheet_size=SHEET, rotation_feature_backend="cuda",
              rotation_feature_solver="colored-sor")

@@ -674,8 +674,8 @@ __global__ void k_resize(const T* __restrict__ src, T* __restrict__ dst, int snx
 // cluster the neighbours' edge rows are written straight into each other's shared memory and
 // a link costs 250-550 ns.  Per V-cycle, against legs of 2-D tiles over one CTA for the
 // coarse levels: two 256 x 128 grids 129 -> 56 us in float64 and 123 -> 57 in float32, 64 x 32
-// 71 -> 27 us, 32 x 16 47 -> 17 us; 32 float32 grids of 256 x 128 369 -> 243 us, 64 float64 grids
-// 731 -> 561 us.  Of the 56 us the first level takes 20, the other split levels 20, the levels of
+// 71 -> 27 us, 32 x 16 47 -> 17 us.  Batches of several waves of clusters take legs on the finer levels
+// (see ResidentCosts).  Of the 56 us the first level takes 20, the other split levels 20, the levels of
 // CTA 0 17.
 //
 // Levels above kCoarsePoints points are split by rows over the cluster's CTAs, each
@@ -697,7 +697,7 @@ constexpr int kMaxCluster = 16;     // 16 CTAs is the largest cluster of the arc
 // A launch of more CTAs than the device's 148 SMs hold as clusters of 16 uses as few CTAs per grid
 // as hold it (64 float64 grids of 128 x 64 per V-cycle: 354 us with 16 CTAs each, 95 with 4; two
 // of them: 36 and 55), and in float32 the kernel of 128 registers, two CTAs to an SM (32 grids of
-// 256 x 128: 286 -> 243 us; two: 57 and 71).
+// 256 x 128, resident throughout: 286 -> 243 us; two: 57 and 71).
 constexpr int kPairedCtas = 128;
 
 // Both components of a field at a point, moved together.

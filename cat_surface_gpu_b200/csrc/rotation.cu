@@ -299,7 +299,7 @@ __device__ __forceinline__ double cost_at(const RotSurface& S, const float (&q)[
         // reach from the first pass and test the survivors of a bit mask, so the threads of a
         // warp loop over their own short lists.
         //
-        // What bounds this is the L1: every thread gathers other triangles' records (79% of
+        // What bounds this is the L1: every thread gathers other triangles' records (87% of
         // the wavefront peak), and a float32 reach per candidate, 256 bytes a thread, left
         // little of it for them.  Codes of 8 bits, four candidates' records in flight and no
         // second test of the first candidate: 25.8 -> 22.7 ms (reading the spheres twice
