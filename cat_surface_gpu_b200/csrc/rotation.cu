@@ -244,17 +244,29 @@ __global__ void k_triangle_records(const float* __restrict__ tri, int n, float* 
 
 // Lower bound of the distance from q to every point the test can return for a record's
 // triangle (0 when q is inside the bounding sphere).
-__device__ __forceinline__ float record_reach(const float* q, const float* rec) {
+__device__ __forceinline__ float record_reach(const float* q, const float* rec, float& radius) {
     const float4 b = __ldg(reinterpret_cast<const float4*>(rec) + 4);
+    radius = b.w;
     const float dx = q[0] - b.x, dy = q[1] - b.y, dz = q[2] - b.z;
     const float dist = sqrtf(dx * dx + dy * dy + dz * dz);
     return dist > b.w ? dist - b.w : 0.0f;
 }
 
-// A reach as a multiple of kReachUnit, rounded down (at most 255): still a lower bound.  The
-// unit is a power of two, so the products are exact.
-constexpr float kReachUnit = 1.0f / 16384.0f;
-__device__ __forceinline__ unsigned reach_code(float r) { return static_cast<unsigned>(fminf(r * (1.0f / kReachUnit), 255.0f)); }
+// A reach as a multiple of a unit, rounded down (at most 255): still a lower bound.  The unit is a
+// power of two, so the products are exact: a 64th of the power of two that a bounding sphere's radius R of the
+// cell lies above, so codes end between 2 R and 4 R.  The candidate of least reach seldom leaves a limit above
+// its sphere's diameter, so what the codes cannot tell apart is beyond the limit.  (A fixed unit of 2^-14 did
+// for the spheres of a 40,962-point target; triangles four times as long, whose limits lay above
+// 255 units, were all tested: 2,562 points in a grid of 32^3, 2.1 -> 4.0 ms for 8 M evaluations.)
+struct ReachUnit {
+    float unit, inverse;
+    __device__ __forceinline__ explicit ReachUnit(float radius) {
+        const int e = min(max((__float_as_int(radius) >> 23 & 255) - 127, -60), 60);
+        unit = __int_as_float((127 + e - 6) << 23);
+        inverse = __int_as_float((127 + 6 - e) << 23);
+    }
+    __device__ __forceinline__ unsigned code(float reach) const { return static_cast<unsigned>(fminf(reach * inverse, 255.0f)); }
+};
 
 // Barycentric weights of `point` in triangle t (surface_rotation.py:335-352).
 __device__ __forceinline__ void barycentric(const float* point, const float* t, float w[3]) {
@@ -308,19 +320,22 @@ __device__ __forceinline__ double cost_at(const RotSurface& S, const float (&q)[
         const int count = end - begin;
         const bool compact = S.records != nullptr && count <= kMaxCompact;
         unsigned reach[kMaxCompact / 4];  // four codes to a word
-        float limit = INFINITY;
+        float limit = INFINITY, unit = 0.0f;
         int pick_at = -1, best_at = 0;
         if (S.records) {
             float least = INFINITY;
             int pick = -1;
+            ReachUnit reaches(0.0f);
             for (int k0 = 0; k0 < count; k0 += 4) {
                 int f[4];
-                float r[4];
+                float r[4], radius[4];
                 unsigned codes = 0;
 #pragma unroll
                 for (int j = 0; j < 4; ++j) f[j] = S.grid_faces[begin + min(k0 + j, count - 1)];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) r[j] = record_reach(q, S.records + kRecordFloats * static_cast<long long>(f[j]));
+                for (int j = 0; j < 4; ++j)
+                    r[j] = record_reach(q, S.records + kRecordFloats * static_cast<long long>(f[j]), radius[j]);
+                if (k0 == 0) reaches = ReachUnit(fmaxf(fmaxf(radius[0], radius[1]), fmaxf(radius[2], radius[3])));
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     if (k0 + j < count && r[j] < least) {
@@ -328,10 +343,11 @@ __device__ __forceinline__ double cost_at(const RotSurface& S, const float (&q)[
                         pick = f[j];
                         pick_at = k0 + j;
                     }
-                    codes |= reach_code(r[j]) << 8 * j;
+                    codes |= reaches.code(r[j]) << 8 * j;
                 }
                 if (compact) reach[k0 / 4] = codes;
             }
+            unit = reaches.unit;
             if (pick >= 0) {
                 float point[3];
                 const float d0 = candidate_record(q, S.records + kRecordFloats * static_cast<long long>(pick), point);
@@ -368,19 +384,25 @@ __device__ __forceinline__ double cost_at(const RotSurface& S, const float (&q)[
                 const unsigned codes = reach[k0 / 4];
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
-                    if (k0 + j < count && !(static_cast<float>(codes >> 8 * j & 255u) * kReachUnit > limit))
+                    if (k0 + j < count && !(static_cast<float>(codes >> 8 * j & 255u) * unit > limit))
                         live |= 1ull << (k0 + j);
             }
             if (pick_at >= 0) live &= ~(1ull << pick_at);
+            // (a query far from the target, or triangles of very unequal sizes: the codes end below the limit)
+            const bool beyond = !(255.0f * unit > limit);
             while (live) {
                 const int k = __ffsll(static_cast<long long>(live)) - 1;
                 live &= live - 1;
-                test(k, S.grid_faces[begin + k]);
+                const int f = S.grid_faces[begin + k];
+                float radius;
+                if (beyond && record_reach(q, S.records + kRecordFloats * static_cast<long long>(f), radius) > limit) continue;
+                test(k, f);
             }
         } else {
             for (int k = begin; k < end; ++k) {
                 const int f = S.grid_faces[k];
-                if (S.records && record_reach(q, S.records + kRecordFloats * static_cast<long long>(f)) > limit)
+                float radius;
+                if (S.records && record_reach(q, S.records + kRecordFloats * static_cast<long long>(f), radius) > limit)
                     continue;
                 if (k - begin != pick_at) test(k - begin, f);
             }

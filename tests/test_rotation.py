@@ -346,3 +346,47 @@ def test_large_launches_equal_single_candidates(native_library, tile, sizes):
     for i, costs in enumerate(together):
         alone = batched_costs([index], [inputs[i]], matrix_sets=[few], tile=tile)[0]
         assert torch.equal(costs, alone.repeat(repeats)), sizes[i]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("subdivisions, grid_size", [(1, 8), (2, 16), (3, 24), (4, 32), (5, 64)])
+@pytest.mark.parametrize("radius", [0.9, 1.0, 1.05])
+@pytest.mark.parametrize("uneven", [False, True])
+def test_reach_codes_on_any_target(native_library, subdivisions, grid_size, radius, uneven):
+    """The records' pruning with triangles of other lengths than the grid's cells, of very unequal lengths in
+    one cell, and for points off the sphere, whose limits lie beyond the codes: the costs without records."""
+
+    import ctypes
+
+    import torch
+
+    from cat_surface_gpu_b200 import _native, synthetic
+    from cat_surface_gpu_b200.surface_rotation import RotationGridIndexDevice, rotation_matrices_flat
+
+    rng = np.random.default_rng(100 * subdivisions + grid_size)
+    tp, tf = synthetic.unit_icosphere(subdivisions)
+    if uneven:  # points drawn together towards a pole: triangles from a thirtieth to three times the even length
+        tp = tp.copy()
+        tp[:, 2] = 1.0 - 2.0 * ((1.0 - tp[:, 2]) / 2.0) ** 2.5
+        ring = np.hypot(tp[:, 0], tp[:, 1])
+        tp[:, :2] *= (np.sqrt(np.maximum(0.0, 1.0 - tp[:, 2] ** 2)) / np.maximum(ring, 1e-12))[:, None]
+    index = RotationGridIndexDevice.build(tp, tf, device="cuda:0", grid_size=grid_size, margin=2)
+    src = rng.normal(size=(1500, 3))
+    src = (radius * src / np.linalg.norm(src, axis=1, keepdims=True)).astype(np.float32)
+    inputs = index.prepare_cost_inputs(src, np.sin(4 * src[:, 0]).astype(np.float64), np.sin(4 * tp[:, 0]))
+    mats = torch.as_tensor(rotation_matrices_flat(rng.uniform(-1, 1, size=(6, 3))), device="cuda:0")
+    n_src, n_cand = (ctypes.c_int * 1)(src.shape[0]), (ctypes.c_int * 1)(6)
+    need = native_library.csg_rotation_scratch_bytes(1, ctypes.addressof(n_src), ctypes.addressof(n_cand), 256)
+    out = []
+    for records in (None, index.target_records.data_ptr()):
+        surface = _native.RotationSurface(
+            inputs.source_points.data_ptr(), inputs.source_values.data_ptr(), index.target_triangles.data_ptr(),
+            index.target_faces.data_ptr(), inputs.target_values.data_ptr(), index.candidate_offsets.data_ptr(),
+            index.candidate_faces.data_ptr(), mats.data_ptr(), src.shape[0], index.grid_size, 6, 1,
+            int(index.target_points.shape[0]), records)
+        scratch = torch.empty(int(need), dtype=torch.uint8, device="cuda:0")
+        costs = torch.empty(6, dtype=torch.float64, device="cuda:0")
+        assert native_library.csg_rotation_cost_batch(1, ctypes.addressof(surface), costs.data_ptr(), 256, 0,
+                                                      scratch.data_ptr(), scratch.numel(), 0) == 0
+        out.append(costs.cpu().numpy())
+    assert np.array_equal(out[0], out[1])
