@@ -205,8 +205,10 @@ __global__ void k_heat_weights(const T* __restrict__ geometry, const int* __rest
 // every series starts from the caller's single value array) and writes
 // out[s * n ...]; `in` and `out` never alias (Jacobi update); a series whose
 // iteration count is reached copies its values through; a grid barrier
-// between iterations.  As above, a thread keeps the neighbours and weights of its first point
-// (40,962 points of a registration: 263 -> 187 us).
+// between iterations.  HELD: as above, a thread keeps the neighbours and weights of its first point
+// (40,962 points of a registration: 263 -> 187 us); else every point reads its own each time, with
+// threads enough for twice as many points at once.  See smooth_held for the choice.
+template <bool HELD>
 __global__ void k_smooth_values_all(const double* __restrict__ in, double* __restrict__ out,
                                     double* __restrict__ tmp, const double* __restrict__ weights,
                                     const double* __restrict__ wsum, const int* __restrict__ off,
@@ -222,20 +224,22 @@ __global__ void k_smooth_values_all(const double* __restrict__ in, double* __res
     const int held_s = tid < total ? static_cast<int>(tid / n) : 0, held_i = static_cast<int>(tid - static_cast<long long>(held_s) * n);
     int held[kHeld], begin = 0, end = 0;
     double weight[kHeld], held_den = 1.0;
-    if (tid < total) {
-        begin = off[held_i];
-        end = off[held_i + 1];
-        held_den = 1.0 + wsum[tid];
-    }
+    if constexpr (HELD) {
+        if (tid < total) {
+            begin = off[held_i];
+            end = off[held_i + 1];
+            held_den = 1.0 + wsum[tid];
+        }
 #pragma unroll
-    for (int k = 0; k < kHeld; ++k) {
-        held[k] = begin + k < end ? nbr[begin + k] : -1;
-        weight[k] = begin + k < end ? weights[static_cast<long long>(held_s) * slots + begin + k] : 0.0;
+        for (int k = 0; k < kHeld; ++k) {
+            held[k] = begin + k < end ? nbr[begin + k] : -1;
+            weight[k] = begin + k < end ? weights[static_cast<long long>(held_s) * slots + begin + k] : 0.0;
+        }
     }
     for (int it = 0; it < max_it; ++it) {
         double* dst = ((max_it - 1 - it) % 2 == 0) ? out : tmp;
         for (long long q = tid; q < total; q += nthreads) {
-            const bool first = q == tid;
+            const bool first = HELD && q == tid;
             const int s = first ? held_s : static_cast<int>(q / n);
             const int i = first ? held_i : static_cast<int>(q - static_cast<long long>(s) * n);
             const double* from = src + static_cast<long long>(s) * stride;
@@ -269,16 +273,27 @@ __global__ void k_smooth_values_all(const double* __restrict__ in, double* __res
     }
 }
 
-// Grid of a cooperative launch of `kernel`: as many kSmoothThreads-blocks as `work`
-// needs, at most as many as the device holds at once.
-int cooperative_grid(const void* kernel, long long work, unsigned* grid) {
+// Grid of a cooperative launch of `kernel`: as many blocks of `threads` as `work` needs, at most as many as
+// the device holds at once (*at_once threads).
+int cooperative_grid(const void* kernel, long long work, int threads, unsigned* grid, long long* at_once = nullptr) {
     int device = 0, sms = 0, per_sm = 0;
     CSG_CUDA_CHECK(cudaGetDevice(&device));
     CSG_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    CSG_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kSmoothThreads, 0));
+    CSG_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0));
     const long long resident = static_cast<long long>(sms) * (per_sm > 0 ? per_sm : 1);
-    *grid = static_cast<unsigned>(std::max(1LL, std::min(resident, (work + kSmoothThreads - 1) / kSmoothThreads)));
+    *grid = static_cast<unsigned>(std::max(1LL, std::min(resident, (work + threads - 1) / threads)));
+    if (at_once) *at_once = resident * threads;
     return CSG_OK;
+}
+
+// Whether k_smooth_values_all keeps lists in registers, for `work` points of which the device holds at_once threads
+// of that kernel (113,664).  It gains where every thread has one point, and from about twice to eleven times as many
+// points, where the held lists are a good part of what an iteration reads.  In between some threads
+// have a second point and all wait for them, and beyond, its fewer threads count.  An iteration, in us, held and
+// not: 81,924 points 3.5 and 4.4, 122,886 5.6 and 4.9, 163,848 6.6 and 5.5, 204,810 6.5 and 6.5,
+// 327,696 8.1 and 11.7, 983,052 18.5 and 21.4, 1,310,736 26.3 and 25.5, 2,621,448 66 and 48.
+bool smooth_held(long long work, long long at_once) {
+    return work <= at_once || (4 * work >= 7 * at_once && work <= 11 * at_once);
 }
 
 size_t align_up_256(size_t x) { return (x + 255) & ~static_cast<size_t>(255); }
@@ -541,7 +556,7 @@ int csg_feature_smooth_geometry(int n_points, const int32_t* nbr_off, const int3
     csg::Control* ctl = reinterpret_cast<csg::Control*>(static_cast<char*>(scratch) + control_at);
     CSG_CUDA_CHECK(cudaMemsetAsync(ctl, 0, sizeof(csg::Control), s));
     unsigned grid = 1;
-    int rc = cooperative_grid(reinterpret_cast<const void*>(k_smooth_geometry_all), n_points, &grid);
+    int rc = cooperative_grid(reinterpret_cast<const void*>(k_smooth_geometry_all), n_points, kSmoothThreads, &grid);
     if (rc) return rc;
     unsigned long long timeout_ns = 2000000000ULL;
     const float* in = vertices;
@@ -591,16 +606,24 @@ int csg_feature_smooth_values(int n_points, const int32_t* nbr_off, const int32_
         csg::Control* ctl = reinterpret_cast<csg::Control*>(
             static_cast<char*>(scratch) + align_up_256(8ULL * series * (static_cast<size_t>(n_slots) + 2ULL * n_points)));
         CSG_CUDA_CHECK(cudaMemsetAsync(ctl, 0, sizeof(csg::Control), s));
+        const void* kernel = reinterpret_cast<const void*>(k_smooth_values_all<true>);
+        int threads = kSmoothThreads;
+        const long long work = static_cast<long long>(series) * n_points;
         unsigned cgrid = 1;
-        int rc = cooperative_grid(reinterpret_cast<const void*>(k_smooth_values_all),
-                                  static_cast<long long>(series) * n_points, &cgrid);
+        long long at_once = 0;
+        int rc = cooperative_grid(kernel, work, threads, &cgrid, &at_once);
         if (rc) return rc;
+        if (!smooth_held(work, at_once)) {
+            kernel = reinterpret_cast<const void*>(k_smooth_values_all<false>);
+            threads = kThreads;
+            rc = cooperative_grid(kernel, work, threads, &cgrid);
+            if (rc) return rc;
+        }
         unsigned long long timeout_ns = 2000000000ULL;
         const double* in = values;
         void* args[] = {&in, &out, &tmp, &weights, &wsum, const_cast<int32_t**>(&nbr_off), const_cast<int32_t**>(&nbr),
                         &n_points, &series, &sp, &max_it, &ctl, &timeout_ns};
-        CSG_CUDA_CHECK(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_smooth_values_all), dim3(cgrid),
-                                                   dim3(kSmoothThreads), args, 0, s));
+        CSG_CUDA_CHECK(cudaLaunchCooperativeKernel(kernel, dim3(cgrid), dim3(threads), args, 0, s));
         csg::note_launch();
     }
     if (max_it == 0)

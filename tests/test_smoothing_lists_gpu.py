@@ -74,3 +74,34 @@ def test_values(native_library, n):
         ctypes.addressof(sigmas), ctypes.addressof(iterations), 0, out.data_ptr(), scratch.data_ptr(), scratch.numel(), 0) == 0
     torch.cuda.synchronize()
     np.testing.assert_array_equal(out.cpu().numpy(), np.stack(want))
+
+
+@pytest.mark.parametrize("n, series", [(120_000, 1), (45_000, 3), (110_000, 2), (660_000, 2)])
+def test_values_of_more_points_than_threads(native_library, n, series):
+    """Launches of more points than threads that keep lists: just more, twice as many, and more than eleven times."""
+
+    import ctypes
+
+    rng = np.random.default_rng(n + series)
+    degree, offsets, neighbours = _lists(n, rng)
+    values = rng.normal(size=n)
+    want = []
+    for count in range(1, series + 1):
+        field = values.copy()
+        for _ in range(count):
+            total = np.zeros(n)
+            for k in range(int(degree.max(initial=0))):
+                has = degree > k
+                total[has] = total[has] + field[neighbours[offsets[:-1][has] + k]]
+            field = (field + total) / (1.0 + degree)
+        want.append(field)
+    v, off, nbr = _device(values), _device(offsets), _device(neighbours)
+    geometry = torch.zeros(n, 3, dtype=torch.float64, device="cuda")  # coincident points: every weight is exactly 1
+    out = torch.empty(series, n, dtype=torch.float64, device="cuda")
+    scratch = torch.empty(16 * series * (neighbours.size + 3 * n) + (1 << 20), dtype=torch.uint8, device="cuda")
+    sigmas, iterations = (ctypes.c_double * series)(*[1.0] * series), (ctypes.c_int32 * series)(*range(1, series + 1))
+    assert native_library.csg_feature_smooth_values(
+        n, off.data_ptr(), nbr.data_ptr(), int(neighbours.size), 1, geometry.data_ptr(), v.data_ptr(), series,
+        ctypes.addressof(sigmas), ctypes.addressof(iterations), 0, out.data_ptr(), scratch.data_ptr(), scratch.numel(), 0) == 0
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(out.cpu().numpy(), np.stack(want))
